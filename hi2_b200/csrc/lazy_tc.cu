@@ -453,18 +453,21 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_ahi, const __grid_constan
 }
 
 // TF32 parts of a [rows, cols] block with leading dimension ldx, written with leading dimension ldo.
+// lower: x is lower triangular and what lies above its diagonal is not read; its parts are zeros.
 __global__ void __launch_bounds__(256)
 split_block_kernel(const float* __restrict__ x, int64_t ldx, int64_t rows, int64_t cols,
-                   float* __restrict__ hi, float* __restrict__ lo, int64_t ldo) {
+                   float* __restrict__ hi, float* __restrict__ lo, int64_t ldo, bool lower) {
   const int64_t c4 = cols / 4;  // cols is a multiple of 4
   const int64_t total = rows * c4, stride = (int64_t)gridDim.x * 256;
   for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < total; i += stride) {
     const int64_t r = i / c4, c = (i % c4) * 4;
-    const float4 v = *reinterpret_cast<const float4*>(x + r * ldx + c);
-    const float in[4] = {v.x, v.y, v.z, v.w};
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (!lower || c <= r) v = *reinterpret_cast<const float4*>(x + r * ldx + c);
+    float in[4] = {v.x, v.y, v.z, v.w};
     float h[4], l[4];
 #pragma unroll
     for (int t = 0; t < 4; ++t) {
+      if (lower && c + t > r) in[t] = 0.0f;
       uint32_t hb, lb;
       asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(hb) : "f"(in[t]));
       h[t] = __uint_as_float(hb);
@@ -479,12 +482,12 @@ split_block_kernel(const float* __restrict__ x, int64_t ldx, int64_t rows, int64
 // The same for the transpose: x [rows, cols] (ldx) -> hi, lo [cols, rows] (ldo).
 __global__ void __launch_bounds__(256)
 split_block_transposed_kernel(const float* __restrict__ x, int64_t ldx, int64_t rows, int64_t cols,
-                              float* __restrict__ hi, float* __restrict__ lo, int64_t ldo) {
+                              float* __restrict__ hi, float* __restrict__ lo, int64_t ldo, bool lower) {
   __shared__ float tile[32][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int64_t c0 = (int64_t)blockIdx.x * 32, r0 = (int64_t)blockIdx.y * 32;
   for (int i = ty; i < 32; i += 8)
-    tile[i][tx] = (r0 + i < rows && c0 + tx < cols) ? x[(r0 + i) * ldx + c0 + tx] : 0.0f;
+    tile[i][tx] = (r0 + i < rows && c0 + tx < cols && !(lower && c0 + tx > r0 + i)) ? x[(r0 + i) * ldx + c0 + tx] : 0.0f;
   __syncthreads();
   for (int i = ty; i < 32; i += 8) {
     if (c0 + i < cols && r0 + tx < rows) {
@@ -643,15 +646,15 @@ int launch_gemm_tc2(int64_t m, int64_t n, int64_t kk, const float* a_hi, const f
 }
 
 int launch_split_block(const float* x, int64_t ldx, int64_t rows, int64_t cols, float* hi, float* lo,
-                       int64_t ldo, bool transposed, cudaStream_t stream) {
+                       int64_t ldo, bool transposed, bool lower, cudaStream_t stream) {
   if (rows <= 0 || cols <= 0) return HI2_OK;
   if (transposed) {
     dim3 grid((unsigned)ceil_div(cols, 32), (unsigned)ceil_div(rows, 32));
-    split_block_transposed_kernel<<<grid, 256, 0, stream>>>(x, ldx, rows, cols, hi, lo, ldo);
+    split_block_transposed_kernel<<<grid, 256, 0, stream>>>(x, ldx, rows, cols, hi, lo, ldo, lower);
   } else {
     int64_t blocks = ceil_div(rows * (cols / 4), 256);
     if (blocks > 148 * 16) blocks = 148 * 16;
-    split_block_kernel<<<(unsigned)blocks, 256, 0, stream>>>(x, ldx, rows, cols, hi, lo, ldo);
+    split_block_kernel<<<(unsigned)blocks, 256, 0, stream>>>(x, ldx, rows, cols, hi, lo, ldo, lower);
   }
   return check_launch("split_block");
 }
