@@ -1,278 +1,408 @@
 // Fixed-ladder GPTQ rounding (hi2/gptq_kernel.py:59-127, hi2/hessian.py:267-315).
 //
-// Block kernel: one LANE per row (see gptq_block_kernel).  Each product, sum and quotient is
+// Block kernel: four lanes per row (see gptq_block_kernel).  Each product, sum and quotient is
 // rounded on its own (the library is built without FMA contraction) and wq is rounded to fp16
 // before the error is formed, so given the same inputs the codes equal those of the
 // column-by-column loop.
 //
-// Trailing update: wc[:, i2:] -= err1 @ U[i1:i2, i2:] in fp32 FMA arithmetic (gemm.cuh).
+// Trailing update: wc[:, i2:] -= err1 @ U[i1:i2, i2:], in fp32 FMA arithmetic (gemm.cuh) or as three
+// TF32 products (lazy_tc.cu); neighbouring units with one factor share a launch.
 #include "gemm.cuh"
+
+#include <vector>
 
 namespace hi2 {
 
 int launch_lazy_tc(float* wc, int64_t n_rows, int64_t k, int64_t i1, const float* err_hi,
                    const float* err_lo, const float* u_hi, const float* u_lo, int* status,
                    cudaStream_t stream);
-int launch_split_tf32(const float* x, float* hi, float* lo, int64_t n, cudaStream_t stream);
 
 namespace {
 
 constexpr int LMAX = 128;
-constexpr int ROWS_PER_CTA = 64;  // one lane per row; three thread blocks (and staged factor blocks) per SM
+constexpr int WIN = 16;           // columns rounded between two updates of the columns behind them
+constexpr int GROUP_LANES = 4;    // lanes that share a row
+constexpr int BLOCK_THREADS = 128;
+// Shared memory: the factor block as windows of 16 rows that start at their own first column, then
+// (U[j, j], its reciprocal) per column, then per row the ladders of the window's columns and 16
+// exchange floats (row strides of 4 and 20 banks: a 128-bit access of eight rows meets every bank once).
+constexpr int U_FLOATS = WIN * (LMAX / WIN) * (LMAX + WIN) / 2;
+constexpr int U_DIAG = U_FLOATS;
+constexpr int ROW_STAGE = U_DIAG + 2 * LMAX;
+constexpr int LADDER_STRIDE = 4 * WIN + 4, SWAP_STRIDE = WIN + 4;
+__host__ __device__ constexpr int window_base(int win) { return WIN * (LMAX * win - (WIN / 2) * win * (win - 1)); }
+static_assert(window_base(LMAX / WIN) == U_FLOATS, "the windows fill the factor stage");
 
-// One LANE per row.  The row's segment of up to 128 columns lives in registers as 64 pairs and
-// moves down by one pair every two steps, so the columns being rounded are always the first
-// pair, every register index is static and two steps are a compact loop body.  The updates use
-// a packed fp32 multiply for two columns at a time (see sub_scaled):
-// new pair[t] = pair[t+1] - eA * U[j, ..] - eB * U[j+1, ..].  The block
-// U[i1:i1+len, i1:i1+len] is staged in shared memory with every row already shifted to the
-// column its first pair starts at, where U[j, c] is the same address for every lane (a
-// broadcast), and the dependent chain of a column carries no shuffle.  The loop is
-// software-pipelined: the error of column j is applied while column j+1 is rounded from the one
-// value it needs, and so on, so the chains run inside the updates instead of between them.  The
-// live width shrinks in four phases (128, 96, 64, 32 registers) as the columns are used up.
-// Rows of one thread block that read different factors (a block that straddles two tensors) are
-// served one factor after the other.
-constexpr int U_DIAG = LMAX * LMAX;          // diagonal U[j, j] (padded with ones)
-constexpr int U_NEXT = U_DIAG + 2 * LMAX;    // U[j, j+1]
-constexpr int U_STAGE_FLOATS = U_NEXT + LMAX;
-
-// pair - e * (u0, u1) with the product and the difference rounded separately.  The product is one
+// (w0, w1) - e * (u0, u1) with the product and the difference rounded separately.  The product is one
 // packed multiply; the two additions stay scalar on purpose: a packed multiply feeding a packed
 // add is contracted into a packed FMA by the assembler even with contraction switched off, and
 // a fused update no longer gives the codes of the reference's separately rounded one.
-__device__ __forceinline__ float2 sub_scaled(float2 w, float2 neg_e, float u0, float u1) {
+__device__ __forceinline__ void sub_scaled(float& w0, float& w1, float2 neg_e, float u0, float u1) {
   const float2 p = __fmul2_rn(neg_e, make_float2(u0, u1));
-  return make_float2(w.x + p.x, w.y + p.y);
+  w0 += p.x, w1 += p.y;
 }
 
-struct Ladder {
-  float lo, st;
-};
-
-// Code and scaled error of one column (hi2/gptq_kernel.py:88-101): exactly the IEEE quotients
-// the reference forms.  The fast path (one reciprocal product per division) is computed
-// unconditionally and redone with true divisions in the rare unsafe case, so the common path is
-// straight-line code.
-__device__ __forceinline__ void round_column(float col, Ladder p, float ud, float nm, float& q_out, float& e_out) {
-  const float safe = (p.st == 0.0f) ? 1.0f : p.st;
-  const Recip rs = make_recip(safe), ru = make_recip(ud);
-  const float a = col - p.lo;
-  const float t = a * rs.r;
-  float q = rintf(t);
-  const bool near = fabsf(fabsf(t - q) - 0.5f) < 2.5e-4f && fabsf(t) < 1024.0f;
-  if (!rs.fast || !ru.fast || near) {  // rare
-    q = rintf(__fdiv_rn(a, safe));
-    q = (q < 0.0f) ? 0.0f : q;
-    q = (q > nm) ? nm : q;
-    if (p.st == 0.0f) q = 0.0f;
-    const float wq = round_f16(p.lo + q * p.st);
-    q_out = q;
-    e_out = __fdiv_rn(col - wq, ud);
-    return;
-  }
+// Code and scaled error of one column (hi2/gptq_kernel.py:88-101) with true divisions.
+__device__ __noinline__ float2 round_careful(float col, float lo, float st, float ud, float nm) {
+  const float safe = (st == 0.0f) ? 1.0f : st;
+  float q = rintf(__fdiv_rn(col - lo, safe));
   q = (q < 0.0f) ? 0.0f : q;
   q = (q > nm) ? nm : q;
-  if (p.st == 0.0f) q = 0.0f;
-  const float wq = round_f16(p.lo + q * p.st);
-  const float num = col - wq;
-  const float q0 = num * ru.r;
-  q_out = q;
-  e_out = fmaf(fmaf(-q0, ud, num), ru.r, q0);
+  if (st == 0.0f) q = 0.0f;
+  const float wq = round_f16(lo + q * st);
+  return make_float2(q, __fdiv_rn(col - wq, ud));
 }
 
-// Per-row state between steps.  Everything that a load fills is addressed by column modulo 4 with
-// the step loop unrolled four times, so a value in flight is never moved: a register copy of it
-// would wait for the load and put its latency back on every step.
-template <bool WITH_COMP>
-struct RowState {
-  int j;      // the column whose error is applied next (a multiple of 4 between iterations)
-  float e;    // its scaled error
-  float ev[4], cv[4];  // outputs of the current quad of columns
-  uint32_t qk;
-  Ladder p[4];  // ladders of columns j+1 .. j+4
-  int b[4];     // block indices of columns j+5 .. j+8
-};
-
-// Steps while more than W - 32 columns remain (W registers live: w[0] holds columns s.j, s.j+1).
-template <int W, bool WITH_COMP>
-__device__ __forceinline__ void run_phase(float2 (&w)[LMAX / 2], RowState<WITH_COMP>& s, int len, float nm,
-                                          const float* __restrict__ u_stage, const int32_t* __restrict__ brow,
-                                          const float* __restrict__ lorow, const float* __restrict__ strow,
-                                          bool live, float* err_row, uint8_t* code_row, float* comp_row) {
-  const int last = len - 1;
-  constexpr int P = W / 2;  // live pairs
-#pragma unroll 1
-  while (len - s.j > W - 32 && s.j < len) {
-    const int j0 = s.j;
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int j = j0 + 2 * h;                      // even: the column whose error is known
-      const float* ua = u_stage + j * LMAX;          // ua[t] = U[j, j+2+t]
-      const float* ub = ua + LMAX;                   // ub[t] = U[j+1, j+2+t]
-      const float ea = s.e;
-      // column j+1: one scalar update, then its rounding (overlaps the packed updates below)
-      const float cb = w[0].y - ea * u_stage[U_NEXT + j];
-      float qb, eb;
-      round_column(cb, s.p[(2 * h + 1) & 3], u_stage[U_DIAG + j + 1], nm, qb, eb);
-      const float2 na = make_float2(-ea, -ea);
-#pragma unroll
-      for (int t = 0; t + 1 < P; t += 2) {
-        const float4 v = *reinterpret_cast<const float4*>(ua + 2 * t);
-        w[t] = sub_scaled(w[t + 1], na, v.x, v.y);
-        if (t + 2 < P) w[t + 1] = sub_scaled(w[t + 2], na, v.z, v.w);
-      }
-      w[P - 1] = make_float2(0.0f, 0.0f);
-      // column j+2 (ignored past the last column)
-      const float4 fb = *reinterpret_cast<const float4*>(ub);
-      const float ca = w[0].x - eb * fb.x;
-      float qa, ea2;
-      round_column(ca, s.p[(2 * h + 2) & 3], u_stage[U_DIAG + j + 2], nm, qa, ea2);
-      const float2 nb = make_float2(-eb, -eb);
-      w[0] = sub_scaled(w[0], nb, fb.x, fb.y);
-      if (1 < P) w[1] = sub_scaled(w[1], nb, fb.z, fb.w);
-#pragma unroll
-      for (int t = 2; t < P; t += 2) {
-        const float4 v = *reinterpret_cast<const float4*>(ub + 2 * t);
-        w[t] = sub_scaled(w[t], nb, v.x, v.y);
-        if (t + 1 < P) w[t + 1] = sub_scaled(w[t + 1], nb, v.z, v.w);
-      }
-      // outputs of columns j+1 and j+2 (slot 3 completes the quad j0 .. j0+3, slot 0 opens the next)
-      const int sb = (2 * h + 1) & 3, sa = (2 * h + 2) & 3;
-      s.ev[sb] = eb;
-      if (WITH_COMP) s.cv[sb] = cb;
-      s.qk = (s.qk >> 8) | ((uint32_t)qb << 24);
-      if (sb == 3 && live) {
-        *reinterpret_cast<float4*>(err_row + j0) = make_float4(s.ev[0], s.ev[1], s.ev[2], s.ev[3]);
-        *reinterpret_cast<uint32_t*>(code_row + j0) = s.qk;
-        if (WITH_COMP) *reinterpret_cast<float4*>(comp_row + j0) = make_float4(s.cv[0], s.cv[1], s.cv[2], s.cv[3]);
-      }
-      s.ev[sa] = ea2;
-      if (WITH_COMP) s.cv[sa] = ca;
-      s.qk = (s.qk >> 8) | ((uint32_t)qa << 24);
-      // ladders of columns j+5 and j+6 into the slots just used, block indices of j+9 and j+10 behind them
-      s.p[sb].lo = lorow[s.b[sb]], s.p[sb].st = strow[s.b[sb]];
-      s.b[sb] = brow[min(j + 9, last)];
-      s.p[sa].lo = lorow[s.b[sa]], s.p[sa].st = strow[s.b[sa]];
-      s.b[sa] = brow[min(j + 10, last)];
-      s.e = ea2;
-    }
-    s.j = j0 + 4;
+// The same from prepared values: ladder = (lo, st, 1 / st, highest code: 0 for st == 0), diag = (U_jj,
+// 1 / U_jj).  a * (1 / st) is within 2 ulp of the quotient and rounds to the same integer unless it lies
+// within a few ulp of a half-integer; such columns, NaNs, and ladders and pivots whose reciprocal is
+// not usable (stored as NaN) take the careful path.  The integer is taken by adding and removing
+// 1.5 * 2^23, which rounds to nearest even below 2^22 and keeps anything larger beyond every ladder.
+// The error's quotient is finished with Markstein's fused correction and is the IEEE one.
+__device__ __forceinline__ void round_column(float col, float4 ladder, float2 diag, float nm, float& q_out,
+                                             float& e_out) {
+  const float t = (col - ladder.x) * ladder.z;
+  float q = (t + 12582912.0f) - 12582912.0f;
+  const bool clear = fabsf(fabsf(t - q) - 0.5f) >= 2.5e-4f;  // false for NaN
+  q = fminf(fmaxf(q, 0.0f), ladder.w);
+  const float num = col - round_f16(ladder.x + q * ladder.y);
+  const float q0 = num * diag.y;
+  q_out = q;
+  e_out = fmaf(fmaf(-q0, diag.x, num), diag.y, q0);
+  if (!clear) {
+    const float2 r = round_careful(col, ladder.x, ladder.y, diag.x, nm);
+    q_out = r.x, e_out = r.y;
   }
 }
 
-template <bool WITH_COMP>
-__global__ void __launch_bounds__(ROWS_PER_CTA, 3)
+__device__ __forceinline__ void tf32_parts(float x, float& hi, float& lo) {
+  uint32_t hb, lb;
+  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(hb) : "f"(x));
+  hi = __uint_as_float(hb);
+  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(lb) : "f"(x - hi));
+  lo = __uint_as_float(lb);
+}
+
+// The M quads a lane holds behind the window lose the window's sixteen errors, in column order.
+template <int R, int M>
+__device__ __forceinline__ void update_behind(float4 (&w)[R][LMAX / WIN], const float* u, int width, int quad,
+                                              const float* const (&swap)[R]) {
+#pragma unroll 1
+  for (int j = 0; j < WIN; j += 4) {
+    float4 e[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) e[r] = *reinterpret_cast<const float4*>(swap[r] + j);
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+      const float* row = u + (j + t) * width + 4 * quad;
+#pragma unroll
+      for (int m = 1; m <= M; ++m) {
+        const float4 v = *reinterpret_cast<const float4*>(row + WIN * m);
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          const float x = t == 0 ? e[r].x : t == 1 ? e[r].y : t == 2 ? e[r].z : e[r].w;
+          const float2 ne = make_float2(-x, -x);
+          sub_scaled(w[r][m].x, w[r][m].y, ne, v.x, v.y);
+          sub_scaled(w[r][m].z, w[r][m].w, ne, v.z, v.w);
+        }
+      }
+    }
+  }
+}
+
+// One lazy block: up to 128 columns of every row, rounded column by column.
+//
+// Four lanes share a row.  The block is taken in windows of 16 columns.  The window's values are kept by
+// all four lanes and every lane rounds its columns and applies their errors inside the window, so the
+// chain from one column to the next carries no exchange between lanes; the columns behind the window
+// are dealt out to the lanes in quads (lane h holds columns 16 m + 4 h .. + 3 of every later window)
+// and lose the window's sixteen errors afterwards, in column order, so every element sees the
+// operations of the column-by-column loop in their order.  After a window the quads move down by one
+// and every register index stays static.  Ladders, their reciprocals and the pivots' are prepared by the
+// lane that owns the column, a window ahead, and wait in shared memory; the factor block is staged
+// there once per thread block.  R rows per lane share the reads of the factor and give R independent
+// chains: R = 2 where the rows still fill the SMs, 1 below.
+// What bounds it: few rows, the chain (about 110 cycles a column); many rows, shared-memory reads of the
+// factor.  One lane per row with the 128 columns in its registers was bound by the chain at every size
+// and left most SMs idle at a few thousand rows; a block, lane per row -> this: 256 rows 79 -> 25 us,
+// 4096 81 -> 25, 11008 88 -> 40, 22016 107 -> 64, 32768 163 -> 89.
+// Rows of one thread block that read different factors (a block that straddles two tensors) are
+// served one factor after the other: everybody computes, only the rows of that factor store.
+template <int R, bool WITH_COMP, bool SPLIT>
+__global__ void __launch_bounds__(BLOCK_THREADS, (R == 1 ? 4 : 3))
 gptq_block_kernel(const float* __restrict__ wc, int64_t n_rows, int64_t k, int64_t i1, int len,
-                  float* __restrict__ err1, uint8_t* __restrict__ codes,
+                  float* __restrict__ err, float* __restrict__ err_lo, uint8_t* __restrict__ codes,
                   const float* __restrict__ lo, const float* __restrict__ st, int64_t ldp,
                   const int32_t* __restrict__ row_grp, const int64_t* __restrict__ u_ptrs,
                   const int32_t* __restrict__ blk, const float* __restrict__ nmax,
                   float* __restrict__ comp) {
-  extern __shared__ float4 u_stage4[];
-  float* u_stage = reinterpret_cast<float*>(u_stage4);
+  extern __shared__ __align__(16) float gptq_smem[];
   __shared__ unsigned long long next_factor;
+  constexpr int QUADS = LMAX / WIN;
+  const int lane = threadIdx.x & 31, quad = lane & 3;
+  const int row0 = (threadIdx.x >> 5) * 8 * R + (lane >> 2);  // this lane's rows of the block: row0 + 8 r
+  float* u = gptq_smem;
+  const float2* diag = reinterpret_cast<const float2*>(gptq_smem + U_DIAG);
+  float* ladders = gptq_smem + ROW_STAGE;
+  float* swaps = ladders + (BLOCK_THREADS / GROUP_LANES) * R * LADDER_STRIDE;
+  const int windows = len / WIN;
 
-  const int64_t row_raw = (int64_t)blockIdx.x * ROWS_PER_CTA + threadIdx.x;
-  const bool live = row_raw < n_rows;
-  const int64_t row = live ? row_raw : n_rows - 1;  // spare lanes shadow the last row and store nothing
-  const int g = row_grp[row];
-  const unsigned long long my_factor = (unsigned long long)u_ptrs[g];
-  const float nm = nmax[g];
-  const float* wrow = wc + row * k + i1;
-  const int32_t* brow = blk + (int64_t)g * k + i1;
-  const float* lorow = lo + row * ldp;
-  const float* strow = st + row * ldp;
-  float* err_row = err1 + row * len;
-  uint8_t* code_row = codes + row * k + i1;
-  float* comp_row = WITH_COMP ? comp + row * k + i1 : nullptr;
-  const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
-  const int last = len - 1;
+  int64_t row[R];
+  bool live[R], done[R];
+  unsigned long long factor_of[R];
+  float nm[R];
+  int group[R];
+  const float* swap[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int64_t raw = (int64_t)blockIdx.x * (BLOCK_THREADS / GROUP_LANES * R) + row0 + 8 * r;
+    live[r] = raw < n_rows;
+    row[r] = live[r] ? raw : n_rows - 1;  // spare lanes shadow the last row and store nothing
+    group[r] = row_grp[row[r]];
+    factor_of[r] = (unsigned long long)u_ptrs[group[r]];
+    nm[r] = nmax[group[r]];
+    done[r] = false;
+    swap[r] = swaps + (row0 + 8 * r) * SWAP_STRIDE;
+  }
 
-  bool done = false;
   while (true) {
     if (threadIdx.x == 0) next_factor = ~0ull;
     __syncthreads();
-    if (!done) atomicMin(&next_factor, my_factor);
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+      if (!done[r]) atomicMin(&next_factor, factor_of[r]);
     __syncthreads();
     const unsigned long long factor = next_factor;
     if (factor == ~0ull) break;
     {
-      // u_stage[j][t] = U[i1+j, i1+first(j)+t] with first(j) = j+2 for even j and j+1 for odd j (zero
-      // past the segment); then the diagonal and U[j, j+1]
       const float* src = reinterpret_cast<const float*>(factor) + i1 * k + i1;
-      for (int idx = threadIdx.x; idx < LMAX * LMAX / 4; idx += ROWS_PER_CTA)
-        u_stage4[idx] = zero4;
-      __syncthreads();
-      const int quads = len / 4;
-      for (int idx = threadIdx.x; idx < len * quads; idx += ROWS_PER_CTA) {
-        const int j = idx / quads, c = (idx % quads) * 4;
-        const int first = j + 2 - (j & 1);
-        if (c + 3 < first) continue;
-        const float4 v = *reinterpret_cast<const float4*>(src + j * k + c);
-        float* dst = u_stage + j * LMAX + (c - first);
-        if (c >= first) dst[0] = v.x;
-        if (c + 1 >= first) dst[1] = v.y;
-        if (c + 2 >= first) dst[2] = v.z;
-        dst[3] = v.w;
+      for (int idx = threadIdx.x; idx < len * 32; idx += BLOCK_THREADS) {
+        const int j = idx >> 5, c = (idx & 31) * 4, win = j / WIN, first = win * WIN;
+        if (c < first || c >= len) continue;
+        const float* from = src + (int64_t)j * k + c;
+        float* to = u + window_base(win) + (j - first) * (LMAX - first) + (c - first);
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(to)), "l"(from)
+                     : "memory");
       }
-      for (int idx = threadIdx.x; idx < 2 * LMAX; idx += ROWS_PER_CTA)
-        u_stage[U_DIAG + idx] = idx < len ? src[idx * k + idx] : 1.0f;
-      for (int idx = threadIdx.x; idx < LMAX; idx += ROWS_PER_CTA)
-        u_stage[U_NEXT + idx] = idx + 1 < len ? src[idx * k + idx + 1] : 0.0f;
+      for (int j = threadIdx.x; j < len; j += BLOCK_THREADS) {
+        const float ud = src[(int64_t)j * k + j];
+        const Recip rc = make_recip(ud);
+        reinterpret_cast<float2*>(gptq_smem + U_DIAG)[j] = make_float2(ud, rc.fast ? rc.r : __int_as_float(0x7fc00000));
+      }
     }
+    float4 w[R][QUADS];
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+      for (int m = 0; m < QUADS; ++m)
+        w[r][m] = WIN * m < len ? *reinterpret_cast<const float4*>(wc + row[r] * k + i1 + WIN * m + 4 * quad)
+                                : make_float4(0.f, 0.f, 0.f, 0.f);
+    // ladders of this lane's quad of window 0, and the block indices of window 1 behind them
+    float lo_n[R][4], st_n[R][4];
+    int4 blk_n[R] = {};
+    auto fetch_ladders = [&](int r) {
+      const float *l = lo + row[r] * ldp, *s = st + row[r] * ldp;
+      lo_n[r][0] = l[blk_n[r].x], lo_n[r][1] = l[blk_n[r].y], lo_n[r][2] = l[blk_n[r].z], lo_n[r][3] = l[blk_n[r].w];
+      st_n[r][0] = s[blk_n[r].x], st_n[r][1] = s[blk_n[r].y], st_n[r][2] = s[blk_n[r].z], st_n[r][3] = s[blk_n[r].w];
+    };
+    auto fetch_blocks = [&](int r, int win) {
+      blk_n[r] = *reinterpret_cast<const int4*>(blk + (int64_t)group[r] * k + i1 + WIN * min(win, windows - 1) + 4 * quad);
+    };
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      fetch_blocks(r, 0);
+      fetch_ladders(r);
+      fetch_blocks(r, 1);
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
-    if (!done && my_factor == factor) {
-      done = true;
-      float2 w[LMAX / 2];
+
+#pragma unroll 1
+    for (int win = 0; win < windows; ++win) {
+      // ---- the window's values and ladders for all four lanes
 #pragma unroll
-      for (int q = 0; q < LMAX / 4; ++q) {
-        const float4 v = (4 * q < len) ? *reinterpret_cast<const float4*>(wrow + 4 * q) : zero4;
-        w[2 * q] = make_float2(v.x, v.y), w[2 * q + 1] = make_float2(v.z, v.w);
-      }
-      RowState<WITH_COMP> s;
-      s.j = 0, s.qk = 0;
-      auto ladder = [&](int c) {
-        const int b = brow[min(c, last)];
-        Ladder p;
-        p.lo = lorow[b], p.st = strow[b];
-        return p;
-      };
+      for (int r = 0; r < R; ++r) {
+        float* lad = ladders + (row0 + 8 * r) * LADDER_STRIDE + 16 * quad;
 #pragma unroll
-      for (int c = 1; c <= 4; ++c) s.p[c & 3] = ladder(c), s.b[c & 3] = brow[min(c + 4, last)];
-      {  // column 0 opens the pipeline
-        float q0, e0;
-        round_column(w[0].x, ladder(0), u_stage[U_DIAG], nm, q0, e0);
-        s.ev[0] = e0, s.ev[1] = s.ev[2] = s.ev[3] = 0.0f;
-        s.cv[0] = w[0].x, s.cv[1] = s.cv[2] = s.cv[3] = 0.0f;
-        s.qk = (uint32_t)q0 << 24;
-        s.e = e0;
+        for (int t = 0; t < 4; ++t) {
+          const float s = st_n[r][t];
+          const Recip rc = make_recip(s == 0.0f ? 1.0f : s);
+          const float pivot = diag[WIN * win + 4 * quad + t].y;
+          const float z = rc.fast && pivot == pivot ? rc.r : __int_as_float(0x7fc00000);
+          *reinterpret_cast<float4*>(lad + 4 * t) = make_float4(lo_n[r][t], s, z, s == 0.0f ? 0.0f : nm[r]);
+        }
+        *reinterpret_cast<float4*>(const_cast<float*>(swap[r]) + 4 * quad) = w[r][0];
       }
-      run_phase<128, WITH_COMP>(w, s, len, nm, u_stage, brow, lorow, strow, live, err_row, code_row, comp_row);
-      run_phase<96, WITH_COMP>(w, s, len, nm, u_stage, brow, lorow, strow, live, err_row, code_row, comp_row);
-      run_phase<64, WITH_COMP>(w, s, len, nm, u_stage, brow, lorow, strow, live, err_row, code_row, comp_row);
-      run_phase<32, WITH_COMP>(w, s, len, nm, u_stage, brow, lorow, strow, live, err_row, code_row, comp_row);
+      __syncwarp();
+      float v[R][WIN];
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+#pragma unroll
+        for (int t = 0; t < WIN; t += 4) {
+          const float4 x = *reinterpret_cast<const float4*>(swap[r] + t);
+          v[r][t] = x.x, v[r][t + 1] = x.y, v[r][t + 2] = x.z, v[r][t + 3] = x.w;
+        }
+        if (win + 1 < windows) {  // loads for the next window, in flight during this one
+          fetch_ladders(r);
+          fetch_blocks(r, win + 2);
+        }
+      }
+      __syncwarp();  // the exchange floats take the errors from here on
+      const int width = LMAX - WIN * win;
+      const float* uw = u + window_base(win);
+      uint32_t code[R][4];
+      float seen[WITH_COMP ? R : 1][WITH_COMP ? WIN : 1];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        float e[R][4];
+#pragma unroll
+        for (int r = 0; r < R; ++r) code[r][q] = 0;
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+          const int j = 4 * q + t;
+          const float2 dj = diag[WIN * win + j];
+#pragma unroll
+          for (int r = 0; r < R; ++r) {
+            const float4 lad = *reinterpret_cast<const float4*>(ladders + (row0 + 8 * r) * LADDER_STRIDE + 4 * j);
+            float code_j;
+            if (WITH_COMP) seen[r][j] = v[r][j];
+            round_column(v[r][j], lad, dj, nm[r], code_j, e[r][t]);
+            code[r][q] |= (uint32_t)code_j << (8 * t);
+          }
+          const float* urow = uw + j * width;
+#pragma unroll
+          for (int c = (j + 1) & ~3; c < WIN; c += 4) {
+            const float4 x = *reinterpret_cast<const float4*>(urow + c);
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+              const float2 ne = make_float2(-e[r][t], -e[r][t]);
+              if (c > j) {
+                sub_scaled(v[r][c], v[r][c + 1], ne, x.x, x.y);
+                sub_scaled(v[r][c + 2], v[r][c + 3], ne, x.z, x.w);
+              } else {  // the quad of column j itself
+                if (c + 1 > j) v[r][c + 1] = v[r][c + 1] - e[r][t] * x.y;
+                if (c + 2 > j) v[r][c + 2] = v[r][c + 2] - e[r][t] * x.z;
+                v[r][c + 3] = v[r][c + 3] - e[r][t] * x.w;
+              }
+            }
+          }
+        }
+        if (quad == 0) {
+#pragma unroll
+          for (int r = 0; r < R; ++r)
+            *reinterpret_cast<float4*>(const_cast<float*>(swap[r]) + 4 * q) = make_float4(e[r][0], e[r][1], e[r][2], e[r][3]);
+        }
+      }
+      __syncwarp();
+      // ---- outputs: each lane stores its quad of the window
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        if (!live[r] || done[r] || factor_of[r] != factor) continue;
+        const int64_t at = WIN * win + 4 * quad;
+        const float4 e = *reinterpret_cast<const float4*>(swap[r] + 4 * quad);
+        if (SPLIT) {
+          float4 h, l;
+          tf32_parts(e.x, h.x, l.x), tf32_parts(e.y, h.y, l.y), tf32_parts(e.z, h.z, l.z), tf32_parts(e.w, h.w, l.w);
+          *reinterpret_cast<float4*>(err + row[r] * len + at) = h;
+          *reinterpret_cast<float4*>(err_lo + row[r] * len + at) = l;
+        } else {
+          *reinterpret_cast<float4*>(err + row[r] * len + at) = e;
+        }
+        const uint32_t c01 = quad & 1 ? code[r][1] : code[r][0], c23 = quad & 1 ? code[r][3] : code[r][2];
+        *reinterpret_cast<uint32_t*>(codes + row[r] * k + i1 + at) = quad & 2 ? c23 : c01;
+        if (WITH_COMP) {
+          float x[4];
+#pragma unroll
+          for (int t = 0; t < 4; ++t) {
+            const float x01 = quad & 1 ? seen[r][4 + t] : seen[r][t], x23 = quad & 1 ? seen[r][12 + t] : seen[r][8 + t];
+            x[t] = quad & 2 ? x23 : x01;
+          }
+          *reinterpret_cast<float4*>(comp + row[r] * k + i1 + at) = make_float4(x[0], x[1], x[2], x[3]);
+        }
+      }
+      // ---- the columns behind the window (up to one quad more than there are: it is never used)
+      const int behind = windows - 1 - win;
+      if (behind > 5) update_behind<R, 7>(w, uw, width, quad, swap);
+      else if (behind > 3) update_behind<R, 5>(w, uw, width, quad, swap);
+      else if (behind > 1) update_behind<R, 3>(w, uw, width, quad, swap);
+      else if (behind > 0) update_behind<R, 1>(w, uw, width, quad, swap);
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int m = 0; m + 1 < QUADS; ++m) w[r][m] = w[r][m + 1];
+      __syncwarp();  // the exchange floats are overwritten next
     }
+#pragma unroll
+    for (int r = 0; r < R; ++r) done[r] = done[r] || factor_of[r] == factor;
     __syncthreads();  // the staged block is replaced in the next round
   }
 }
 
-int launch_block(const float* wc, int64_t n_rows, int64_t k, int64_t i1, int len, float* err1,
+template <int R, bool WITH_COMP, bool SPLIT>
+int launch_block_as(const float* wc, int64_t n_rows, int64_t k, int64_t i1, int len, float* err, float* err_lo,
+                    uint8_t* codes, const float* lo, const float* st, int64_t ldp, const int32_t* row_grp,
+                    const int64_t* u_ptrs, const int32_t* blk, const float* nmax, float* comp, cudaStream_t stream) {
+  constexpr int rows = BLOCK_THREADS / GROUP_LANES * R;
+  constexpr int smem = (ROW_STAGE + rows * (LADDER_STRIDE + SWAP_STRIDE)) * (int)sizeof(float);
+  auto kernel = gptq_block_kernel<R, WITH_COMP, SPLIT>;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+    return fail(HI2_ERR_LAUNCH, "gptq_block: cannot reserve shared memory");
+  kernel<<<(unsigned)ceil_div(n_rows, (int64_t)rows), BLOCK_THREADS, smem, stream>>>(
+      wc, n_rows, k, i1, len, err, err_lo, codes, lo, st, ldp, row_grp, u_ptrs, blk, nmax, comp);
+  return check_launch("gptq_block");
+}
+
+// Rows per lane, by how many waves of thread blocks the rows make (four blocks of 32 rows per SM with one
+// row per lane, three blocks of 64 with two): a wave of pairs takes 4/3 of the time of a wave of
+// single rows.  Measured at K = 2048, one row / two rows per lane: 4096 rows 25 / 42 us, 16384 50 / 52,
+// 22016 74 / 64, 32768 89 / 96.
+bool two_rows_per_lane(int64_t n_rows) {
+  int device = 0, sms = 148;
+  cudaGetDevice(&device);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+  return 3 * ceil_div(n_rows, (int64_t)sms * 4 * 32) > 4 * ceil_div(n_rows, (int64_t)sms * 3 * 64);
+}
+
+// err_lo null: err receives the errors; else err and err_lo their TF32 parts.
+int launch_block(const float* wc, int64_t n_rows, int64_t k, int64_t i1, int len, float* err, float* err_lo,
                  uint8_t* codes, const float* lo, const float* st, int64_t ldp,
                  const int32_t* row_grp, const int64_t* u_ptrs, const int32_t* blk,
                  const float* nmax, float* comp, cudaStream_t stream) {
-  const unsigned grid = (unsigned)ceil_div(n_rows, ROWS_PER_CTA);
-  const int smem = U_STAGE_FLOATS * (int)sizeof(float);
-  if (cudaFuncSetAttribute(gptq_block_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
-      cudaFuncSetAttribute(gptq_block_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-    return fail(HI2_ERR_LAUNCH, "gptq_block: cannot reserve shared memory");
-  if (comp != nullptr)
-    gptq_block_kernel<true><<<grid, ROWS_PER_CTA, smem, stream>>>(wc, n_rows, k, i1, len, err1, codes, lo, st,
-                                                               ldp, row_grp, u_ptrs, blk, nmax, comp);
-  else
-    gptq_block_kernel<false><<<grid, ROWS_PER_CTA, smem, stream>>>(wc, n_rows, k, i1, len, err1, codes, lo, st,
-                                                                ldp, row_grp, u_ptrs, blk, nmax, comp);
-  return check_launch("gptq_block");
+#define HI2_GPTQ_BLOCK(RR, CC, SS)                                                                              \
+  return launch_block_as<RR, CC, SS>(wc, n_rows, k, i1, len, err, err_lo, codes, lo, st, ldp, row_grp, u_ptrs, blk, \
+                                     nmax, comp, stream)
+  const bool pair = two_rows_per_lane(n_rows);
+  if (comp != nullptr) {
+    if (err_lo != nullptr) {
+      if (pair) HI2_GPTQ_BLOCK(2, true, true);
+      HI2_GPTQ_BLOCK(1, true, true);
+    }
+    if (pair) HI2_GPTQ_BLOCK(2, true, false);
+    HI2_GPTQ_BLOCK(1, true, false);
+  }
+  if (err_lo != nullptr) {
+    if (pair) HI2_GPTQ_BLOCK(2, false, true);
+    HI2_GPTQ_BLOCK(1, false, true);
+  }
+  if (pair) HI2_GPTQ_BLOCK(2, false, false);
+  HI2_GPTQ_BLOCK(1, false, false);
+#undef HI2_GPTQ_BLOCK
+}
+
+// Consecutive rows with one factor: units of one tensor (its candidate groups), and of tensors that
+// read the same input, lie next to each other, and their trailing updates are one product.
+struct Span {
+  int64_t r0, r1, factor;
+};
+std::vector<Span> factor_spans(int n_units, const int64_t* unit_rows, const int64_t* unit_factor) {
+  std::vector<Span> spans;
+  for (int un = 0; un < n_units; ++un) {
+    const int64_t r0 = unit_rows[un], r1 = unit_rows[un + 1];
+    if (r1 <= r0) continue;
+    if (!spans.empty() && spans.back().factor == unit_factor[un] && spans.back().r1 == r0) spans.back().r1 = r1;
+    else spans.push_back({r0, r1, unit_factor[un]});
+  }
+  return spans;
 }
 
 int launch_lazy(float* wc, int64_t n_rows, int64_t k, int64_t i1, int64_t i2, const float* err1,
@@ -316,7 +446,7 @@ extern "C" int hi2_gptq_block(const float* wc, int64_t n_rows, int64_t k, int64_
   int rc = check_block_args(wc, n_rows, k, i1, len, err1, codes, lo, st, ldp, row_grp, u_ptrs, blk,
                             nmax, comp);
   if (rc != HI2_OK) return rc;
-  return launch_block(wc, n_rows, k, i1, len, err1, codes, lo, st, ldp, row_grp, u_ptrs, blk, nmax,
+  return launch_block(wc, n_rows, k, i1, len, err1, nullptr, codes, lo, st, ldp, row_grp, u_ptrs, blk, nmax,
                       comp, static_cast<cudaStream_t>(stream));
 }
 
@@ -340,6 +470,7 @@ extern "C" int hi2_gptq_round(float* wc, int64_t n_rows, int64_t k, float* err1,
   HI2_REQUIRE(unit_rows_host[0] == 0 && unit_rows_host[n_units] == n_rows,
               "gptq_round: units must cover the rows");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const std::vector<Span> spans = factor_spans(n_units, unit_rows_host, u_host);
   ChainGraph chain(s);  // the K/128 segments and their trailing updates as one graph launch
   auto enqueue = [&]() -> int {
     for (int64_t i1 = 0; i1 < k; i1 += LMAX) {
@@ -348,15 +479,13 @@ extern "C" int hi2_gptq_round(float* wc, int64_t n_rows, int64_t k, float* err1,
       int rc = check_block_args(wc, n_rows, k, i1, len, err1, codes, lo, st, ldp, row_grp, u_ptrs,
                                 blk, nmax, comp);
       if (rc != HI2_OK) return rc;
-      rc = launch_block(wc, n_rows, k, i1, len, err1, codes, lo, st, ldp, row_grp, u_ptrs, blk, nmax,
+      rc = launch_block(wc, n_rows, k, i1, len, err1, nullptr, codes, lo, st, ldp, row_grp, u_ptrs, blk, nmax,
                         comp, s);
       if (rc != HI2_OK) return rc;
       if (i2 == k) break;
-      for (int un = 0; un < n_units; ++un) {
-        const int64_t r0 = unit_rows_host[un], r1 = unit_rows_host[un + 1];
-        if (r1 <= r0) continue;
-        rc = launch_lazy(wc + r0 * k, r1 - r0, k, i1, i2, err1 + r0 * len,
-                         reinterpret_cast<const float*>(u_host[un]), s);
+      for (const Span& x : spans) {
+        rc = launch_lazy(wc + x.r0 * k, x.r1 - x.r0, k, i1, i2, err1 + x.r0 * len,
+                         reinterpret_cast<const float*>(x.factor), s);
         if (rc != HI2_OK) return rc;
       }
     }
@@ -394,6 +523,7 @@ extern "C" int hi2_gptq_round_tc(float* wc, int64_t n_rows, int64_t k, float* er
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   float* err_hi = err_split;
   float* err_lo = err_split + n_rows * LMAX;
+  const std::vector<Span> spans = factor_spans(n_units, unit_rows_host, u_split_host);
   ChainGraph chain(s);  // the K/128 segments and their trailing updates as one graph launch
   auto enqueue = [&]() -> int {
     if (cudaMemsetAsync(status, 0, sizeof(int32_t), s) != cudaSuccess)
@@ -404,17 +534,15 @@ extern "C" int hi2_gptq_round_tc(float* wc, int64_t n_rows, int64_t k, float* er
       int rc = check_block_args(wc, n_rows, k, i1, len, err1, codes, lo, st, ldp, row_grp, u_ptrs,
                                 blk, nmax, comp);
       if (rc != HI2_OK) return rc;
-      rc = launch_block(wc, n_rows, k, i1, len, err1, codes, lo, st, ldp, row_grp, u_ptrs, blk, nmax,
-                        comp, s);
+      // the block leaves its errors as the TF32 parts the trailing update takes
+      const bool last = i2 == k;  // a block shorter than 128 columns is always the last one
+      rc = launch_block(wc, n_rows, k, i1, len, last ? err1 : err_hi, last ? nullptr : err_lo, codes, lo, st, ldp,
+                        row_grp, u_ptrs, blk, nmax, comp, s);
       if (rc != HI2_OK) return rc;
-      if (i2 == k) break;  // a block shorter than 128 columns is always the last one
-      rc = launch_split_tf32(err1, err_hi, err_lo, n_rows * LMAX, s);
-      if (rc != HI2_OK) return rc;
-      for (int un = 0; un < n_units; ++un) {
-        const int64_t r0 = unit_rows_host[un], r1 = unit_rows_host[un + 1];
-        if (r1 <= r0) continue;
-        const float* u_hi = reinterpret_cast<const float*>(u_split_host[un]);
-        rc = launch_lazy_tc(wc + r0 * k, r1 - r0, k, i1, err_hi + r0 * LMAX, err_lo + r0 * LMAX, u_hi,
+      if (last) break;
+      for (const Span& x : spans) {
+        const float* u_hi = reinterpret_cast<const float*>(x.factor);
+        rc = launch_lazy_tc(wc + x.r0 * k, x.r1 - x.r0, k, i1, err_hi + x.r0 * LMAX, err_lo + x.r0 * LMAX, u_hi,
                             u_hi + k * k, reinterpret_cast<int*>(status), s);
         if (rc != HI2_OK) return rc;
       }

@@ -1,0 +1,95 @@
+"""The GPTQ block kernel where its mapping changes: block lengths of one to eight windows, one and
+two rows per lane, thread blocks whose rows read several factors, and launches shared by neighbouring
+units with one factor.  Same inputs, same arithmetic: everything is compared bit for bit."""
+
+import pytest
+import torch
+
+from helpers import gen
+
+pytestmark = pytest.mark.gpu
+
+
+def case(rows, k, groups, seed, nbits=(2, 4, 8)):
+    g = gen(seed)
+    wc = torch.randn(rows, k, generator=g) * 0.02
+    us = [torch.triu(torch.randn(k, k, generator=g) * 0.05) + torch.eye(k) * (0.5 + torch.rand(k, generator=g)) for _ in range(groups)]
+    us[0][3, 3] = 1.0 - 2.0**-24  # a pivot whose significand is all ones: no usable reciprocal
+    lo, st = -0.04 - 0.01 * torch.rand(rows, k // 16, generator=g), 0.005 + 0.02 * torch.rand(rows, k // 16, generator=g)
+    lo, st = lo.half().float(), st.half().float()
+    st[::7, 0] = 0.0
+    grp = torch.randint(0, groups, (rows,), generator=g).to(torch.int32)
+    blk = torch.stack([torch.randint(0, k // 16, (k,), generator=g) for _ in range(groups)]).to(torch.int32)
+    nmax = torch.tensor([2.0 ** nbits[i % len(nbits)] - 1 for i in range(groups)])
+    return wc, us, lo, st, grp, blk, nmax
+
+
+def column_loop(wc, us, lo, st, grp, blk, nmax, i1, length):
+    """The block one column at a time on the CPU, every operation rounded on its own."""
+    seg = wc[:, i1 : i1 + length].clone()
+    u = torch.stack(us)[grp.long()][:, i1 : i1 + length, i1 : i1 + length]
+    codes, err, comp = torch.zeros_like(seg), torch.zeros_like(seg), torch.zeros_like(seg)
+    rows = torch.arange(wc.shape[0])
+    for i in range(length):
+        b = blk[grp.long(), i1 + i].long()
+        l, s, col = lo[rows, b], st[rows, b], seg[:, i].clone()
+        q = torch.round((col - l) / torch.where(s == 0, 1.0, s)).clamp_min(0).minimum(nmax[grp.long()])
+        q = torch.where(s == 0, 0.0, q)
+        e = (col - (l + q * s).half().float()) / u[:, i, i]
+        seg[:, i + 1 :] -= e[:, None] * u[:, i, i + 1 :]
+        codes[:, i], err[:, i], comp[:, i] = q, e, col
+    return codes.to(torch.uint8), err, comp
+
+
+def block(args, i1, length, comp=True):
+    from hi2_b200 import gptq_kernel
+
+    wc, us, lo, st, grp, blk, nmax = args
+    dev = "cuda"
+    rows, k = wc.shape
+    u = [x.to(dev) for x in us]
+    codes = torch.zeros(rows, k, dtype=torch.uint8, device=dev)
+    err = torch.zeros(rows, length, device=dev)
+    seen = torch.zeros(rows, k, device=dev) if comp else None
+    gptq_kernel.gptq_block(wc.to(dev), i1, length, err, codes, lo.to(dev), st.to(dev), grp.to(dev),
+                           torch.tensor([x.data_ptr() for x in u], device=dev), blk.to(dev), nmax.to(dev), seen)
+    torch.cuda.synchronize()
+    return codes[:, i1 : i1 + length].cpu(), err.cpu(), seen[:, i1 : i1 + length].cpu() if comp else None
+
+
+@pytest.mark.parametrize("length", [16, 32, 48, 64, 80, 96, 112, 128])
+@pytest.mark.parametrize("rows,groups", [(1, 1), (31, 1), (33, 2), (200, 3)])
+def test_block_against_the_column_loop(length, rows, groups):
+    args = case(rows, 160, groups, 31 * length + rows)
+    codes, err, comp = column_loop(*args, 32, length)
+    got = block(args, 32, length)
+    assert torch.equal(got[0], codes) and torch.equal(got[1], err) and torch.equal(got[2], comp)
+    plain = block(args, 32, length, comp=False)
+    assert torch.equal(plain[0], codes) and torch.equal(plain[1], err)
+
+
+@pytest.mark.parametrize("rows", [18944, 18945, 19007, 28416, 28417])
+def test_rows_per_lane_do_not_change_anything(rows):
+    args = case(rows, 128, 2, rows)
+    whole = block(args, 0, 128)
+    for r0 in (0, 9000, rows - 1500):
+        part = slice(r0, r0 + 1500)
+        wc, us, lo, st, grp, blk, nmax = args
+        got = block((wc[part], us, lo[part], st[part], grp[part], blk, nmax), 0, 128)
+        for a, b in zip(whole, got):
+            assert torch.equal(a[part], b)
+
+
+@pytest.mark.parametrize("nbits", [(2, 4), (8, 8)])  # tensor-core and FMA trailing updates
+def test_units_of_one_factor_share_a_launch_and_nothing_else(nbits):
+    """Jobs with one factor next to each other give what each of them gives alone."""
+    from hi2_b200.hessian import GptqJob, encode_jobs_gptq
+
+    k = 640
+    w, us, *_ = case(700, k, 2, 5)
+    w, us, d = w.cuda(), [u.cuda() for u in us], torch.ones(k, device="cuda")
+    cuts = [(0, 130, 0, nbits[0]), (130, 131, 0, nbits[1]), (131, 400, 0, nbits[0]), (400, 533, 1, nbits[1]), (533, 700, 0, nbits[1])]
+    jobs = [GptqJob(w[a:b].contiguous(), d, us[f], nb, 32) for a, b, f, nb in cuts]
+    for job, got in zip(jobs, encode_jobs_gptq(jobs, "fast", comp=True)):
+        alone = encode_jobs_gptq([job], "fast", comp=True)[0]
+        assert torch.equal(got.codes, alone.codes) and torch.equal(got.comp, alone.comp) and torch.equal(got.params, alone.params)
