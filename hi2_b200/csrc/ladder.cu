@@ -1,10 +1,10 @@
 // Ladder search and row quantisation (hi2/encode.py:53-173, hi2/ladder_kernel.py:44-101).
 //
-// fit kernel   one thread per (row, block).  The 32 lanes of a warp take 32 consecutive ROWS of
-//              the same block, so the column weights d of the block are warp-uniform (one
-//              broadcast load serves the warp) and the block's weights stay in registers for the
-//              whole grid search and the least-squares refits.  The work is ~800 fp32
-//              instructions per weight (effort "normal") against 4 bytes read: ALU-bound.
+// fit kernel   one thread per (row, block), two for blocks of 64.  The lanes of a warp take consecutive
+//              ROWS of the same block, so the column weights d of the block are warp-uniform (staged
+//              in shared memory) and the block's weights stay in registers for the whole grid search
+//              and the least-squares refits.  The work is about 350 instructions per weight (effort
+//              "normal") against 4 bytes read: bound by the fp32 pipe (70 % busy at blocks of 32).
 // row kernel   one thread block per row: row-wide extrema of (lo, step), the three fp16 row
 //              constants, the parameter bytes, the decoded fp16 ladders, and optionally the
 //              nearest codes and the weighted error of the row.  One pass over the row: HBM-bound.
@@ -16,22 +16,7 @@ namespace {
 struct GridSpec {
   float v[8];
   int g;
-};
-
-// Codes are rint((x - lo) / safe) with an IEEE division in the reference.  Here one correctly
-// rounded reciprocal of `safe` serves the block and every quotient is finished with Markstein's
-// fused correction (div_by), which yields the correctly rounded quotient itself, so rint sees the
-// very number the division would give.  Divisors outside the range the correction covers
-// (rc.fast false: tiny, huge, or a significand of all ones) take true divisions.
-//
-// WIDE (blocks of 16 and 32): the column weights d and the differences x - lo of the current grid
-// row are kept in registers next to x, which removes one load and one subtraction per element
-// and pass; a block of 64 has no registers to spare for that.
-template <int B, bool WIDE>
-struct BlockRegs {
-  float x[B];
-  float d[WIDE ? B : 1];
-  float a[WIDE ? B : 1];  // x - lo of the current lo
+  float one;  // 1.0, as a kernel argument
 };
 
 // Block sums are formed in the order of torch's CPU reduction over a contiguous inner dimension
@@ -51,183 +36,311 @@ __device__ __forceinline__ float fold_lane(const float (&v)[B / 8]) {
   }
 }
 
-template <int B, bool WIDE>
-__device__ __forceinline__ float block_error(const BlockRegs<B, WIDE>& r, const float* __restrict__ dd,
-                                             bool a_valid, float lo, float step, float nmax) {
+// Codes are rint((x - lo) / safe) with an IEEE division in the reference.  Here one correctly
+// rounded reciprocal of `safe` serves the block and every quotient is finished with Markstein's
+// fused correction, which yields the correctly rounded quotient itself, so rint sees the very number
+// the division would give.  Steps outside the range the correction covers (rc.fast false: tiny, huge,
+// or a significand of all ones) and negative ones take true divisions.
+//
+// Everything else is done for two neighbouring columns per instruction (packed fp32 multiplies and
+// fused multiply-adds), since the search is bound by instruction issue: 12 instructions a pair where
+// the scalar form had 28.  A packed add would be contracted with the packed multiply that feeds it, and
+// the sum of a separately rounded product is what the reference has; so additions are written as
+// a * one + b with a `one` the compiler cannot see through, which rounds exactly like a + b.
+// Signs are turned so that one constant serves all: the block is kept as -x, the differences as
+// lo - x, never above zero (a code below zero becomes zero either way), and multiplied by -1 / step.
+// Rounding to an integer is one addition of 2^23, and the product of the integer with the step comes
+// out of the same fused multiply-add that takes the 2^23 off again (2^23 * step is exact).
+constexpr float SHIFT = 8388608.0f;
+
+__device__ __forceinline__ float2 both(float v) { return make_float2(v, v); }
+__device__ __forceinline__ float2 add2(float2 a, float2 b, float2 one) { return __ffma2_rn(a, one, b); }
+__device__ __forceinline__ float2 min2(float2 a, float b) { return make_float2(fminf(a.x, b), fminf(a.y, b)); }
+
+// The columns one thread keeps, as pairs of -x.  Blocks of 16 and 32 belong to one thread: pair 4 j + 2 h + i
+// holds columns 8 j + 4 h + 2 i and its right neighbour.  A block of 64 is shared by two neighbouring
+// lanes (one thread's registers hold the values but not the differences, and the unrolled code of 64
+// columns no longer fits the instruction cache): lane `half` keeps the columns with h = half, as pair
+// 2 j + i.
+template <int B>
+struct Block {
+  static constexpr bool SHARED = B == 64;
+  static constexpr int PAIRS = SHARED ? 16 : B / 2;
+  float2 nx[PAIRS];
+};
+
+// Column weights of a block: shared memory, or (tensors that read different inputs) global memory.
+template <bool GROUPED>
+__device__ __forceinline__ float4 weights4(const float* d) {
+  if (GROUPED) return __ldg(reinterpret_cast<const float4*>(d));
+  return *reinterpret_cast<const float4*>(d);
+}
+
+// One ladder prepared for the packed loop.
+struct Step {
+  float2 neg_r, safe, step, off;  // -1 / step, step, step, -2^23 step
+  bool fast;
+};
+__device__ __forceinline__ Step make_step(float step) {
+  Step s;
   const float safe = (step == 0.0f) ? 1.0f : step;
   const Recip rc = make_recip(safe);
-  float err = 0.0f;
-  if (rc.fast) {
+  s.fast = rc.fast && safe > 0.0f;
+  s.neg_r = both(-rc.r), s.safe = both(safe), s.step = both(step), s.off = both(-SHIFT * step);
+  return s;
+}
+// 2^23 + the code of two columns, an = min(lo - x, 0)
+__device__ __forceinline__ float2 shifted_codes(float2 an, const Step& s, float top, float2 one) {
+  const float2 q0 = __fmul2_rn(an, s.neg_r);
+  const float2 q = __ffma2_rn(__ffma2_rn(q0, s.safe, an), s.neg_r, q0);
+  return min2(add2(q, both(SHIFT), one), top);
+}
+// d * (x_hat - x)^2 of two columns
+__device__ __forceinline__ float2 weighted_square(float2 an, float2 nx, float2 d, const Step& s, float2 lo, float top,
+                                                  float2 one) {
+  const float2 rec = add2(__ffma2_rn(shifted_codes(an, s, top, one), s.step, s.off), lo, one);
+  const float2 diff = add2(rec, nx, one);
+  return __fmul2_rn(d, __fmul2_rn(diff, diff));
+}
+
+// N sums over the block in the reference's order; v(j, h, first pair, t) gives the terms of the two pairs
+// of one 128-bit load of the weights.  Lanes that share a block exchange the four partial sums of
+// their half, so all lanes of the warp have to call this together.
+template <int B, int N, typename F>
+__device__ __forceinline__ void block_sums(float (&out)[N], int half, float2 one, F&& v) {
+  if constexpr (Block<B>::SHARED) {
+    float2 s[2][N];
 #pragma unroll
-    for (int l = 0; l < 8; ++l) {
-      float v[B / 8];
+    for (int j = 0; j < 4; ++j) {
+      float2 t[2][N], far[2][N];
+      v(j, half, 2 * j, t);
+      v(j + 4, half, 2 * (j + 4), far);
 #pragma unroll
-      for (int j = 0; j < B / 8; ++j) {
-        const int t = 8 * j + l;
-        const float num = (WIDE && a_valid) ? r.a[t] : r.x[t] - lo;
-        const float q0 = num * rc.r;
-        float q = rintf(fmaf(fmaf(-q0, safe, num), rc.r, q0));
-        q = fminf(fmaxf(q, 0.0f), nmax);
-        const float diff = (lo + q * step) - r.x[t];
-        v[j] = (WIDE ? r.d[t] : __ldg(dd + t)) * (diff * diff);
-      }
-      const float s = fold_lane<B>(v);
-      err = (l == 0) ? s : err + s;
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+          t[i][k] = add2(t[i][k], far[i][k], one);
+          s[i][k] = j == 0 ? t[i][k] : add2(s[i][k], t[i][k], one);
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+      const float mine[4] = {s[0][k].x, s[0][k].y, s[1][k].x, s[1][k].y};
+      float other[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) other[i] = __shfl_xor_sync(0xffffffffu, mine[i], 1);
+      out[k] = half ? other[0] : mine[0];
+#pragma unroll
+      for (int i = 1; i < 4; ++i) out[k] = out[k] + (half ? other[i] : mine[i]);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) out[k] = out[k] + (half ? mine[i] : other[i]);
     }
   } else {
 #pragma unroll
-    for (int l = 0; l < 8; ++l) {
-      float v[B / 8];
+    for (int h = 0; h < 2; ++h) {
+      float2 s[2][N];
 #pragma unroll
       for (int j = 0; j < B / 8; ++j) {
-        const int t = 8 * j + l;
-        float q = rintf(__fdiv_rn(r.x[t] - lo, safe));
-        q = fminf(fmaxf(q, 0.0f), nmax);
-        const float diff = (lo + q * step) - r.x[t];
-        v[j] = (WIDE ? r.d[t] : __ldg(dd + t)) * (diff * diff);
+        float2 t[2][N];
+        v(j, h, 4 * j + 2 * h, t);
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+          for (int k = 0; k < N; ++k) s[i][k] = j == 0 ? t[i][k] : add2(s[i][k], t[i][k], one);
       }
-      const float s = fold_lane<B>(v);
-      err = (l == 0) ? s : err + s;
+#pragma unroll
+      for (int k = 0; k < N; ++k) {
+        out[k] = h == 0 ? s[0][k].x : out[k] + s[0][k].x;
+        out[k] = out[k] + s[0][k].y;
+        out[k] = out[k] + s[1][k].x;
+        out[k] = out[k] + s[1][k].y;
+      }
     }
+  }
+}
+
+// The error of one ladder with true divisions, for steps the packed loop does not cover.
+template <int B>
+__device__ __noinline__ float block_error_careful(const float* __restrict__ x, const float* d, float lo, float step,
+                                                  float nmax) {
+  const float safe = (step == 0.0f) ? 1.0f : step;
+  float err = 0.0f;
+#pragma unroll 1
+  for (int l = 0; l < 8; ++l) {
+    float v[B / 8];
+#pragma unroll
+    for (int j = 0; j < B / 8; ++j) {
+      const int t = 8 * j + l;
+      float q = rintf(__fdiv_rn(x[t] - lo, safe));
+      q = fminf(fmaxf(q, 0.0f), nmax);
+      const float diff = (lo + q * step) - x[t];
+      v[j] = d[t] * (diff * diff);
+    }
+    const float s = fold_lane<B>(v);
+    err = (l == 0) ? s : err + s;
   }
   return err;
 }
 
-// Two ladders with the same lo at once (two neighbouring points of a grid row): the differences
-// x - lo and the column weights are fetched once, and the two error sums are independent chains,
-// which doubles the instruction-level parallelism of the loop.  Each sum is formed exactly as
-// block_error forms it.
-template <int B, bool WIDE>
-__device__ __forceinline__ void block_error2(const BlockRegs<B, WIDE>& r, const float* __restrict__ dd, float lo,
-                                             float step_a, float step_b, float nmax, float& err_a, float& err_b) {
-  const float safe_a = (step_a == 0.0f) ? 1.0f : step_a, safe_b = (step_b == 0.0f) ? 1.0f : step_b;
-  const Recip ra = make_recip(safe_a), rb = make_recip(safe_b);
-  if (!(ra.fast && rb.fast)) {
-    err_a = block_error<B, WIDE>(r, dd, true, lo, step_a, nmax);
-    err_b = block_error<B, WIDE>(r, dd, true, lo, step_b, nmax);
-    return;
-  }
-  float ea = 0.0f, eb = 0.0f;
+// lo - x of a pair, never above zero
+__device__ __forceinline__ float2 below(float2 nx, float2 lo, float2 one) { return min2(add2(nx, lo, one), 0.0f); }
+
+// Error of one ladder.  `an` (HAVE_AN) holds the differences of this lo; x and d are the block's in
+// memory.
+template <int B, bool GROUPED, bool HAVE_AN>
+__device__ __forceinline__ float block_error_exact(const Block<B>& blk, const float2* an, const float* __restrict__ x,
+                                                   const float* d, int half, float lo, float step, float nmax, float2 one) {
+  const Step s = make_step(step);
+  const float2 lo2 = both(lo);
+  const float top = SHIFT + nmax;
+  float err[1];
+  block_sums<B, 1>(err, half, one, [&](int j, int h, int p, float2 (&t)[2][1]) {
+    const float4 dv = weights4<GROUPED>(d + 8 * j + 4 * h);
 #pragma unroll
-  for (int l = 0; l < 8; ++l) {
-    float va[B / 8], vb[B / 8];
-#pragma unroll
-    for (int j = 0; j < B / 8; ++j) {
-      const int t = 8 * j + l;
-      const float num = WIDE ? r.a[t] : r.x[t] - lo;
-      const float dt = WIDE ? r.d[t] : __ldg(dd + t);
-      const float qa0 = num * ra.r, qb0 = num * rb.r;
-      float qa = rintf(fmaf(fmaf(-qa0, safe_a, num), ra.r, qa0));
-      float qb = rintf(fmaf(fmaf(-qb0, safe_b, num), rb.r, qb0));
-      qa = fminf(fmaxf(qa, 0.0f), nmax);
-      qb = fminf(fmaxf(qb, 0.0f), nmax);
-      const float da = (lo + qa * step_a) - r.x[t], db = (lo + qb * step_b) - r.x[t];
-      va[j] = dt * (da * da);
-      vb[j] = dt * (db * db);
+    for (int i = 0; i < 2; ++i) {
+      const float2 a = HAVE_AN ? an[p + i] : below(blk.nx[p + i], lo2, one);
+      t[i][0] = weighted_square(a, blk.nx[p + i], i == 0 ? make_float2(dv.x, dv.y) : make_float2(dv.z, dv.w), s, lo2, top, one);
     }
-    const float sa = fold_lane<B>(va), sb = fold_lane<B>(vb);
-    ea = (l == 0) ? sa : ea + sa;
-    eb = (l == 0) ? sb : eb + sb;
-  }
-  err_a = ea, err_b = eb;
+  });
+  return s.fast ? err[0] : block_error_careful<B>(x, d, lo, step, nmax);
 }
 
-template <int B, bool WIDE>
-__global__ void __launch_bounds__(256, (B == 16 ? 3 : 2))
-fit_kernel(const float* __restrict__ w, int64_t ldw, const float* __restrict__ d,
+// The same with codes rint(num * (1 / step)), one instruction a pair instead of four, for ladders of at
+// most 16 levels.  The product can round to another integer than the quotient only where the column
+// lies within delta of the middle between two levels, that is where |x_hat - x| is within delta of
+// step / 2: the two quotients differ by 2^-23 of at most nmax - 1/2, and num, q * step, lo + q * step and
+// the difference were each rounded once, so delta = 2^-24 (5 nmax step + |lo|).  The squares the sum
+// needs anyway are compared with step^2 / 4 (their own rounding is in the sixth nmax * step below); a
+// block with such a column, about one in 500 warps and ladders at 4 levels and one in 100 at 16, is
+// done again exactly.  At 256 levels it would be one in eight, and the exact form is used at once.
+// 11008 x 4096, normal effort, 4 levels, blocks of 16 / 32 / 64, us: scalar form 914 / 862 / 973 us, packed
+// 790 / 710 / 742, this 713 / 670 / 709 (682 / 645 / 682 at 16 levels, 770 / 739 / 780 at 256).
+template <int B, bool GROUPED>
+__device__ __forceinline__ float block_error(const Block<B>& blk, const float2 (&an)[Block<B>::PAIRS],
+                                             const float* __restrict__ x, const float* d, int half, float lo, float step,
+                                             float nmax, float2 one) {
+  bool sure = nmax <= 15.0f && step > 1e-15f && step < 1e15f;
+  if (Block<B>::SHARED) sure = __all_sync(0xffffffffu, sure);
+  if (sure) {
+    const float2 lo2 = both(lo), neg_r = both(-__frcp_rn(step)), step2 = both(step), off = both(-SHIFT * step);
+    const float2 neg_mid = both(-((0.5f * step) * (0.5f * step)));
+    const float top = SHIFT + nmax;
+    float near = INFINITY;
+    float err[1];
+    block_sums<B, 1>(err, half, one, [&](int j, int h, int p, float2 (&t)[2][1]) {
+      const float4 dv = weights4<GROUPED>(d + 8 * j + 4 * h);
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const float2 c = min2(__ffma2_rn(an[p + i], neg_r, both(SHIFT)), top);
+        const float2 diff = add2(add2(__ffma2_rn(c, step2, off), lo2, one), blk.nx[p + i], one);
+        const float2 sq = __fmul2_rn(diff, diff);
+        const float2 mid = add2(sq, neg_mid, one);
+        near = fminf(fminf(near, fabsf(mid.x)), fabsf(mid.y));
+        t[i][0] = __fmul2_rn(i == 0 ? make_float2(dv.x, dv.y) : make_float2(dv.z, dv.w), sq);
+      }
+    });
+    sure = near > 6.3e-8f * step * (6.0f * nmax * step + fabsf(lo));
+    if (Block<B>::SHARED) sure = __all_sync(0xffffffffu, sure);
+    if (sure) return err[0];
+  }
+  return block_error_exact<B, GROUPED, true>(blk, an, x, d, half, lo, step, nmax, one);
+}
+
+constexpr int FIT_THREADS = 128, FIT_WARPS = FIT_THREADS / 32;
+
+template <int B, bool GROUPED>
+__global__ void __launch_bounds__(FIT_THREADS, (B == 16 ? 5 : 4))
+fit_kernel(const float* __restrict__ w, int64_t ldw, const float* __restrict__ d_all,
            const int32_t* __restrict__ row_d, int64_t n_rows, int64_t nb, GridSpec grid, int refits, float nmax, float* __restrict__ lo_out,
            float* __restrict__ st_out, float* __restrict__ err_out) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t blk = (int64_t)blockIdx.y * 8 + warp;
+  __shared__ __align__(16) float d_stage[FIT_WARPS][B];
+  constexpr bool SHARED = Block<B>::SHARED;
+  constexpr int PAIRS = Block<B>::PAIRS, ROWS = SHARED ? 16 : 32;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, half = SHARED ? lane & 1 : 0;
+  const int64_t blk = (int64_t)blockIdx.y * FIT_WARPS + warp;
   if (blk >= nb) return;  // uniform over the warp
-  const int64_t row = (int64_t)blockIdx.x * 32 + lane;
+  const int64_t row = (int64_t)blockIdx.x * ROWS + (SHARED ? lane >> 1 : lane);
   const bool live = row < n_rows;
   const int64_t row_c = live ? row : n_rows - 1;
   const float* src = w + row_c * ldw + blk * B;
-  // row_d given: d is [groups, k] and row r is weighted by d[row_d[r]] (tensors that read different
+  const float2 one = both(grid.one);
+  // GROUPED: d is [groups, k] and row r is weighted by d[row_d[r]] (tensors that read different
   // inputs, e.g. the experts of a layer, searched in one launch)
-  const float* dd = d + (row_d != nullptr ? (int64_t)row_d[row_c] * (nb * B) : 0) + blk * B;
-
-  BlockRegs<B, WIDE> r;
-#pragma unroll
-  for (int t = 0; t < B; t += 4) {
-    const float4 v = *reinterpret_cast<const float4*>(src + t);
-    r.x[t] = v.x, r.x[t + 1] = v.y, r.x[t + 2] = v.z, r.x[t + 3] = v.w;
-    if (WIDE) {
-      const float4 dv = __ldg(reinterpret_cast<const float4*>(dd + t));
-      r.d[t] = dv.x, r.d[t + 1] = dv.y, r.d[t + 2] = dv.z, r.d[t + 3] = dv.w;
-    }
+  const float* d;
+  if (GROUPED) {
+    d = d_all + (int64_t)row_d[row_c] * (nb * B) + blk * B;
+  } else {
+    for (int t = lane; t < B / 4; t += 32)
+      reinterpret_cast<float4*>(d_stage[warp])[t] = __ldg(reinterpret_cast<const float4*>(d_all + blk * B) + t);
+    __syncwarp();
+    d = d_stage[warp];
   }
-  float mn = r.x[0], mx = r.x[0];
+
+  Block<B> r;
+  float mn = 0.0f, mx = 0.0f;
 #pragma unroll
-  for (int t = 1; t < B; ++t) mn = fminf(mn, r.x[t]), mx = fmaxf(mx, r.x[t]);
+  for (int q = 0; q < PAIRS / 2; ++q) {
+    const float4 v = *reinterpret_cast<const float4*>(src + (SHARED ? 8 * q + 4 * half : 4 * q));
+    if (q == 0) mn = v.x, mx = v.x;
+    mn = fminf(fminf(fminf(fminf(mn, v.x), v.y), v.z), v.w), mx = fmaxf(fmaxf(fmaxf(fmaxf(mx, v.x), v.y), v.z), v.w);
+    r.nx[2 * q] = make_float2(-v.x, -v.y), r.nx[2 * q + 1] = make_float2(-v.z, -v.w);
+  }
+  if (SHARED) {
+    mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, 1));
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+  }
   const float span = mx - mn;
   const Recip rc_n = make_recip(nmax);  // nmax is 3, 15 or 255: div_by is the IEEE quotient
 
   float best_lo = 0.0f, best_st = 0.0f, best_err = 0.0f;
+#pragma unroll 1
   for (int gi = 0; gi < grid.g; ++gi) {
     const float lo = mn + grid.v[gi] * span;
-    if (WIDE) {
+    float2 an[PAIRS];
 #pragma unroll
-      for (int t = 0; t < B; ++t) r.a[t] = r.x[t] - lo;
-    }
-    int gj = 0;
-    // Blocks of 64 take two grid points per pass, in their order (6 % faster); the narrower blocks
-    // keep x - lo and d in registers and have none left for a second chain.
-    for (; !WIDE && gj + 1 < grid.g; gj += 2) {
-      const float step_a = div_by((mx - grid.v[gj] * span) - lo, nmax, rc_n);
-      const float step_b = div_by((mx - grid.v[gj + 1] * span) - lo, nmax, rc_n);
-      float err_a, err_b;
-      block_error2<B, WIDE>(r, dd, lo, step_a, step_b, nmax, err_a, err_b);
-      if ((gi | gj) == 0 || err_a < best_err) best_lo = lo, best_st = step_a, best_err = err_a;
-      if (err_b < best_err) best_lo = lo, best_st = step_b, best_err = err_b;
-    }
-    for (; gj < grid.g; ++gj) {
+    for (int p = 0; p < PAIRS; ++p) an[p] = below(r.nx[p], both(lo), one);
+#pragma unroll 1
+    for (int gj = 0; gj < grid.g; ++gj) {
       const float step = div_by((mx - grid.v[gj] * span) - lo, nmax, rc_n);
-      const float err = block_error<B, WIDE>(r, dd, true, lo, step, nmax);
+      const float err = block_error<B, GROUPED>(r, an, src, d, half, lo, step, nmax, one);
       if ((gi | gj) == 0 || err < best_err) best_lo = lo, best_st = step, best_err = err;
     }
   }
 
+#pragma unroll 1
   for (int it = 0; it < refits; ++it) {
-    const float safe = (best_st == 0.0f) ? 1.0f : best_st;
-    const Recip rc = make_recip(safe);
-    float sd = 0.f, sc = 0.f, scc = 0.f, sw = 0.f, scw = 0.f, sum = 0.f;
+    // sums over the block of d, d c, d c^2, -d x, -d c x and -x, c the code
+    float sums[6];
+    const Step s = make_step(best_st);
+    const float2 lo2 = both(best_lo);
+    const float top = SHIFT + nmax, safe = s.safe.x;
+    block_sums<B, 6>(sums, half, one, [&](int j, int h, int p, float2 (&t)[2][6]) {
+      const float4 dv = weights4<GROUPED>(d + 8 * j + 4 * h);
 #pragma unroll
-    for (int l = 0; l < 8; ++l) {
-      float vd[B / 8], vc[B / 8], vcc[B / 8], vw[B / 8], vcw[B / 8], vx[B / 8];
-#pragma unroll
-      for (int j = 0; j < B / 8; ++j) {
-        const int t = 8 * j + l;
-        const float num = r.x[t] - best_lo;
-        float c;
-        if (rc.fast) {
-          const float q0 = num * rc.r;
-          c = rintf(fmaf(fmaf(-q0, safe, num), rc.r, q0));
+      for (int i = 0; i < 2; ++i) {
+        const float2 nx = r.nx[p + i], dp = i == 0 ? make_float2(dv.x, dv.y) : make_float2(dv.z, dv.w);
+        float2 c;
+        if (s.fast) {
+          c = add2(shifted_codes(below(nx, lo2, one), s, top, one), both(-SHIFT), one);
         } else {
-          c = rintf(__fdiv_rn(num, safe));
+          c.x = fminf(fmaxf(rintf(__fdiv_rn(-nx.x - best_lo, safe)), 0.0f), nmax);
+          c.y = fminf(fmaxf(rintf(__fdiv_rn(-nx.y - best_lo, safe)), 0.0f), nmax);
         }
-        c = fminf(fmaxf(c, 0.0f), nmax);
-        const float dt = WIDE ? r.d[t] : __ldg(dd + t), dc = dt * c;
-        vd[j] = dt, vc[j] = dc, vcc[j] = dc * c, vw[j] = dt * r.x[t], vcw[j] = dc * r.x[t], vx[j] = r.x[t];
+        const float2 dc = __fmul2_rn(dp, c);
+        t[i][0] = dp, t[i][1] = dc, t[i][2] = __fmul2_rn(dc, c), t[i][3] = __fmul2_rn(dp, nx);
+        t[i][4] = __fmul2_rn(dc, nx), t[i][5] = nx;
       }
-      const float fd = fold_lane<B>(vd), fc = fold_lane<B>(vc), fcc = fold_lane<B>(vcc), fw = fold_lane<B>(vw),
-                  fcw = fold_lane<B>(vcw), fx = fold_lane<B>(vx);
-      if (l == 0) {
-        sd = fd, sc = fc, scc = fcc, sw = fw, scw = fcw, sum = fx;
-      } else {
-        sd += fd, sc += fc, scc += fcc, sw += fw, scw += fcw, sum += fx;
-      }
-    }
+    });
+    const float sd = sums[0], sc = sums[1], scc = sums[2], sw = -sums[3], scw = -sums[4], sum = -sums[5];
     const float det = sd * scc - sc * sc;
     const bool ok = fabsf(det) > 1e-20f;
     const float step = ok ? __fdiv_rn(sd * scw - sc * sw, det) : 0.0f;
     const float lo = ok ? __fdiv_rn(sw - step * sc, fmaxf(sd, 1e-20f)) : __fdiv_rn(sum, (float)B);
-    const float err = block_error<B, WIDE>(r, dd, false, lo, step, nmax);
+    const float err = block_error_exact<B, GROUPED, false>(r, nullptr, src, d, half, lo, step, nmax, one);
     if (err < best_err && step > 0.0f) best_lo = lo, best_st = step, best_err = err;
   }
 
-  if (live) {
+  if (live && half == 0) {
     const int64_t o = row * nb + blk;
     lo_out[o] = best_lo;
     st_out[o] = best_st;
@@ -239,12 +352,17 @@ int launch_fit(const float* w, int64_t ldw, const float* d, const int32_t* row_d
                int refits, int n, int64_t n_rows, int64_t nb, int block, float* lo, float* st,
                float* err, cudaStream_t stream) {
   GridSpec spec;
-  spec.g = g;
+  spec.g = g, spec.one = 1.0f;
   for (int i = 0; i < 8; ++i) spec.v[i] = i < g ? grid_host[i] : 0.0f;
-  dim3 grid((unsigned)ceil_div(n_rows, 32), (unsigned)ceil_div(nb, 8));
+  dim3 grid((unsigned)ceil_div(n_rows, block == 64 ? 16 : 32), (unsigned)ceil_div(nb, FIT_WARPS));
   const float nmax = (float)(n - 1);
-#define HI2_FIT(BB)                                                                              \
-  fit_kernel<BB, (BB <= 32)><<<grid, 256, 0, stream>>>(w, ldw, d, row_d, n_rows, nb, spec, refits, nmax, lo, st, err)
+#define HI2_FIT(BB)                                                                                              \
+  do {                                                                                                           \
+    if (row_d != nullptr)                                                                                        \
+      fit_kernel<BB, true><<<grid, FIT_THREADS, 0, stream>>>(w, ldw, d, row_d, n_rows, nb, spec, refits, nmax, lo, st, err); \
+    else                                                                                                         \
+      fit_kernel<BB, false><<<grid, FIT_THREADS, 0, stream>>>(w, ldw, d, row_d, n_rows, nb, spec, refits, nmax, lo, st, err); \
+  } while (0)
   if (block == 16) HI2_FIT(16);
   if (block == 32) HI2_FIT(32);
   if (block == 64) HI2_FIT(64);
