@@ -8,6 +8,7 @@
 // Trailing update: wc[:, i2:] -= err1 @ U[i1:i2, i2:], in fp32 FMA arithmetic (gemm.cuh) or as three
 // TF32 products (lazy_tc.cu); neighbouring units with one factor share a launch.
 #include "gemm.cuh"
+#include "row_window.cuh"
 
 #include <vector>
 
@@ -19,28 +20,7 @@ int launch_lazy_tc(float* wc, int64_t n_rows, int64_t k, int64_t i1, const float
 
 namespace {
 
-constexpr int LMAX = 128;
-constexpr int WIN = 16;           // columns rounded between two updates of the columns behind them
-constexpr int GROUP_LANES = 4;    // lanes that share a row
-constexpr int BLOCK_THREADS = 128;
-// Shared memory: the factor block as windows of 16 rows that start at their own first column, then
-// (U[j, j], its reciprocal) per column, then per row the ladders of the window's columns and 16
-// exchange floats (row strides of 4 and 20 banks: a 128-bit access of eight rows meets every bank once).
-constexpr int U_FLOATS = WIN * (LMAX / WIN) * (LMAX + WIN) / 2;
-constexpr int U_DIAG = U_FLOATS;
-constexpr int ROW_STAGE = U_DIAG + 2 * LMAX;
-constexpr int LADDER_STRIDE = 4 * WIN + 4, SWAP_STRIDE = WIN + 4;
-__host__ __device__ constexpr int window_base(int win) { return WIN * (LMAX * win - (WIN / 2) * win * (win - 1)); }
-static_assert(window_base(LMAX / WIN) == U_FLOATS, "the windows fill the factor stage");
-
-// (w0, w1) - e * (u0, u1) with the product and the difference rounded separately.  The product is one
-// packed multiply; the two additions stay scalar on purpose: a packed multiply feeding a packed
-// add is contracted into a packed FMA by the assembler even with contraction switched off, and
-// a fused update no longer gives the codes of the reference's separately rounded one.
-__device__ __forceinline__ void sub_scaled(float& w0, float& w1, float2 neg_e, float u0, float u1) {
-  const float2 p = __fmul2_rn(neg_e, make_float2(u0, u1));
-  w0 += p.x, w1 += p.y;
-}
+using namespace row_window;
 
 // Code and scaled error of one column (hi2/gptq_kernel.py:88-101) with true divisions.
 __device__ __noinline__ float2 round_careful(float col, float lo, float st, float ud, float nm) {
@@ -75,53 +55,8 @@ __device__ __forceinline__ void round_column(float col, float4 ladder, float2 di
   }
 }
 
-__device__ __forceinline__ void tf32_parts(float x, float& hi, float& lo) {
-  uint32_t hb, lb;
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(hb) : "f"(x));
-  hi = __uint_as_float(hb);
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(lb) : "f"(x - hi));
-  lo = __uint_as_float(lb);
-}
-
-// The M quads a lane holds behind the window lose the window's sixteen errors, in column order.
-template <int R, int M>
-__device__ __forceinline__ void update_behind(float4 (&w)[R][LMAX / WIN], const float* u, int width, int quad,
-                                              const float* const (&swap)[R]) {
-#pragma unroll 1
-  for (int j = 0; j < WIN; j += 4) {
-    float4 e[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) e[r] = *reinterpret_cast<const float4*>(swap[r] + j);
-#pragma unroll
-    for (int t = 0; t < 4; ++t) {
-      const float* row = u + (j + t) * width + 4 * quad;
-#pragma unroll
-      for (int m = 1; m <= M; ++m) {
-        const float4 v = *reinterpret_cast<const float4*>(row + WIN * m);
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          const float x = t == 0 ? e[r].x : t == 1 ? e[r].y : t == 2 ? e[r].z : e[r].w;
-          const float2 ne = make_float2(-x, -x);
-          sub_scaled(w[r][m].x, w[r][m].y, ne, v.x, v.y);
-          sub_scaled(w[r][m].z, w[r][m].w, ne, v.z, v.w);
-        }
-      }
-    }
-  }
-}
-
-// One lazy block: up to 128 columns of every row, rounded column by column.
-//
-// Four lanes share a row.  The block is taken in windows of 16 columns.  The window's values are kept by
-// all four lanes and every lane rounds its columns and applies their errors inside the window, so the
-// chain from one column to the next carries no exchange between lanes; the columns behind the window
-// are dealt out to the lanes in quads (lane h holds columns 16 m + 4 h .. + 3 of every later window)
-// and lose the window's sixteen errors afterwards, in column order, so every element sees the
-// operations of the column-by-column loop in their order.  After a window the quads move down by one
-// and every register index stays static.  Ladders, their reciprocals and the pivots' are prepared by the
-// lane that owns the column, a window ahead, and wait in shared memory; the factor block is staged
-// there once per thread block.  R rows per lane share the reads of the factor and give R independent
-// chains: R = 2 where the rows still fill the SMs, 1 below.
+// One lazy block: up to 128 columns of every row, rounded column by column, in the mapping of
+// row_window.cuh.  The prepared values of a column are its ladder and the ladder's reciprocal.
 // What bounds it: few rows, the chain (about 110 cycles a column); many rows, shared-memory reads of the
 // factor.  One lane per row with the 128 columns in its registers was bound by the chain at every size
 // and left most SMs idle at a few thousand rows; a block, lane per row -> this: 256 rows 79 -> 25 us,
@@ -138,13 +73,12 @@ gptq_block_kernel(const float* __restrict__ wc, int64_t n_rows, int64_t k, int64
                   float* __restrict__ comp) {
   extern __shared__ __align__(16) float gptq_smem[];
   __shared__ unsigned long long next_factor;
-  constexpr int QUADS = LMAX / WIN;
   const int lane = threadIdx.x & 31, quad = lane & 3;
   const int row0 = (threadIdx.x >> 5) * 8 * R + (lane >> 2);  // this lane's rows of the block: row0 + 8 r
   float* u = gptq_smem;
   const float2* diag = reinterpret_cast<const float2*>(gptq_smem + U_DIAG);
   float* ladders = gptq_smem + ROW_STAGE;
-  float* swaps = ladders + (BLOCK_THREADS / GROUP_LANES) * R * LADDER_STRIDE;
+  float* swaps = ladders + rows_per_block<R>() * COLUMN_STRIDE;
   const int windows = len / WIN;
 
   int64_t row[R];
@@ -155,7 +89,7 @@ gptq_block_kernel(const float* __restrict__ wc, int64_t n_rows, int64_t k, int64
   const float* swap[R];
 #pragma unroll
   for (int r = 0; r < R; ++r) {
-    const int64_t raw = (int64_t)blockIdx.x * (BLOCK_THREADS / GROUP_LANES * R) + row0 + 8 * r;
+    const int64_t raw = (int64_t)blockIdx.x * rows_per_block<R>() + row0 + 8 * r;
     live[r] = raw < n_rows;
     row[r] = live[r] ? raw : n_rows - 1;  // spare lanes shadow the last row and store nothing
     group[r] = row_grp[row[r]];
@@ -176,14 +110,7 @@ gptq_block_kernel(const float* __restrict__ wc, int64_t n_rows, int64_t k, int64
     if (factor == ~0ull) break;
     {
       const float* src = reinterpret_cast<const float*>(factor) + i1 * k + i1;
-      for (int idx = threadIdx.x; idx < len * 32; idx += BLOCK_THREADS) {
-        const int j = idx >> 5, c = (idx & 31) * 4, win = j / WIN, first = win * WIN;
-        if (c < first || c >= len) continue;
-        const float* from = src + (int64_t)j * k + c;
-        float* to = u + window_base(win) + (j - first) * (LMAX - first) + (c - first);
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(to)), "l"(from)
-                     : "memory");
-      }
+      stage_block(u, src, k, len);
       for (int j = threadIdx.x; j < len; j += BLOCK_THREADS) {
         const float ud = src[(int64_t)j * k + j];
         const Recip rc = make_recip(ud);
@@ -222,7 +149,7 @@ gptq_block_kernel(const float* __restrict__ wc, int64_t n_rows, int64_t k, int64
       // ---- the window's values and ladders for all four lanes
 #pragma unroll
       for (int r = 0; r < R; ++r) {
-        float* lad = ladders + (row0 + 8 * r) * LADDER_STRIDE + 16 * quad;
+        float* lad = ladders + (row0 + 8 * r) * COLUMN_STRIDE + 16 * quad;
 #pragma unroll
         for (int t = 0; t < 4; ++t) {
           const float s = st_n[r][t];
@@ -263,29 +190,16 @@ gptq_block_kernel(const float* __restrict__ wc, int64_t n_rows, int64_t k, int64
           const float2 dj = diag[WIN * win + j];
 #pragma unroll
           for (int r = 0; r < R; ++r) {
-            const float4 lad = *reinterpret_cast<const float4*>(ladders + (row0 + 8 * r) * LADDER_STRIDE + 4 * j);
+            const float4 lad = *reinterpret_cast<const float4*>(ladders + (row0 + 8 * r) * COLUMN_STRIDE + 4 * j);
             float code_j;
             if (WITH_COMP) seen[r][j] = v[r][j];
             round_column(v[r][j], lad, dj, nm[r], code_j, e[r][t]);
             code[r][q] |= (uint32_t)code_j << (8 * t);
           }
-          const float* urow = uw + j * width;
+          float f[R];
 #pragma unroll
-          for (int c = (j + 1) & ~3; c < WIN; c += 4) {
-            const float4 x = *reinterpret_cast<const float4*>(urow + c);
-#pragma unroll
-            for (int r = 0; r < R; ++r) {
-              const float2 ne = make_float2(-e[r][t], -e[r][t]);
-              if (c > j) {
-                sub_scaled(v[r][c], v[r][c + 1], ne, x.x, x.y);
-                sub_scaled(v[r][c + 2], v[r][c + 3], ne, x.z, x.w);
-              } else {  // the quad of column j itself
-                if (c + 1 > j) v[r][c + 1] = v[r][c + 1] - e[r][t] * x.y;
-                if (c + 2 > j) v[r][c + 2] = v[r][c + 2] - e[r][t] * x.z;
-                v[r][c + 3] = v[r][c + 3] - e[r][t] * x.w;
-              }
-            }
-          }
+          for (int r = 0; r < R; ++r) f[r] = -e[r][t];
+          update_window<R>(v, f, j, uw + j * width);
         }
         if (quad == 0) {
 #pragma unroll
@@ -300,14 +214,7 @@ gptq_block_kernel(const float* __restrict__ wc, int64_t n_rows, int64_t k, int64
         if (!live[r] || done[r] || factor_of[r] != factor) continue;
         const int64_t at = WIN * win + 4 * quad;
         const float4 e = *reinterpret_cast<const float4*>(swap[r] + 4 * quad);
-        if (SPLIT) {
-          float4 h, l;
-          tf32_parts(e.x, h.x, l.x), tf32_parts(e.y, h.y, l.y), tf32_parts(e.z, h.z, l.z), tf32_parts(e.w, h.w, l.w);
-          *reinterpret_cast<float4*>(err + row[r] * len + at) = h;
-          *reinterpret_cast<float4*>(err_lo + row[r] * len + at) = l;
-        } else {
-          *reinterpret_cast<float4*>(err + row[r] * len + at) = e;
-        }
+        store_factors(err + row[r] * len + at, SPLIT ? err_lo + row[r] * len + at : nullptr, e);
         const uint32_t c01 = quad & 1 ? code[r][1] : code[r][0], c23 = quad & 1 ? code[r][3] : code[r][2];
         *reinterpret_cast<uint32_t*>(codes + row[r] * k + i1 + at) = quad & 2 ? c23 : c01;
         if (WITH_COMP) {
@@ -320,16 +227,7 @@ gptq_block_kernel(const float* __restrict__ wc, int64_t n_rows, int64_t k, int64
           *reinterpret_cast<float4*>(comp + row[r] * k + i1 + at) = make_float4(x[0], x[1], x[2], x[3]);
         }
       }
-      // ---- the columns behind the window (up to one quad more than there are: it is never used)
-      const int behind = windows - 1 - win;
-      if (behind > 5) update_behind<R, 7>(w, uw, width, quad, swap);
-      else if (behind > 3) update_behind<R, 5>(w, uw, width, quad, swap);
-      else if (behind > 1) update_behind<R, 3>(w, uw, width, quad, swap);
-      else if (behind > 0) update_behind<R, 1>(w, uw, width, quad, swap);
-#pragma unroll
-      for (int r = 0; r < R; ++r)
-#pragma unroll
-        for (int m = 0; m + 1 < QUADS; ++m) w[r][m] = w[r][m + 1];
+      update_behind<R, true>(w, uw, width, quad, swap, windows - 1 - win);
       __syncwarp();  // the exchange floats are overwritten next
     }
 #pragma unroll
@@ -342,25 +240,13 @@ template <int R, bool WITH_COMP, bool SPLIT>
 int launch_block_as(const float* wc, int64_t n_rows, int64_t k, int64_t i1, int len, float* err, float* err_lo,
                     uint8_t* codes, const float* lo, const float* st, int64_t ldp, const int32_t* row_grp,
                     const int64_t* u_ptrs, const int32_t* blk, const float* nmax, float* comp, cudaStream_t stream) {
-  constexpr int rows = BLOCK_THREADS / GROUP_LANES * R;
-  constexpr int smem = (ROW_STAGE + rows * (LADDER_STRIDE + SWAP_STRIDE)) * (int)sizeof(float);
+  constexpr int rows = rows_per_block<R>(), smem = smem_bytes<R>();
   auto kernel = gptq_block_kernel<R, WITH_COMP, SPLIT>;
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
     return fail(HI2_ERR_LAUNCH, "gptq_block: cannot reserve shared memory");
   kernel<<<(unsigned)ceil_div(n_rows, (int64_t)rows), BLOCK_THREADS, smem, stream>>>(
       wc, n_rows, k, i1, len, err, err_lo, codes, lo, st, ldp, row_grp, u_ptrs, blk, nmax, comp);
   return check_launch("gptq_block");
-}
-
-// Rows per lane, by how many waves of thread blocks the rows make (four blocks of 32 rows per SM with one
-// row per lane, three blocks of 64 with two): a wave of pairs takes 4/3 of the time of a wave of
-// single rows.  Measured at K = 2048, one row / two rows per lane: 4096 rows 25 / 42 us, 16384 50 / 52,
-// 22016 74 / 64, 32768 89 / 96.
-bool two_rows_per_lane(int64_t n_rows) {
-  int device = 0, sms = 148;
-  cudaGetDevice(&device);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-  return 3 * ceil_div(n_rows, (int64_t)sms * 4 * 32) > 4 * ceil_div(n_rows, (int64_t)sms * 3 * 64);
 }
 
 // err_lo null: err receives the errors; else err and err_lo their TF32 parts.
