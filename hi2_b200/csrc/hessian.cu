@@ -29,6 +29,7 @@
 #include <mutex>
 
 #include "gemm.cuh"
+#include "moment_reduce.cuh"
 
 namespace hi2 {
 
@@ -351,25 +352,10 @@ hessian_tc_kernel(const __grid_constant__ CUtensorMap map, const TcParams p) {
   }
 }
 
-// S[i][j] += sum over splits (ascending) of the item tiles, for i <= j; S[j][i] = S[i][j].
-__global__ void __launch_bounds__(256)
-hessian_reduce_kernel(const float* __restrict__ scratch, int splits, int tiles, int njb, int64_t k,
-                      float* __restrict__ s, const int* __restrict__ status) {
-  // a product that gave up on a bounded wait left stale or partial tiles: S stays as it was and the
-  // caller sees the status word
-  if (*status != 0) return;
-  const int64_t j = (int64_t)blockIdx.x * 256 + threadIdx.x;
-  const int64_t i = blockIdx.y;
-  if (j >= k || j < i) return;
-  const int ib = (int)(i / BM), jb = (int)(j / BN);
-  const int tile = tile_slot(ib, jb, njb);
-  const size_t off = (size_t)tile * TILE_ELEMS + (size_t)(i % BM) * BN + (size_t)(j % BN);
-  float sum = 0.0f;
-  for (int sp = 0; sp < splits; ++sp) sum += scratch[(size_t)sp * tiles * TILE_ELEMS + off];
-  const float v = s[i * k + j] + sum;
-  s[i * k + j] = v;
-  if (i != j) s[j * k + i] = v;
-}
+struct TileSlot {
+  int njb;
+  __device__ __forceinline__ int operator()(int ib, int jb) const { return tile_slot(ib, jb, njb); }
+};
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
                                   const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
@@ -468,9 +454,8 @@ int accumulate_tc(const void* x, int dtype, int64_t tokens, int64_t k, float* s,
   hessian_tc_kernel<<<grid, TC_THREADS, TC_SMEM, stream>>>(map, p);
   int rc = check_launch("hessian_accumulate (tcgen05)");
   if (rc != HI2_OK) return rc;
-  dim3 rgrid((unsigned)ceil_div(k, 256), (unsigned)k);
-  hessian_reduce_kernel<<<rgrid, 256, 0, stream>>>(scratch, pl.splits, pl.tiles, pl.njb, k, s, status);
-  return check_launch("hessian_accumulate (reduce)");
+  return launch_moment_reduce<BM, BN>(scratch, pl.splits, pl.tiles, k, s, status, TileSlot{pl.njb}, stream,
+                                      "hessian_accumulate (reduce)");
 }
 
 template <typename TX>
@@ -621,8 +606,6 @@ extern "C" int hi2_hessian_accumulate_noalloc(const void* x, int dtype, int64_t 
   hessian_tc_kernel<<<items < sms ? items : sms, TC_THREADS, TC_SMEM, st>>>(map, p);
   int rc = check_launch("hessian_accumulate_noalloc (tcgen05)");
   if (rc != HI2_OK) return rc;
-  dim3 rgrid((unsigned)ceil_div(k, 256), (unsigned)k);
-  hessian_reduce_kernel<<<rgrid, 256, 0, st>>>(tiles, pl.splits, pl.tiles, pl.njb, k, s,
-                                               reinterpret_cast<const int*>(status));
-  return check_launch("hessian_accumulate_noalloc (reduce)");
+  return launch_moment_reduce<BM, BN>(tiles, pl.splits, pl.tiles, k, s, reinterpret_cast<const int*>(status),
+                                      TileSlot{pl.njb}, st, "hessian_accumulate_noalloc (reduce)");
 }

@@ -19,6 +19,7 @@
 #include <cuda.h>
 
 #include "common.cuh"
+#include "moment_reduce.cuh"
 
 namespace hi2 {
 namespace {
@@ -321,24 +322,10 @@ hessian_pair_kernel(const __grid_constant__ CUtensorMap map, const Params p) {
   }
 }
 
-// S[i][j] += sum over splits (ascending) of the item tiles, for i <= j; S[j][i] = S[i][j].
-__global__ void __launch_bounds__(256)
-pair_reduce_kernel(const float* __restrict__ scratch, int splits, int tiles, int nb, int64_t k,
-                   float* __restrict__ s, const int* __restrict__ status) {
-  // a product that gave up on a bounded wait left stale or partial tiles: S stays as it was and the
-  // caller sees the status word
-  if (*status != 0) return;
-  const int64_t j = (int64_t)blockIdx.x * 256 + threadIdx.x;
-  const int64_t i = blockIdx.y;
-  if (j >= k || j < i) return;
-  const int tile = tile_slot((int)(i / T2), (int)(j / T2), nb);
-  const size_t off = (size_t)tile * TILE_ELEMS + (size_t)(i % T2) * T2 + (size_t)(j % T2);
-  float sum = 0.0f;
-  for (int sp = 0; sp < splits; ++sp) sum += scratch[(size_t)sp * tiles * TILE_ELEMS + off];
-  const float v = s[i * k + j] + sum;
-  s[i * k + j] = v;
-  if (i != j) s[j * k + i] = v;
-}
+struct TileSlot {
+  int nb;
+  __device__ __forceinline__ int operator()(int i, int j) const { return tile_slot(i, j, nb); }
+};
 
 typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                              const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
@@ -433,9 +420,8 @@ int accumulate_pair(const void* x, int dtype, int64_t tokens, int64_t k, float* 
   hessian_pair_kernel<<<grid, THREADS, SMEM, stream>>>(map, p);
   int rc = check_launch("hessian_accumulate (tcgen05 pair)");
   if (rc != HI2_OK) return rc;
-  dim3 rgrid((unsigned)ceil_div(k, (int64_t)256), (unsigned)k);
-  pair_reduce_kernel<<<rgrid, 256, 0, stream>>>(scratch, pl.splits, pl.tiles, pl.nb, k, s, status);
-  return check_launch("hessian_accumulate (reduce)");
+  return launch_moment_reduce<T2, T2>(scratch, pl.splits, pl.tiles, k, s, status, TileSlot{pl.nb}, stream,
+                                      "hessian_accumulate (reduce)");
 }
 
 }  // namespace hi2
