@@ -53,6 +53,10 @@ SIGNATURES = {
         _I,
         [_P, _L, _L, _P, _P, _P, _P, _P, _L, _P, _P, _P, _P, _P, _I, _P, _P, _P, _P],
     ),
+    "hi2_gptq_round_tc_grouped": (
+        _I,
+        [_P, _L, _L, _P, _L, _P, _P, _P, _L, _P, _P, _P, _P, _P, _I, _P, _P, _P, _P],
+    ),
     "hi2_gptq_lazy_update_tc": (_I, [_P, _L, _L, _L, _P, _P, _P, _P]),
     "hi2_split_tf32_transposed": (_I, [_P, _P, _P, _L, _L, _P]),
     "hi2_split_tf32": (_I, [_P, _P, _P, _L, _P]),

@@ -14,9 +14,13 @@
 
 namespace hi2 {
 
-int launch_lazy_tc(float* wc, int64_t n_rows, int64_t k, int64_t i1, const float* err_hi,
-                   const float* err_lo, const float* u_hi, const float* u_lo, int* status,
+// lazy_tc.cu
+int launch_lazy_tc(float* wc, int64_t n_rows, int64_t k, int64_t i1, int64_t col_end, const float* err_hi,
+                   const float* err_lo, int64_t lde, const float* u_hi, const float* u_lo, int* status,
                    cudaStream_t stream);
+int launch_lazy_group(float* wc, int64_t n_rows, int64_t k, int64_t i1, int blocks, const float* err_hi,
+                      const float* err_lo, int64_t lde, const float* u_hi, const float* u_lo, int* status,
+                      cudaStream_t stream);
 
 namespace {
 
@@ -66,7 +70,7 @@ __device__ __forceinline__ void round_column(float col, float4 ladder, float2 di
 template <int R, bool WITH_COMP, bool SPLIT>
 __global__ void __launch_bounds__(BLOCK_THREADS, (R == 1 ? 4 : 3))
 gptq_block_kernel(const float* __restrict__ wc, int64_t n_rows, int64_t k, int64_t i1, int len,
-                  float* __restrict__ err, float* __restrict__ err_lo, uint8_t* __restrict__ codes,
+                  float* __restrict__ err, float* __restrict__ err_lo, int64_t lde, uint8_t* __restrict__ codes,
                   const float* __restrict__ lo, const float* __restrict__ st, int64_t ldp,
                   const int32_t* __restrict__ row_grp, const int64_t* __restrict__ u_ptrs,
                   const int32_t* __restrict__ blk, const float* __restrict__ nmax,
@@ -214,7 +218,7 @@ gptq_block_kernel(const float* __restrict__ wc, int64_t n_rows, int64_t k, int64
         if (!live[r] || done[r] || factor_of[r] != factor) continue;
         const int64_t at = WIN * win + 4 * quad;
         const float4 e = *reinterpret_cast<const float4*>(swap[r] + 4 * quad);
-        store_factors(err + row[r] * len + at, SPLIT ? err_lo + row[r] * len + at : nullptr, e);
+        store_factors(err + row[r] * lde + at, SPLIT ? err_lo + row[r] * lde + at : nullptr, e);
         const uint32_t c01 = quad & 1 ? code[r][1] : code[r][0], c23 = quad & 1 ? code[r][3] : code[r][2];
         *reinterpret_cast<uint32_t*>(codes + row[r] * k + i1 + at) = quad & 2 ? c23 : c01;
         if (WITH_COMP) {
@@ -238,24 +242,24 @@ gptq_block_kernel(const float* __restrict__ wc, int64_t n_rows, int64_t k, int64
 
 template <int R, bool WITH_COMP, bool SPLIT>
 int launch_block_as(const float* wc, int64_t n_rows, int64_t k, int64_t i1, int len, float* err, float* err_lo,
-                    uint8_t* codes, const float* lo, const float* st, int64_t ldp, const int32_t* row_grp,
+                    int64_t lde, uint8_t* codes, const float* lo, const float* st, int64_t ldp, const int32_t* row_grp,
                     const int64_t* u_ptrs, const int32_t* blk, const float* nmax, float* comp, cudaStream_t stream) {
   constexpr int rows = rows_per_block<R>(), smem = smem_bytes<R>();
   auto kernel = gptq_block_kernel<R, WITH_COMP, SPLIT>;
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
     return fail(HI2_ERR_LAUNCH, "gptq_block: cannot reserve shared memory");
   kernel<<<(unsigned)ceil_div(n_rows, (int64_t)rows), BLOCK_THREADS, smem, stream>>>(
-      wc, n_rows, k, i1, len, err, err_lo, codes, lo, st, ldp, row_grp, u_ptrs, blk, nmax, comp);
+      wc, n_rows, k, i1, len, err, err_lo, lde, codes, lo, st, ldp, row_grp, u_ptrs, blk, nmax, comp);
   return check_launch("gptq_block");
 }
 
-// err_lo null: err receives the errors; else err and err_lo their TF32 parts.
+// err_lo null: err (leading dimension lde) receives the errors; else err and err_lo their TF32 parts.
 int launch_block(const float* wc, int64_t n_rows, int64_t k, int64_t i1, int len, float* err, float* err_lo,
-                 uint8_t* codes, const float* lo, const float* st, int64_t ldp,
+                 int64_t lde, uint8_t* codes, const float* lo, const float* st, int64_t ldp,
                  const int32_t* row_grp, const int64_t* u_ptrs, const int32_t* blk,
                  const float* nmax, float* comp, cudaStream_t stream) {
 #define HI2_GPTQ_BLOCK(RR, CC, SS)                                                                              \
-  return launch_block_as<RR, CC, SS>(wc, n_rows, k, i1, len, err, err_lo, codes, lo, st, ldp, row_grp, u_ptrs, blk, \
+  return launch_block_as<RR, CC, SS>(wc, n_rows, k, i1, len, err, err_lo, lde, codes, lo, st, ldp, row_grp, u_ptrs, blk, \
                                      nmax, comp, stream)
   const bool pair = two_rows_per_lane(n_rows);
   if (comp != nullptr) {
@@ -332,7 +336,7 @@ extern "C" int hi2_gptq_block(const float* wc, int64_t n_rows, int64_t k, int64_
   int rc = check_block_args(wc, n_rows, k, i1, len, err1, codes, lo, st, ldp, row_grp, u_ptrs, blk,
                             nmax, comp);
   if (rc != HI2_OK) return rc;
-  return launch_block(wc, n_rows, k, i1, len, err1, nullptr, codes, lo, st, ldp, row_grp, u_ptrs, blk, nmax,
+  return launch_block(wc, n_rows, k, i1, len, err1, nullptr, len, codes, lo, st, ldp, row_grp, u_ptrs, blk, nmax,
                       comp, static_cast<cudaStream_t>(stream));
 }
 
@@ -365,7 +369,7 @@ extern "C" int hi2_gptq_round(float* wc, int64_t n_rows, int64_t k, float* err1,
       int rc = check_block_args(wc, n_rows, k, i1, len, err1, codes, lo, st, ldp, row_grp, u_ptrs,
                                 blk, nmax, comp);
       if (rc != HI2_OK) return rc;
-      rc = launch_block(wc, n_rows, k, i1, len, err1, nullptr, codes, lo, st, ldp, row_grp, u_ptrs, blk, nmax,
+      rc = launch_block(wc, n_rows, k, i1, len, err1, nullptr, len, codes, lo, st, ldp, row_grp, u_ptrs, blk, nmax,
                         comp, s);
       if (rc != HI2_OK) return rc;
       if (i2 == k) break;
@@ -389,8 +393,68 @@ extern "C" int hi2_gptq_lazy_update_tc(float* wc, int64_t n_rows, int64_t k, int
   if (n_rows == 0 || i1 + LMAX == k) return HI2_OK;
   HI2_REQUIRE(wc && err_split && u_split && status, "gptq_lazy_update_tc: null pointer");
   HI2_REQUIRE(aligned16(wc) && aligned16(err_split) && aligned16(u_split), "gptq_lazy_update_tc: alignment");
-  return launch_lazy_tc(wc, n_rows, k, i1, err_split, err_split + n_rows * LMAX, u_split, u_split + k * k,
+  return launch_lazy_tc(wc, n_rows, k, i1, k, err_split, err_split + n_rows * LMAX, LMAX, u_split, u_split + k * k,
                         reinterpret_cast<int*>(status), static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int hi2_gptq_round_tc_grouped(float* wc, int64_t n_rows, int64_t k, float* err_split, int64_t err_columns,
+                                         uint8_t* codes, const float* lo, const float* st, int64_t ldp,
+                                         const int32_t* row_grp, const int64_t* u_ptrs, const int32_t* blk,
+                                         const float* nmax, float* comp, int n_units,
+                                         const int64_t* unit_rows_host, const int64_t* u_split_host,
+                                         int32_t* status, void* stream) {
+  using namespace hi2;
+  if (n_rows == 0) return HI2_OK;
+  HI2_REQUIRE(n_units >= 1 && unit_rows_host && u_split_host, "gptq_round_tc: unit table missing");
+  HI2_REQUIRE(unit_rows_host[0] == 0 && unit_rows_host[n_units] == n_rows,
+              "gptq_round_tc: units must cover the rows");
+  HI2_REQUIRE(err_split && status && aligned16(err_split), "gptq_round_tc: scratch missing or unaligned");
+  HI2_REQUIRE(k % 4 == 0, "gptq_round_tc: k must be a multiple of 4");
+  HI2_REQUIRE(err_columns >= LMAX && err_columns % LMAX == 0, "gptq_round_tc: err_columns must be a multiple of 128");
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  float* err_hi = err_split;
+  float* err_lo = err_split + n_rows * err_columns;
+  int* word = reinterpret_cast<int*>(status);
+  const std::vector<Span> spans = factor_spans(n_units, unit_rows_host, u_split_host);
+  ChainGraph chain(s);  // the K/128 segments and their trailing updates as one graph launch
+  auto enqueue = [&]() -> int {
+    if (cudaMemsetAsync(status, 0, sizeof(int32_t), s) != cudaSuccess)
+      return fail(HI2_ERR_LAUNCH, "gptq_round_tc: memset failed");
+    for (int64_t g0 = 0; g0 < k; g0 += err_columns) {
+      const int64_t g1 = (g0 + err_columns < k) ? g0 + err_columns : k;
+      for (int64_t i1 = g0; i1 < g1; i1 += LMAX) {
+        const int64_t i2 = (i1 + LMAX < k) ? i1 + LMAX : k;
+        const int len = (int)(i2 - i1);
+        float *eh = err_hi + (i1 - g0), *el = err_lo + (i1 - g0);
+        int rc = check_block_args(wc, n_rows, k, i1, len, eh, codes, lo, st, ldp, row_grp, u_ptrs, blk, nmax, comp);
+        if (rc != HI2_OK) return rc;
+        // the block leaves its errors as the TF32 parts the trailing updates take
+        rc = launch_block(wc, n_rows, k, i1, len, eh, el, err_columns, codes, lo, st, ldp, row_grp, u_ptrs, blk, nmax,
+                          comp, s);
+        if (rc != HI2_OK) return rc;
+        if (i2 >= g1) break;  // a block shorter than 128 columns is always the last one
+        for (const Span& x : spans) {  // the rest of the group needs this block's errors now
+          const float* u_hi = reinterpret_cast<const float*>(x.factor);
+          rc = launch_lazy_tc(wc + x.r0 * k, x.r1 - x.r0, k, i1, g1, eh + x.r0 * err_columns, el + x.r0 * err_columns,
+                              err_columns, u_hi, u_hi + k * k, word, s);
+          if (rc != HI2_OK) return rc;
+        }
+      }
+      if (g1 == k) break;
+      for (const Span& x : spans) {  // the columns behind it take all of its blocks in one pass
+        const float* u_hi = reinterpret_cast<const float*>(x.factor);
+        const float *eh = err_hi + x.r0 * err_columns, *el = err_lo + x.r0 * err_columns;
+        const int blocks = (int)(err_columns / LMAX);
+        int rc = blocks == 1 ? launch_lazy_tc(wc + x.r0 * k, x.r1 - x.r0, k, g0, k, eh, el, err_columns, u_hi,
+                                              u_hi + k * k, word, s)
+                             : launch_lazy_group(wc + x.r0 * k, x.r1 - x.r0, k, g0, blocks, eh, el, err_columns, u_hi,
+                                                 u_hi + k * k, word, s);
+        if (rc != HI2_OK) return rc;
+      }
+    }
+    return HI2_OK;
+  };
+  return chain.finish(enqueue(), "gptq_round_tc");
 }
 
 extern "C" int hi2_gptq_round_tc(float* wc, int64_t n_rows, int64_t k, float* err1, float* err_split,
@@ -399,43 +463,9 @@ extern "C" int hi2_gptq_round_tc(float* wc, int64_t n_rows, int64_t k, float* er
                                  const float* nmax, float* comp, int n_units,
                                  const int64_t* unit_rows_host, const int64_t* u_split_host,
                                  int32_t* status, void* stream) {
-  using namespace hi2;
-  if (n_rows == 0) return HI2_OK;
-  HI2_REQUIRE(n_units >= 1 && unit_rows_host && u_split_host, "gptq_round_tc: unit table missing");
-  HI2_REQUIRE(unit_rows_host[0] == 0 && unit_rows_host[n_units] == n_rows,
-              "gptq_round_tc: units must cover the rows");
-  HI2_REQUIRE(err_split && status && aligned16(err_split), "gptq_round_tc: scratch missing or unaligned");
-  HI2_REQUIRE(k % 4 == 0, "gptq_round_tc: k must be a multiple of 4");
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  float* err_hi = err_split;
-  float* err_lo = err_split + n_rows * LMAX;
-  const std::vector<Span> spans = factor_spans(n_units, unit_rows_host, u_split_host);
-  ChainGraph chain(s);  // the K/128 segments and their trailing updates as one graph launch
-  auto enqueue = [&]() -> int {
-    if (cudaMemsetAsync(status, 0, sizeof(int32_t), s) != cudaSuccess)
-      return fail(HI2_ERR_LAUNCH, "gptq_round_tc: memset failed");
-    for (int64_t i1 = 0; i1 < k; i1 += LMAX) {
-      const int64_t i2 = (i1 + LMAX < k) ? i1 + LMAX : k;
-      const int len = (int)(i2 - i1);
-      int rc = check_block_args(wc, n_rows, k, i1, len, err1, codes, lo, st, ldp, row_grp, u_ptrs,
-                                blk, nmax, comp);
-      if (rc != HI2_OK) return rc;
-      // the block leaves its errors as the TF32 parts the trailing update takes
-      const bool last = i2 == k;  // a block shorter than 128 columns is always the last one
-      rc = launch_block(wc, n_rows, k, i1, len, last ? err1 : err_hi, last ? nullptr : err_lo, codes, lo, st, ldp,
-                        row_grp, u_ptrs, blk, nmax, comp, s);
-      if (rc != HI2_OK) return rc;
-      if (last) break;
-      for (const Span& x : spans) {
-        const float* u_hi = reinterpret_cast<const float*>(x.factor);
-        rc = launch_lazy_tc(wc + x.r0 * k, x.r1 - x.r0, k, i1, err_hi + x.r0 * LMAX, err_lo + x.r0 * LMAX, u_hi,
-                            u_hi + k * k, reinterpret_cast<int*>(status), s);
-        if (rc != HI2_OK) return rc;
-      }
-    }
-    return HI2_OK;
-  };
-  return chain.finish(enqueue(), "gptq_round_tc");
+  (void)err1;
+  return hi2_gptq_round_tc_grouped(wc, n_rows, k, err_split, hi2::row_window::LMAX, codes, lo, st, ldp, row_grp, u_ptrs, blk, nmax,
+                                   comp, n_units, unit_rows_host, u_split_host, status, stream);
 }
 
 extern "C" int hi2_gemm_f32(int trans_a, int trans_b, int64_t m, int64_t n, int64_t kk, float alpha,

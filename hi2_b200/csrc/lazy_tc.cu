@@ -80,6 +80,10 @@ __device__ __forceinline__ void tma_reduce_add(const CUtensorMap* map, const voi
       "cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3}], [%1];"
       ::"l"(reinterpret_cast<uint64_t>(map)), "r"(s32(src)), "r"(x), "r"(y) : "memory");
 }
+__device__ __forceinline__ void tma_store(const CUtensorMap* map, const void* src, int x, int y) {
+  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%2, %3}], [%1];"
+               ::"l"(reinterpret_cast<uint64_t>(map)), "r"(s32(src)), "r"(x), "r"(y) : "memory");
+}
 // K-major 128-byte-swizzled operand (rows of 128 B, 8-row groups 1024 B apart)
 __device__ __forceinline__ uint64_t desc_kmajor(uint32_t saddr) {
   uint64_t d = (uint64_t)((saddr & 0x3ffffu) >> 4);
@@ -452,6 +456,169 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_ahi, const __grid_constan
   }
 }
 
+// ------------------------------------------------------------------------------------------------
+// The trailing updates of several consecutive blocks of 128 columns in one pass over wc:
+//
+//     wc[:, i2:] = ((wc[:, i2:] - err_0 U_0) - err_1 U_1) - ...
+//
+// One update per block reads and writes all of wc behind the block: at 32768 x 4096 that is 1.07 GB for
+// 200 GFLOP, and memory was the bound (267 us, 375 TFLOP/s of TF32 products).  Here a tile of wc comes
+// into the registers of the eight epilogue warps once, every block's product (its own TMEM buffer, the
+// very operations of lazy_tc_kernel) is added to it round-to-nearest in the order of the blocks, and
+// the tile goes back once: the sums are the bits that one update after the other gives.  The columns
+// inside the group are brought up to date after each block by lazy_tc_kernel.
+// Updates of a column loop of 4096 x 11008, one by one -> groups of 512 columns: 3.90 -> 3.17 ms.
+struct QParams {
+  int* status;
+  float* wc;
+  int64_t n_rows, k;
+  int row_tiles, col_tiles;
+  int k0, col0;  // first reduction row of U, first output column
+  int blocks;
+};
+
+__global__ void __launch_bounds__(G_THREADS, 1)
+lazy_group_kernel(const __grid_constant__ CUtensorMap map_ahi, const __grid_constant__ CUtensorMap map_alo,
+                  const __grid_constant__ CUtensorMap map_bhi, const __grid_constant__ CUtensorMap map_blo,
+                  const __grid_constant__ CUtensorMap map_c, const QParams p) {
+  extern __shared__ uint8_t raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(raw) + 1023) & ~(uintptr_t)1023);
+  uint8_t* stage_c = smem + (size_t)LSTAGES * LSTAGE_BYTES;
+  LControl* ctl = reinterpret_cast<LControl*>(stage_c + 2 * C_BOX);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < LSTAGES; ++s) bar_init(&ctl->full[s], 1), bar_init(&ctl->empty[s], 1);
+    for (int b = 0; b < 2; ++b) bar_init(&ctl->acc_full[b], 1), bar_init(&ctl->acc_empty[b], 8);
+    ctl->abort = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 9) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s32(&ctl->tmem_base)), "r"(512) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  fence_before();
+  __syncthreads();
+  fence_after();
+  const uint32_t tmem_base = ctl->tmem_base;
+  const int tiles = p.row_tiles * p.col_tiles, stages = p.blocks * (LK / KSTAGE);
+
+  if (warp == 8 && lane == 0) {
+    // ------------------------------------------------------------ TMA producer
+    int stage = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
+      const int tr = tile % p.row_tiles, tc = tile / p.row_tiles;  // neighbours share the U tile
+      for (int ks = 0; ks < stages; ++ks) {
+        if (!(ok = bar_wait(&ctl->empty[stage], phase ^ 1, ctl, p.status))) break;
+        bar_expect(&ctl->full[stage], LSTAGE_BYTES);
+        uint8_t* dst = smem + (size_t)stage * LSTAGE_BYTES;
+        tma_load(dst, &map_ahi, &ctl->full[stage], ks * KSTAGE, tr * LM);
+        tma_load(dst + A_BOX, &map_alo, &ctl->full[stage], ks * KSTAGE, tr * LM);
+        tma_load(dst + 2 * A_BOX, &map_bhi, &ctl->full[stage], p.k0 + ks * KSTAGE, p.col0 + tc * LN);
+        tma_load(dst + 2 * A_BOX + B_PART, &map_blo, &ctl->full[stage], p.k0 + ks * KSTAGE, p.col0 + tc * LN);
+        if (++stage == LSTAGES) stage = 0, phase ^= 1;
+      }
+    }
+    if (!ok) {
+      const long long t0 = clock64();
+      while (clock64() - t0 < 2000000LL) {
+      }
+    }
+  } else if (warp == 9 && lane == 0) {
+    // ------------------------------------------------------------ MMA issuer
+    int stage = 0;
+    uint32_t phase = 0, n = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
+      for (int b = 0; b < p.blocks && ok; ++b, ++n) {
+        const int buf = n & 1;
+        if (!(ok = bar_wait(&ctl->acc_empty[buf], ((n >> 1) & 1) ^ 1, ctl, p.status))) break;
+        fence_after();
+        const uint32_t d_tmem = tmem_base + buf * LN;
+        for (int ks = 0; ks < LK / KSTAGE && ok; ++ks) {
+          if (!(ok = bar_wait(&ctl->full[stage], phase, ctl, p.status))) break;
+          fence_after();
+          const uint32_t sa = s32(smem + (size_t)stage * LSTAGE_BYTES);
+#pragma unroll
+          for (int kk = 0; kk < KSTAGE / 8; ++kk) {
+            const uint64_t ahi = desc_kmajor(sa + kk * 32), alo = desc_kmajor(sa + A_BOX + kk * 32);
+            const uint64_t bhi = desc_kmajor(sa + 2 * A_BOX + kk * 32);
+            const uint64_t blo = desc_kmajor(sa + 2 * A_BOX + B_PART + kk * 32);
+            mma_tf32(d_tmem, ahi, bhi, (ks > 0 || kk > 0) ? 1u : 0u);
+            mma_tf32(d_tmem, alo, bhi, 1u);
+            mma_tf32(d_tmem, ahi, blo, 1u);
+          }
+          commit_to(&ctl->empty[stage]);
+          if (++stage == LSTAGES) stage = 0, phase ^= 1;
+        }
+        if (ok) commit_to(&ctl->acc_full[buf]);
+      }
+    }
+  } else if (warp < 8) {
+    // ------------------------------------------------------------ epilogue
+    // Warp w owns tensor-memory lanes 32 (w mod 4) .. +31 (the rows of the tile) and columns
+    // 128 (w / 4) .. +127.
+    const int quarter = warp & 3, half = warp >> 2;
+    uint32_t n = 0;
+    bool ok = true;
+    uint8_t* box = stage_c + warp * (C_BOX / 4);  // one 32 x 32 staging box per warp
+    for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
+      const int tr = tile % p.row_tiles, tc = tile / p.row_tiles;
+      const int64_t row = (int64_t)tr * LM + quarter * 32 + lane, col = (int64_t)p.col0 + tc * LN + half * 128;
+      float acc[128];
+#pragma unroll
+      for (int i = 0; i < 128; i += 4) {
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (row < p.n_rows && col + i < p.k) v = *reinterpret_cast<const float4*>(p.wc + row * p.k + col + i);
+        acc[i] = v.x, acc[i + 1] = v.y, acc[i + 2] = v.z, acc[i + 3] = v.w;
+      }
+      for (int b = 0; b < p.blocks && ok; ++b, ++n) {
+        const int buf = n & 1;
+        if (!(ok = bar_wait(&ctl->acc_full[buf], (n >> 1) & 1, ctl, p.status))) break;
+        fence_after();
+        const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + buf * LN + half * 128;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          uint32_t v[32];
+          tmem_ld32(taddr + c * 32, v);
+#pragma unroll
+          for (int i = 0; i < 32; ++i) acc[c * 32 + i] += __uint_as_float(v[i]);
+        }
+        fence_before();
+        __syncwarp();
+        if (lane == 0) bar_arrive(&ctl->acc_empty[buf]);
+      }
+      if (!ok) break;
+      uint8_t* rowp = box + lane * 128;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // the box is free again
+        __syncwarp();
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+          *reinterpret_cast<float4*>(rowp + ((q ^ (lane & 7)) << 4)) =
+              make_float4(acc[c * 32 + 4 * q], acc[c * 32 + 4 * q + 1], acc[c * 32 + 4 * q + 2], acc[c * 32 + 4 * q + 3]);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) {
+          tma_store(&map_c, box, p.col0 + tc * LN + half * 128 + c * 32, tr * LM + quarter * 32);
+          asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+        }
+      }
+    }
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+  }
+
+  fence_before();
+  __syncthreads();
+  if (warp == 9) {
+    fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512) : "memory");
+  }
+}
+
 // TF32 parts of a [rows, cols] block with leading dimension ldx, written with leading dimension ldo.
 // lower: x is lower triangular and what lies above its diagonal is not read; its parts are zeros.
 __global__ void __launch_bounds__(256)
@@ -576,25 +743,25 @@ bool make_map(CUtensorMap* map, const float* base, int64_t inner, int64_t outer,
 
 }  // namespace
 
-// Used by gptq.cu.  err_hi/err_lo [n_rows, 128], ut_hi/ut_lo [k, k] = the TF32 parts of U^T,
-// wc [n_rows, k]; i2 = i1 + 128.
-int launch_lazy_tc(float* wc, int64_t n_rows, int64_t k, int64_t i1, const float* err_hi,
-                   const float* err_lo, const float* ut_hi, const float* ut_lo, int* status,
+// Used by gptq.cu.  wc[:, i2:col_end] -= err U[i1:i2, i2:col_end] with i2 = i1 + 128: err_hi/err_lo [n_rows, 128]
+// with leading dimension lde, ut_hi/ut_lo [k, k] the TF32 parts of U^T, wc [n_rows, k].
+int launch_lazy_tc(float* wc, int64_t n_rows, int64_t k, int64_t i1, int64_t col_end, const float* err_hi,
+                   const float* err_lo, int64_t lde, const float* ut_hi, const float* ut_lo, int* status,
                    cudaStream_t stream) {
   const int64_t i2 = i1 + LK;
-  if (n_rows <= 0 || i2 >= k) return HI2_OK;
+  if (n_rows <= 0 || i2 >= col_end) return HI2_OK;
   if (encoder() == nullptr) return fail(HI2_ERR_DRIVER, "gptq_lazy_update: cuTensorMapEncodeTiled unavailable");
   CUtensorMap mah, mal, mbh, mbl, mc;
-  if (!make_map(&mah, err_hi, LK, n_rows, LK, 32, LM) || !make_map(&mal, err_lo, LK, n_rows, LK, 32, LM) ||
+  if (!make_map(&mah, err_hi, LK, n_rows, lde, 32, LM) || !make_map(&mal, err_lo, LK, n_rows, lde, 32, LM) ||
       !make_map(&mbh, ut_hi, k, k, k, 32, LN) || !make_map(&mbl, ut_lo, k, k, k, 32, LN) ||
-      !make_map(&mc, wc, k, n_rows, k, 32, 32))
+      !make_map(&mc, wc, col_end, n_rows, k, 32, 32))  // boxes are clipped at col_end
     return fail(HI2_ERR_DRIVER, "gptq_lazy_update: cuTensorMapEncodeTiled failed");
   if (cudaFuncSetAttribute(lazy_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L_SMEM) != cudaSuccess)
     return fail(HI2_ERR_LAUNCH, "gptq_lazy_update: cannot reserve shared memory");
   LParams p;
   p.status = status;
   p.row_tiles = (int)ceil_div(n_rows, LM);
-  p.col_tiles = (int)ceil_div(k - i2, LN);
+  p.col_tiles = (int)ceil_div(col_end - i2, LN);
   p.k0 = (int)i1, p.col0 = (int)i2;
   const int tiles = p.row_tiles * p.col_tiles;
   int device = 0, sms = 148;
@@ -602,6 +769,34 @@ int launch_lazy_tc(float* wc, int64_t n_rows, int64_t k, int64_t i1, const float
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
   lazy_tc_kernel<<<tiles < sms ? tiles : sms, L_THREADS, L_SMEM, stream>>>(mah, mal, mbh, mbl, mc, p);
   return check_launch("gptq_lazy_update (tcgen05)");
+}
+
+// The updates of the `blocks` blocks of 128 columns that start at i1, for the columns behind all of them:
+// err_hi/err_lo [n_rows, 128 * blocks] with leading dimension lde.
+int launch_lazy_group(float* wc, int64_t n_rows, int64_t k, int64_t i1, int blocks, const float* err_hi,
+                      const float* err_lo, int64_t lde, const float* ut_hi, const float* ut_lo, int* status,
+                      cudaStream_t stream) {
+  const int64_t i2 = i1 + (int64_t)blocks * LK;
+  if (n_rows <= 0 || i2 >= k) return HI2_OK;
+  if (encoder() == nullptr) return fail(HI2_ERR_DRIVER, "gptq_lazy_update: cuTensorMapEncodeTiled unavailable");
+  CUtensorMap mah, mal, mbh, mbl, mc;
+  if (!make_map(&mah, err_hi, blocks * LK, n_rows, lde, 32, LM) || !make_map(&mal, err_lo, blocks * LK, n_rows, lde, 32, LM) ||
+      !make_map(&mbh, ut_hi, k, k, k, 32, LN) || !make_map(&mbl, ut_lo, k, k, k, 32, LN) ||
+      !make_map(&mc, wc, k, n_rows, k, 32, 32))
+    return fail(HI2_ERR_DRIVER, "gptq_lazy_update: cuTensorMapEncodeTiled failed");
+  if (cudaFuncSetAttribute(lazy_group_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L_SMEM) != cudaSuccess)
+    return fail(HI2_ERR_LAUNCH, "gptq_lazy_update: cannot reserve shared memory");
+  QParams p;
+  p.status = status, p.wc = wc, p.n_rows = n_rows, p.k = k;
+  p.row_tiles = (int)ceil_div(n_rows, LM);
+  p.col_tiles = (int)ceil_div(k - i2, LN);
+  p.k0 = (int)i1, p.col0 = (int)i2, p.blocks = blocks;
+  const int tiles = p.row_tiles * p.col_tiles;
+  int device = 0, sms = 148;
+  cudaGetDevice(&device);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+  lazy_group_kernel<<<tiles < sms ? tiles : sms, G_THREADS, L_SMEM, stream>>>(mah, mal, mbh, mbl, mc, p);
+  return check_launch("gptq_lazy_update group (tcgen05)");
 }
 
 // C[m, n] (ldc) = or += (+-) A . Bt^T with A = a_hi + a_lo [m, kk], Bt = b_hi + b_lo [n, kk], both with

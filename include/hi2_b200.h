@@ -153,6 +153,16 @@ int hi2_gptq_round_tc(float* wc, int64_t n_rows, int64_t k, float* err1, float* 
                       const float* nmax, float* comp, int n_units, const int64_t* unit_rows_host,
                       const int64_t* u_split_host, int32_t* status, void* stream);
 
+/* The same with the trailing updates of err_columns / 128 consecutive blocks taken together for the columns
+ * behind all of them (err_columns a multiple of 128): wc is read and written once per group instead of
+ * once per block, in the same order of additions, so the result is the same bits for every
+ * err_columns.  err_split is caller scratch [2, n_rows, err_columns]. */
+int hi2_gptq_round_tc_grouped(float* wc, int64_t n_rows, int64_t k, float* err_split, int64_t err_columns,
+                              uint8_t* codes, const float* lo, const float* st, int64_t ldp,
+                              const int32_t* row_grp, const int64_t* u_ptrs, const int32_t* blk,
+                              const float* nmax, float* comp, int n_units, const int64_t* unit_rows_host,
+                              const int64_t* u_split_host, int32_t* status, void* stream);
+
 /* One trailing update on the tensor cores: wc[:, i1+128:] -= err @ u[i1:i1+128, i1+128:] with
  * err_split [2, n_rows, 128] the TF32 parts of err and u_split [2, k, k] those of u^T.  *status is NOT
  * cleared here (the caller zeroes it once). */

@@ -93,3 +93,40 @@ def test_units_of_one_factor_share_a_launch_and_nothing_else(nbits):
     for job, got in zip(jobs, encode_jobs_gptq(jobs, "fast", comp=True)):
         alone = encode_jobs_gptq([job], "fast", comp=True)[0]
         assert torch.equal(got.codes, alone.codes) and torch.equal(got.comp, alone.comp) and torch.equal(got.params, alone.params)
+
+
+@pytest.mark.parametrize("k", [640, 1024, 1040, 1536, 2064])
+@pytest.mark.parametrize("rows", [40, 300])
+def test_updates_taken_together_are_the_updates_one_by_one(rows, k):
+    """One pass over the columns behind a group of blocks adds in the order of the blocks."""
+    from hi2_b200 import _lib
+    from hi2_b200.gptq_kernel import split_tf32_transposed
+
+    g = gen(rows + k)
+    u = [(torch.triu(torch.randn(k, k, generator=g) * 0.02) + torch.eye(k)).cuda() for _ in range(2)]
+    split = [split_tf32_transposed(x) for x in u]
+    cut = rows // 3
+    w = (torch.randn(rows, k, generator=g) * 0.02).cuda()
+    lo = (-0.04 - 0.01 * torch.rand(rows, k // 16, generator=g)).half().float().cuda()
+    st = (0.005 + 0.02 * torch.rand(rows, k // 16, generator=g)).half().float().cuda()
+    grp = (torch.arange(rows) >= cut).to(torch.int32).cuda()
+    ptrs = torch.tensor([x.data_ptr() for x in u]).cuda()
+    blk = (torch.arange(k) // 32).to(torch.int32).expand(2, k).contiguous().cuda()
+    nmax = torch.tensor([3.0, 15.0]).cuda()
+
+    def run(name, *scratch):
+        wc, codes, comp = w.clone(), torch.zeros(rows, k, dtype=torch.uint8, device="cuda"), torch.zeros(rows, k, device="cuda")
+        status = torch.zeros(1, dtype=torch.int32, device="cuda")
+        _lib.call(name, _lib.ptr(wc), rows, k, *scratch, _lib.ptr(codes), _lib.ptr(lo), _lib.ptr(st), k // 16, _lib.ptr(grp),
+                  _lib.ptr(ptrs), _lib.ptr(blk), _lib.ptr(nmax), _lib.ptr(comp), 2, _lib.host_i64([0, cut, rows]),
+                  _lib.host_i64([x.data_ptr() for x in split]), _lib.ptr(status), _lib.stream(w.device))
+        assert int(status.item()) == 0
+        return codes, comp, wc
+
+    one, parts = torch.empty(rows, 128, device="cuda"), torch.empty(2, rows, 128, device="cuda")
+    want = run("hi2_gptq_round_tc", _lib.ptr(one), _lib.ptr(parts))
+    for columns in (128, 256, 512, 1024):
+        scratch = torch.empty(2, rows, columns, device="cuda")
+        got = run("hi2_gptq_round_tc_grouped", _lib.ptr(scratch), columns)
+        for a, b in zip(got, want):
+            assert torch.equal(a, b)
