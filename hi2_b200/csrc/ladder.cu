@@ -214,7 +214,7 @@ __device__ __forceinline__ float block_error_exact(const Block<B>& blk, const fl
 // block with such a column, about one in 500 warps and ladders at 4 levels and one in 100 at 16, is
 // done again exactly.  At 256 levels it would be one in eight, and the exact form is used at once.
 // 11008 x 4096, normal effort, 4 levels, blocks of 16 / 32 / 64, us: scalar form 914 / 862 / 973 us, packed
-// 790 / 710 / 742, this 713 / 670 / 709 (682 / 645 / 682 at 16 levels, 770 / 739 / 780 at 256).
+// 790 / 710 / 742, this 713 / 670 / 709.
 template <int B, bool GROUPED>
 __device__ __forceinline__ float block_error(const Block<B>& blk, const float2 (&an)[Block<B>::PAIRS],
                                              const float* __restrict__ x, const float* d, int half, float lo, float step,
@@ -246,14 +246,37 @@ __device__ __forceinline__ float block_error(const Block<B>& blk, const float2 (
   return block_error_exact<B, GROUPED, true>(blk, an, x, d, half, lo, step, nmax, one);
 }
 
+// Sum over the block of d * (distance beyond `edge`)^2, on the side where lo - x > 0 (LOW) or < 0: what the
+// columns that a ladder ending at `edge` clips contribute to its error.  In any order: it serves as a
+// bound.
+template <int B, bool GROUPED, bool LOW>
+__device__ __forceinline__ float clipped_error(const Block<B>& blk, const float* d, int half, float edge, float2 one) {
+  const float2 e2 = both(edge);
+  float2 sum[2] = {both(0.0f), both(0.0f)};
+#pragma unroll
+  for (int g = 0; g < Block<B>::PAIRS / 2; ++g) {
+    const float4 dv = weights4<GROUPED>(d + (Block<B>::SHARED ? 8 * g + 4 * half : 4 * g));
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      float2 m = add2(blk.nx[2 * g + i], e2, one);
+      m = LOW ? make_float2(fmaxf(m.x, 0.0f), fmaxf(m.y, 0.0f)) : min2(m, 0.0f);
+      sum[i] = __ffma2_rn(__fmul2_rn(m, m), i == 0 ? make_float2(dv.x, dv.y) : make_float2(dv.z, dv.w), sum[i]);
+    }
+  }
+  float s = (sum[0].x + sum[0].y) + (sum[1].x + sum[1].y);
+  if (Block<B>::SHARED) s += __shfl_xor_sync(0xffffffffu, s, 1);
+  return s;
+}
+
 constexpr int FIT_THREADS = 128, FIT_WARPS = FIT_THREADS / 32;
 
-template <int B, bool GROUPED>
+template <int B, bool GROUPED, bool BOUND>
 __global__ void __launch_bounds__(FIT_THREADS, (B == 16 ? 5 : 4))
 fit_kernel(const float* __restrict__ w, int64_t ldw, const float* __restrict__ d_all,
            const int32_t* __restrict__ row_d, int64_t n_rows, int64_t nb, GridSpec grid, int refits, float nmax, float* __restrict__ lo_out,
            float* __restrict__ st_out, float* __restrict__ err_out) {
   __shared__ __align__(16) float d_stage[FIT_WARPS][B];
+  __shared__ float high_error[BOUND ? 8 : 1][FIT_THREADS];  // a thread's own, by grid point
   constexpr bool SHARED = Block<B>::SHARED;
   constexpr int PAIRS = Block<B>::PAIRS, ROWS = SHARED ? 16 : 32;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, half = SHARED ? lane & 1 : 0;
@@ -292,6 +315,29 @@ fit_kernel(const float* __restrict__ w, int64_t ldw, const float* __restrict__ d
   const float span = mx - mn;
   const Recip rc_n = make_recip(nmax);  // nmax is 3, 15 or 255: div_by is the IEEE quotient
 
+  // BOUND: a grid point clips the columns outside [lo, hi], hi = mx - v span, and they alone cost it the clipped
+  // errors at both ends.  Where those exceed the best error so far the point cannot win and is passed
+  // over: with 16 levels or more the steps are so fine that few grid points survive.  The codes of these
+  // columns are 0 and the highest; hi is moved out by 1e-6 of the block's range, more than the
+  // roundings that lie between it and the highest level, and 1e-4 covers those of the sums.
+  bool weights_ok = true;
+  const bool bound = BOUND && grid.g > 1;  // a single point has nothing to be measured against
+  if (bound) {
+    const float slack = 1e-6f * (fabsf(mn) + fabsf(mx));
+    float lowest = 0.0f;
+#pragma unroll
+    for (int g = 0; g < PAIRS / 2; ++g) {
+      const float4 dv = weights4<GROUPED>(d + (SHARED ? 8 * g + 4 * half : 4 * g));
+      lowest = fminf(lowest, fminf(fminf(dv.x, dv.y), fminf(dv.z, dv.w)));
+    }
+    if (SHARED) lowest = fminf(lowest, __shfl_xor_sync(0xffffffffu, lowest, 1));
+    weights_ok = lowest >= 0.0f;
+#pragma unroll 1
+    for (int gj = 0; gj < grid.g; ++gj)
+      high_error[gj][threadIdx.x] =
+          grid.v[gj] == 0.0f ? 0.0f : clipped_error<B, GROUPED, false>(r, d, half, (mx - grid.v[gj] * span) + slack, one);
+  }
+
   float best_lo = 0.0f, best_st = 0.0f, best_err = 0.0f;
 #pragma unroll 1
   for (int gi = 0; gi < grid.g; ++gi) {
@@ -299,9 +345,16 @@ fit_kernel(const float* __restrict__ w, int64_t ldw, const float* __restrict__ d
     float2 an[PAIRS];
 #pragma unroll
     for (int p = 0; p < PAIRS; ++p) an[p] = below(r.nx[p], both(lo), one);
+    float low_error = 0.0f;
+    if (bound && grid.v[gi] != 0.0f) low_error = clipped_error<B, GROUPED, true>(r, d, half, lo, one);
 #pragma unroll 1
     for (int gj = 0; gj < grid.g; ++gj) {
       const float step = div_by((mx - grid.v[gj] * span) - lo, nmax, rc_n);
+      if (bound && (gi | gj) != 0) {
+        bool beaten = weights_ok && step > 1e-15f && 0.9999f * (low_error + high_error[gj][threadIdx.x]) > best_err;
+        if (SHARED) beaten = __all_sync(0xffffffffu, beaten);
+        if (beaten) continue;
+      }
       const float err = block_error<B, GROUPED>(r, an, src, d, half, lo, step, nmax, one);
       if ((gi | gj) == 0 || err < best_err) best_lo = lo, best_st = step, best_err = err;
     }
@@ -353,20 +406,31 @@ int launch_fit(const float* w, int64_t ldw, const float* d, const int32_t* row_d
                float* err, cudaStream_t stream) {
   GridSpec spec;
   spec.g = g, spec.one = 1.0f;
-  for (int i = 0; i < 8; ++i) spec.v[i] = i < g ? grid_host[i] : 0.0f;
+  bool clips = true;  // every grid point moves an end of the ladder inwards, by half the range at most
+  for (int i = 0; i < 8; ++i) {
+    spec.v[i] = i < g ? grid_host[i] : 0.0f;
+    clips = clips && spec.v[i] >= 0.0f && spec.v[i] <= 0.5f;
+  }
   dim3 grid((unsigned)ceil_div(n_rows, block == 64 ? 16 : 32), (unsigned)ceil_div(nb, FIT_WARPS));
   const float nmax = (float)(n - 1);
-#define HI2_FIT(BB)                                                                                              \
-  do {                                                                                                           \
-    if (row_d != nullptr)                                                                                        \
-      fit_kernel<BB, true><<<grid, FIT_THREADS, 0, stream>>>(w, ldw, d, row_d, n_rows, nb, spec, refits, nmax, lo, st, err); \
-    else                                                                                                         \
-      fit_kernel<BB, false><<<grid, FIT_THREADS, 0, stream>>>(w, ldw, d, row_d, n_rows, nb, spec, refits, nmax, lo, st, err); \
+  // Passing over grid points that their clipped columns rule out: 11008 x 4096, normal effort, blocks of 16 /
+  // 32 / 64, us: 16 levels 682 / 645 / 682 -> 483 / 502 / 590, 256 levels 770 / 739 / 780 -> 360 / 295 / 301;
+  // at 4 levels next to nothing is ruled out and the bounds cost 6 %.
+  const bool bound = n >= 16 && clips;
+#define HI2_FIT_V(BB, GG, CC)                                                                                       \
+  fit_kernel<BB, GG, CC><<<grid, FIT_THREADS, 0, stream>>>(w, ldw, d, row_d, n_rows, nb, spec, refits, nmax, lo, st, err)
+#define HI2_FIT(BB)                                     \
+  do {                                                  \
+    if (row_d != nullptr && bound) HI2_FIT_V(BB, true, true);    \
+    else if (row_d != nullptr) HI2_FIT_V(BB, true, false);       \
+    else if (bound) HI2_FIT_V(BB, false, true);                  \
+    else HI2_FIT_V(BB, false, false);                            \
   } while (0)
   if (block == 16) HI2_FIT(16);
   if (block == 32) HI2_FIT(32);
   if (block == 64) HI2_FIT(64);
 #undef HI2_FIT
+#undef HI2_FIT_V
   return check_launch("fit_ladder");
 }
 
