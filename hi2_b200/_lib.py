@@ -53,6 +53,7 @@ SIGNATURES = {
         _I,
         [_P, _L, _L, _P, _P, _P, _P, _P, _L, _P, _P, _P, _P, _P, _I, _P, _P, _P, _P],
     ),
+    "hi2_error_table": (_I, [_P, _L, _P, _P, _P, _I, _I, _I, _P, _P, _L, _L, _P, _P, _P, _P, _P]),
     "hi2_gptq_round_tc_grouped": (
         _I,
         [_P, _L, _L, _P, _L, _P, _P, _P, _L, _P, _P, _P, _P, _P, _I, _P, _P, _P, _P],
@@ -215,3 +216,7 @@ def host_floats(values):
 
 def host_i64(values):
     return (C.c_int64 * len(values))(*[int(v) for v in values])
+
+
+def host_i32(values):
+    return (C.c_int32 * len(values))(*[int(v) for v in values])

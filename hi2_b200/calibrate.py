@@ -17,8 +17,9 @@ from dataclasses import dataclass, field
 import torch
 
 from . import _lib
-from .encode import encode_rows
+from .encode import EFFORT, encode_rows
 from .format import GROUP, HI2Tensor, assemble, fwht_groups
+from .ladder_kernel import error_table
 from .stats import ColumnStats
 
 ALL_CANDIDATES = [(nb, b) for nb in (2, 4) for b in (16, 32, 64)]
@@ -210,16 +211,12 @@ def build_table(name: str, w: torch.Tensor, stats: ColumnStats | None, cfg: Conf
     wt = stored_rows(w, s16, had)
     inv = None if s16 is None else 1.0 / s16.to(dev, torch.float32)
     d = _weights(stats, k, had, dev, inv)
-    sse, energy = [], None
-    for i, (nb, b) in enumerate(cfg.candidates):
-        enc = encode_rows(wt, d, nb, b, cfg.effort, want_codes=False, want_energy=(i == 0))
-        sse.append(enc.sse)
-        if i == 0:
-            energy = enc.energy
+    effort = EFFORT[cfg.effort]
+    sse, energy = error_table(wt, d, cfg.candidates, effort["grid"], effort["ls"])
     # nothing is read back here: the smoothing vector stays where it was computed (the device) and
     # the energy is a device scalar, so the host can queue the next table while this one runs
     return TensorTable(
-        name, (r, k), had.cpu(), torch.stack(sse), list(cfg.candidates), energy.sum(),
+        name, (r, k), had.cpu(), sse, list(cfg.candidates), energy.sum(),
         n_tokens if n_tokens is not None else (stats.n if stats else 0), s16,
         transform_ref=given,
     )
@@ -249,13 +246,8 @@ def build_tables_grouped(items: list, cfg: Config) -> list:
         d[e] = _weights(st, k, had, dev, None if scale is None else 1.0 / scale)
         kept.append((None if s16 is None else s16.clone(), had.clone()))
     row_group = torch.arange(len(items), device=dev, dtype=torch.int32).repeat_interleave(r)
-    sse, energy = [], None
-    for i, (nb, b) in enumerate(cfg.candidates):
-        enc = encode_rows(wt, d, nb, b, cfg.effort, want_codes=False, want_energy=(i == 0), row_group=row_group)
-        sse.append(enc.sse)
-        if i == 0:
-            energy = enc.energy
-    sse = torch.stack(sse)
+    effort = EFFORT[cfg.effort]
+    sse, energy = error_table(wt, d, cfg.candidates, effort["grid"], effort["ls"], row_group)
     out = []
     for e, (name, _, st, tr, n) in enumerate(items):
         rows = slice(e * r, (e + 1) * r)

@@ -270,19 +270,24 @@ __device__ __forceinline__ float clipped_error(const Block<B>& blk, const float*
 
 constexpr int FIT_THREADS = 128, FIT_WARPS = FIT_THREADS / 32;
 
+struct FitShared {
+  __align__(16) float d[FIT_WARPS][64];
+  float high_error[8][FIT_THREADS];  // a thread's own, by grid point
+};
+
+// The ladders of one tile: 32 rows (16 for blocks of 64) of FIT_WARPS blocks, a block per warp.
 template <int B, bool GROUPED, bool BOUND>
-__global__ void __launch_bounds__(FIT_THREADS, (B == 16 ? 5 : 4))
-fit_kernel(const float* __restrict__ w, int64_t ldw, const float* __restrict__ d_all,
-           const int32_t* __restrict__ row_d, int64_t n_rows, int64_t nb, GridSpec grid, int refits, float nmax, float* __restrict__ lo_out,
-           float* __restrict__ st_out, float* __restrict__ err_out) {
-  __shared__ __align__(16) float d_stage[FIT_WARPS][B];
-  __shared__ float high_error[BOUND ? 8 : 1][FIT_THREADS];  // a thread's own, by grid point
+__device__ __forceinline__ void fit_tile(FitShared& shared, int64_t row_tile, int64_t blk_tile, const float* __restrict__ w,
+                                         int64_t ldw, const float* __restrict__ d_all, const int32_t* __restrict__ row_d,
+                                         int64_t n_rows, int64_t nb, const GridSpec& grid, int refits, float nmax,
+                                         float* __restrict__ lo_out, float* __restrict__ st_out,
+                                         float* __restrict__ err_out) {
   constexpr bool SHARED = Block<B>::SHARED;
   constexpr int PAIRS = Block<B>::PAIRS, ROWS = SHARED ? 16 : 32;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, half = SHARED ? lane & 1 : 0;
-  const int64_t blk = (int64_t)blockIdx.y * FIT_WARPS + warp;
+  const int64_t blk = blk_tile * FIT_WARPS + warp;
   if (blk >= nb) return;  // uniform over the warp
-  const int64_t row = (int64_t)blockIdx.x * ROWS + (SHARED ? lane >> 1 : lane);
+  const int64_t row = row_tile * ROWS + (SHARED ? lane >> 1 : lane);
   const bool live = row < n_rows;
   const int64_t row_c = live ? row : n_rows - 1;
   const float* src = w + row_c * ldw + blk * B;
@@ -294,9 +299,9 @@ fit_kernel(const float* __restrict__ w, int64_t ldw, const float* __restrict__ d
     d = d_all + (int64_t)row_d[row_c] * (nb * B) + blk * B;
   } else {
     for (int t = lane; t < B / 4; t += 32)
-      reinterpret_cast<float4*>(d_stage[warp])[t] = __ldg(reinterpret_cast<const float4*>(d_all + blk * B) + t);
+      reinterpret_cast<float4*>(shared.d[warp])[t] = __ldg(reinterpret_cast<const float4*>(d_all + blk * B) + t);
     __syncwarp();
-    d = d_stage[warp];
+    d = shared.d[warp];
   }
 
   Block<B> r;
@@ -334,7 +339,7 @@ fit_kernel(const float* __restrict__ w, int64_t ldw, const float* __restrict__ d
     weights_ok = lowest >= 0.0f;
 #pragma unroll 1
     for (int gj = 0; gj < grid.g; ++gj)
-      high_error[gj][threadIdx.x] =
+      shared.high_error[gj][threadIdx.x] =
           grid.v[gj] == 0.0f ? 0.0f : clipped_error<B, GROUPED, false>(r, d, half, (mx - grid.v[gj] * span) + slack, one);
   }
 
@@ -351,7 +356,7 @@ fit_kernel(const float* __restrict__ w, int64_t ldw, const float* __restrict__ d
     for (int gj = 0; gj < grid.g; ++gj) {
       const float step = div_by((mx - grid.v[gj] * span) - lo, nmax, rc_n);
       if (bound && (gi | gj) != 0) {
-        bool beaten = weights_ok && step > 1e-15f && 0.9999f * (low_error + high_error[gj][threadIdx.x]) > best_err;
+        bool beaten = weights_ok && step > 1e-15f && 0.9999f * (low_error + shared.high_error[gj][threadIdx.x]) > best_err;
         if (SHARED) beaten = __all_sync(0xffffffffu, beaten);
         if (beaten) continue;
       }
@@ -401,16 +406,75 @@ fit_kernel(const float* __restrict__ w, int64_t ldw, const float* __restrict__ d
   }
 }
 
+template <int B, bool GROUPED, bool BOUND>
+__global__ void __launch_bounds__(FIT_THREADS, (B == 16 ? 5 : 4))
+fit_kernel(const float* __restrict__ w, int64_t ldw, const float* __restrict__ d_all,
+           const int32_t* __restrict__ row_d, int64_t n_rows, int64_t nb, GridSpec grid, int refits, float nmax, float* __restrict__ lo_out,
+           float* __restrict__ st_out, float* __restrict__ err_out) {
+  __shared__ FitShared shared;
+  fit_tile<B, GROUPED, BOUND>(shared, blockIdx.x, blockIdx.y, w, ldw, d_all, row_d, n_rows, nb, grid, refits, nmax, lo_out,
+                              st_out, err_out);
+}
+
+// Every candidate (levels, block) of an error table in one launch: the tiles of one candidate after the
+// other along the grid, so the last wave of one is filled by the next.
+constexpr int TABLE_MAX = 16;
+struct TableCandidate {
+  float *lo, *st;
+  float nmax;
+  int block, bound;
+  unsigned row_tiles, first_tile;
+};
+struct TableSpec {
+  TableCandidate c[TABLE_MAX];
+  int n;
+};
+
+template <bool GROUPED>
+__global__ void __launch_bounds__(FIT_THREADS, 4)
+table_fit_kernel(const float* __restrict__ w, int64_t ldw, const float* __restrict__ d_all,
+                 const int32_t* __restrict__ row_d, int64_t n_rows, int64_t k, const __grid_constant__ GridSpec grid,
+                 int refits, const __grid_constant__ TableSpec table) {
+  __shared__ FitShared shared;
+  int at = 0;
+  while (at + 1 < table.n && blockIdx.x >= table.c[at + 1].first_tile) ++at;
+  const TableCandidate& c = table.c[at];
+  const unsigned tile = blockIdx.x - c.first_tile;
+  const int64_t row_tile = tile % c.row_tiles, blk_tile = tile / c.row_tiles;
+#define HI2_TILE(BB, CC)                                                                                              \
+  fit_tile<BB, GROUPED, CC>(shared, row_tile, blk_tile, w, ldw, d_all, row_d, n_rows, k / BB, grid, refits, c.nmax, c.lo, \
+                            c.st, nullptr)
+  if (c.block == 16) {
+    if (c.bound) HI2_TILE(16, true);
+    else HI2_TILE(16, false);
+  } else if (c.block == 32) {
+    if (c.bound) HI2_TILE(32, true);
+    else HI2_TILE(32, false);
+  } else {
+    if (c.bound) HI2_TILE(64, true);
+    else HI2_TILE(64, false);
+  }
+#undef HI2_TILE
+}
+
+// The grid as the kernels take it; *clips: every point moves an end of the ladder inwards, by half the
+// range at most.
+GridSpec make_grid(const float* grid_host, int g, bool* clips) {
+  GridSpec spec;
+  spec.g = g, spec.one = 1.0f;
+  *clips = true;
+  for (int i = 0; i < 8; ++i) {
+    spec.v[i] = i < g ? grid_host[i] : 0.0f;
+    *clips = *clips && spec.v[i] >= 0.0f && spec.v[i] <= 0.5f;
+  }
+  return spec;
+}
+
 int launch_fit(const float* w, int64_t ldw, const float* d, const int32_t* row_d, const float* grid_host, int g,
                int refits, int n, int64_t n_rows, int64_t nb, int block, float* lo, float* st,
                float* err, cudaStream_t stream) {
-  GridSpec spec;
-  spec.g = g, spec.one = 1.0f;
-  bool clips = true;  // every grid point moves an end of the ladder inwards, by half the range at most
-  for (int i = 0; i < 8; ++i) {
-    spec.v[i] = i < g ? grid_host[i] : 0.0f;
-    clips = clips && spec.v[i] >= 0.0f && spec.v[i] <= 0.5f;
-  }
+  bool clips;
+  const GridSpec spec = make_grid(grid_host, g, &clips);
   dim3 grid((unsigned)ceil_div(n_rows, block == 64 ? 16 : 32), (unsigned)ceil_div(nb, FIT_WARPS));
   const float nmax = (float)(n - 1);
   // Passing over grid points that their clipped columns rule out: 11008 x 4096, normal effort, blocks of 16 /
@@ -450,6 +514,32 @@ __device__ __forceinline__ float warp_sum(float v) {
   return v;
 }
 
+// The three fp16 constants of a row from the extrema of its ladders (hi2/encode.py:95-119).
+struct RowConstants {
+  __half lm_h, ls_h, ss_h;
+  float lm, ls, ss;
+};
+__device__ __forceinline__ RowConstants row_constants(float mxst, float mnlo, float mxlo) {
+  RowConstants c;
+  c.ss_h = __float2half_rn(__fdiv_rn(mxst, 255.0f)), c.ss = __half2float(c.ss_h);
+  c.lm_h = __float2half_rn(mnlo), c.lm = __half2float(c.lm_h);
+  float spread = mxlo - c.lm;
+  spread = spread < 0.0f ? 0.0f : spread;
+  c.ls_h = __float2half_rn(__fdiv_rn(spread, 255.0f)), c.ls = __half2float(c.ls_h);
+  return c;
+}
+// Parameter bytes of one block against the rounded constants, and the ladder they decode to.
+__device__ __forceinline__ void quantise_block(const RowConstants& c, float lo, float st, uint8_t& lu8, uint8_t& su8,
+                                               float& lod, float& std_) {
+  const float s = st < 0.0f ? 0.0f : st;
+  float su = 0.0f, lu = 0.0f;
+  if (c.ss > 0.0f) su = clamp_keep_nan(rintf(__fdiv_rn(s, fmaxf(c.ss, 1e-30f))), 0.0f, 255.0f);
+  if (c.ls > 0.0f) lu = clamp_keep_nan(rintf(__fdiv_rn(lo - c.lm, fmaxf(c.ls, 1e-30f))), 0.0f, 255.0f);
+  su8 = (uint8_t)su, lu8 = (uint8_t)lu;
+  lod = round_f16(fmaf((float)lu8, c.ls, c.lm));
+  std_ = round_f16((float)su8 * c.ss);
+}
+
 constexpr int ROW_THREADS = 256;
 constexpr int ROW_WARPS = ROW_THREADS / 32;
 constexpr int ROW_UN = 4;  // quads a lane loads before it computes
@@ -486,31 +576,18 @@ row_kernel(const float* __restrict__ lo_in, const float* __restrict__ st_in,
     }
     mxst = warp_max(mxst), mnlo = warp_min(mnlo), mxlo = warp_max(mxlo);
     // ---- the three fp16 row constants -------------------------------------------------------
-    const __half ss_h = __float2half_rn(__fdiv_rn(mxst, 255.0f));
-    const float ss = __half2float(ss_h);
-    const __half lm_h = __float2half_rn(mnlo);
-    const float lm = __half2float(lm_h);
-    float spread = mxlo - lm;
-    spread = spread < 0.0f ? 0.0f : spread;
-    const __half ls_h = __float2half_rn(__fdiv_rn(spread, 255.0f));
-    const float ls = __half2float(ls_h);
+    const RowConstants rc = row_constants(mxst, mnlo, mxlo);
     if (lane == 0 && consts != nullptr) {
-      consts[row * 3 + 0] = __half_as_ushort(lm_h);
-      consts[row * 3 + 1] = __half_as_ushort(ls_h);
-      consts[row * 3 + 2] = __half_as_ushort(ss_h);
+      consts[row * 3 + 0] = __half_as_ushort(rc.lm_h);
+      consts[row * 3 + 1] = __half_as_ushort(rc.ls_h);
+      consts[row * 3 + 2] = __half_as_ushort(rc.ss_h);
     }
     // ---- parameter bytes and decoded ladders ------------------------------------------------
     __syncwarp();  // the previous row's readers of s_lo / s_st are done
     for (int64_t b = lane; b < nb; b += 32) {
-      float s = st_r[b];
-      s = s < 0.0f ? 0.0f : s;
-      float su = 0.0f, lu = 0.0f;
-      if (ss > 0.0f) su = clamp_keep_nan(rintf(__fdiv_rn(s, fmaxf(ss, 1e-30f))), 0.0f, 255.0f);
-      if (ls > 0.0f)
-        lu = clamp_keep_nan(rintf(__fdiv_rn(lo_r[b] - lm, fmaxf(ls, 1e-30f))), 0.0f, 255.0f);
-      const uint8_t su8 = (uint8_t)su, lu8 = (uint8_t)lu;
-      const float lod = round_f16(fmaf((float)lu8, ls, lm));
-      const float std_ = round_f16((float)su8 * ss);
+      uint8_t lu8, su8;
+      float lod, std_;
+      quantise_block(rc, lo_r[b], st_r[b], lu8, su8, lod, std_);
       s_lo[b] = lod;
       s_st[b] = std_;
       if (params != nullptr) {
@@ -575,6 +652,157 @@ row_kernel(const float* __restrict__ lo_in, const float* __restrict__ st_in,
     if (lane == 0) {
       if (sse != nullptr) sse[row] = acc;
       if (ENERGY) energy[row] = en;
+    }
+  }
+}
+
+// The row pass of an error table: what row_kernel does for one candidate without codes, for all of them
+// with one pass over the row.  Per candidate the warp forms the row constants and keeps the decoded
+// ladders in shared memory as (lo, step) in fp16, which they are, and the step's reciprocal; then every
+// 128-bit load of the row and of the weights serves all candidates, two columns per instruction as in
+// the search above.  Each lane sums its columns in row_kernel's order, so the errors are the same bits.
+// Bound by instruction issue.  Six candidates, one pass each -> this: 11008 x 4096 400 -> 216 us, 1024 x 2048
+// 53 -> 22.
+struct TableEntry {
+  __half2 ladder;
+  float r;  // 1 / step; 0 for step == 0 (the code is 0), NaN where the quotient has to be a true division
+};
+
+// d (x_hat - x)^2 of four columns, added in column order.
+__device__ __forceinline__ float table_quad(const float4 w, const float4 d, const TableEntry e, float nmax, float2 one,
+                                            float acc) {
+  const float2 ladder = __half22float2(e.ladder);
+  const float2 lo2 = both(ladder.x), st2 = both(ladder.y), neg_r = both(-e.r), off = both(-SHIFT * ladder.y);
+  const float top = SHIFT + nmax;
+  float2 v[2];
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const float2 nx = i == 0 ? make_float2(-w.x, -w.y) : make_float2(-w.z, -w.w);
+    const float2 an = below(nx, lo2, one);
+    const float2 q0 = __fmul2_rn(an, neg_r);
+    const float2 q = __ffma2_rn(__ffma2_rn(q0, st2, an), neg_r, q0);
+    const float2 c = min2(add2(q, both(SHIFT), one), top);
+    const float2 sum = add2(__ffma2_rn(c, st2, off), lo2, one);
+    const float2 diff = add2(__half22float2(__float22half2_rn(sum)), nx, one);
+    v[i] = __fmul2_rn(i == 0 ? make_float2(d.x, d.y) : make_float2(d.z, d.w), __fmul2_rn(diff, diff));
+  }
+  return (((acc + v[0].x) + v[0].y) + v[1].x) + v[1].y;
+}
+// The same with true divisions, for entries without a usable reciprocal.
+__device__ __noinline__ float table_quad_careful(const float4 w, const float4 d, const TableEntry e, float nmax, float acc) {
+  const float lod = __low2float(e.ladder), step = __high2float(e.ladder);
+  const float ws[4] = {w.x, w.y, w.z, w.w}, ds[4] = {d.x, d.y, d.z, d.w};
+#pragma unroll
+  for (int t = 0; t < 4; ++t) {
+    float c = rintf(__fdiv_rn(ws[t] - lod, step == 0.0f ? 1.0f : step));
+    if (step == 0.0f) c = 0.0f;
+    c = clamp_keep_nan(c, 0.0f, nmax);
+    const float diff = round_f16(lod + c * step) - ws[t];
+    acc += ds[t] * (diff * diff);
+  }
+  return acc;
+}
+
+constexpr int TABLE_ROW_WARPS = 4;
+template <int N>  // candidates [first, first + N)
+__global__ void __launch_bounds__(TABLE_ROW_WARPS * 32)
+table_row_kernel(const float* __restrict__ w, int64_t ldw, const float* __restrict__ d_all,
+                 const int32_t* __restrict__ row_d, int64_t n_rows, int64_t k, const __grid_constant__ TableSpec table,
+                 int first, int entries, float one_arg, float* __restrict__ sse, float* __restrict__ energy) {
+  extern __shared__ __align__(16) TableEntry table_smem[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  TableEntry* own = table_smem + (size_t)warp * entries;
+  const float2 one = both(one_arg);
+  int shift[N];
+  float nmax[N];
+  const TableEntry* ladders[N];
+  {
+    int off = 0;
+#pragma unroll
+    for (int c = 0; c < N; ++c) {
+      shift[c] = table.c[first + c].block == 16 ? 4 : table.c[first + c].block == 32 ? 5 : 6;
+      nmax[c] = table.c[first + c].nmax;
+      ladders[c] = own + off;
+      off += (int)(k >> shift[c]);
+    }
+  }
+  for (int64_t row = (int64_t)blockIdx.x * TABLE_ROW_WARPS + warp; row < n_rows; row += (int64_t)gridDim.x * TABLE_ROW_WARPS) {
+    __syncwarp();  // the previous row's readers are done
+    int off = 0;
+    for (int c = first; c < first + N; ++c) {
+      const int nb = (int)(k / table.c[c].block);
+      const float* lo_r = table.c[c].lo + row * nb;
+      const float* st_r = table.c[c].st + row * nb;
+      float mxst = -INFINITY, mnlo = INFINITY, mxlo = -INFINITY;
+      for (int b = lane; b < nb; b += 32) {
+        const float s = st_r[b], l = lo_r[b];
+        mxst = fmaxf(mxst, s < 0.0f ? 0.0f : s);
+        mnlo = fminf(mnlo, l);
+        mxlo = fmaxf(mxlo, l);
+      }
+      mxst = warp_max(mxst), mnlo = warp_min(mnlo), mxlo = warp_max(mxlo);
+      const RowConstants rc = row_constants(mxst, mnlo, mxlo);
+      for (int b = lane; b < nb; b += 32) {
+        uint8_t lu8, su8;
+        float lod, std_;
+        quantise_block(rc, lo_r[b], st_r[b], lu8, su8, lod, std_);
+        const Recip r = make_recip(std_);
+        TableEntry e;
+        e.ladder = __halves2half2(__float2half_rn(lod), __float2half_rn(std_));
+        e.r = std_ == 0.0f ? 0.0f : (r.fast ? r.r : __int_as_float(0x7fc00000));
+        own[off + b] = e;
+      }
+      off += nb;
+    }
+    __syncwarp();
+    const float* wr = w + row * ldw;
+    const float* d = d_all + (row_d != nullptr ? (int64_t)row_d[row] * k : 0);
+    float acc[N], en = 0.0f;
+#pragma unroll
+    for (int c = 0; c < N; ++c) acc[c] = 0.0f;
+    for (int64_t j0 = (int64_t)lane * 4; j0 < k; j0 += 128 * ROW_UN) {
+      float4 wq[ROW_UN], dq[ROW_UN];
+#pragma unroll
+      for (int u = 0; u < ROW_UN; ++u) {
+        const int64_t j = j0 + u * 128;
+        if (j < k) {
+          wq[u] = *reinterpret_cast<const float4*>(wr + j);
+          dq[u] = *reinterpret_cast<const float4*>(d + j);
+        }
+      }
+#pragma unroll 1
+      for (int u = 0; u < ROW_UN; ++u) {
+        const int j = (int)j0 + u * 128;
+        if (j >= k) break;
+        const float4 wv = u == 0 ? wq[0] : u == 1 ? wq[1] : u == 2 ? wq[2] : wq[3];
+        const float4 dv = u == 0 ? dq[0] : u == 1 ? dq[1] : u == 2 ? dq[2] : dq[3];
+        if (energy != nullptr) {
+          en += dv.x * (wv.x * wv.x);
+          en += dv.y * (wv.y * wv.y);
+          en += dv.z * (wv.z * wv.z);
+          en += dv.w * (wv.w * wv.w);
+        }
+        TableEntry e[N];
+        bool usable = true;
+#pragma unroll
+        for (int c = 0; c < N; ++c) e[c] = ladders[c][j >> shift[c]], usable = usable && e[c].r == e[c].r;
+        if (usable) {
+#pragma unroll
+          for (int c = 0; c < N; ++c) acc[c] = table_quad(wv, dv, e[c], nmax[c], one, acc[c]);
+        } else {
+#pragma unroll
+          for (int c = 0; c < N; ++c) acc[c] = table_quad_careful(wv, dv, e[c], nmax[c], acc[c]);
+        }
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < N; ++c) {
+      const float a = warp_sum(acc[c]);
+      if (lane == 0) sse[(int64_t)(first + c) * n_rows + row] = a;
+    }
+    if (energy != nullptr) {
+      en = warp_sum(en);
+      if (lane == 0) energy[row] = en;
     }
   }
 }
@@ -714,6 +942,81 @@ extern "C" int hi2_quantize_rows(const float* lo, const float* step, const float
                                  void* stream) {
   return hi2_quantize_rows_grouped(lo, step, w, ldw, d, nullptr, nbits, n_rows, k, block, params, consts, lo_d, step_d,
                                    ldp, codes, sse, energy, stream);
+}
+
+extern "C" int hi2_error_table(const float* w, int64_t ldw, const float* d, const int32_t* row_d, const float* grid_host,
+                               int g, int refits, int n_cand, const int32_t* nbits_host, const int32_t* block_host,
+                               int64_t n_rows, int64_t k, float* lo, float* step, float* sse, float* energy, void* stream) {
+  using namespace hi2;
+  HI2_REQUIRE(n_cand >= 1 && n_cand <= TABLE_MAX && nbits_host && block_host, "error_table: one to 16 candidates");
+  HI2_REQUIRE(g >= 1 && g <= 8 && grid_host, "fit_ladder: the grid has 1 to 8 points");
+  HI2_REQUIRE(refits >= 0, "fit_ladder: bad n or refits");
+  for (int c = 0; c < n_cand; ++c) {
+    HI2_REQUIRE(block_ok(block_host[c]), "fit_ladder: block must be 16, 32 or 64");
+    HI2_REQUIRE(k > 0 && k % block_host[c] == 0, "fit_ladder: k must be a multiple of the block");
+    HI2_REQUIRE(nbits_host[c] >= 1 && nbits_host[c] <= 8, "quantize_rows: nbits out of range");
+    HI2_REQUIRE(ROW_WARPS * 2 * (k / block_host[c]) * (int64_t)sizeof(float) <= 200 * 1024,
+                "quantize_rows: k too large for the ladder cache");  // the limit of the one-candidate pass
+  }
+  if (n_rows == 0) return HI2_OK;
+  HI2_REQUIRE(w && d && lo && step && sse, "fit_ladder: null pointer");
+  HI2_REQUIRE(aligned16(w) && aligned16(d) && ldw % 4 == 0 && ldw >= k, "fit_ladder: w, d alignment or ldw");
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  bool clips;
+  const GridSpec spec = make_grid(grid_host, g, &clips);
+  TableSpec table;
+  table.n = n_cand;
+  int64_t tiles = 0, offset = 0;
+  for (int c = 0; c < n_cand; ++c) {
+    TableCandidate& x = table.c[c];
+    const int64_t nb = k / block_host[c], row_tiles = ceil_div(n_rows, block_host[c] == 64 ? 16 : 32);
+    x.block = block_host[c], x.nmax = (float)((1 << nbits_host[c]) - 1);
+    x.bound = nbits_host[c] >= 4 && clips;
+    x.lo = lo + offset, x.st = step + offset;
+    x.row_tiles = (unsigned)row_tiles, x.first_tile = (unsigned)tiles;
+    offset += n_rows * nb;
+    tiles += row_tiles * ceil_div(nb, (int64_t)FIT_WARPS);
+    HI2_REQUIRE(tiles < ((int64_t)1 << 31), "error_table: too many rows");
+  }
+  if (row_d != nullptr)
+    table_fit_kernel<true><<<(unsigned)tiles, FIT_THREADS, 0, s>>>(w, ldw, d, row_d, n_rows, k, spec, refits, table);
+  else
+    table_fit_kernel<false><<<(unsigned)tiles, FIT_THREADS, 0, s>>>(w, ldw, d, row_d, n_rows, k, spec, refits, table);
+  int rc = check_launch("fit_ladder");
+  if (rc != HI2_OK) return rc;
+  // the row pass takes as many candidates at a time as their ladders fit in shared memory, six at most
+  constexpr int AT_ONCE = 6;
+  constexpr int64_t ROOM = 200 * 1024 / (TABLE_ROW_WARPS * (int64_t)sizeof(TableEntry));
+  for (int first = 0; first < n_cand;) {
+    int n = 0;
+    int64_t entries = 0;
+    while (first + n < n_cand && n < AT_ONCE && entries + k / block_host[first + n] <= ROOM)
+      entries += k / block_host[first + n], ++n;
+    const int smem = (int)(entries * TABLE_ROW_WARPS * (int64_t)sizeof(TableEntry));
+    const int64_t want = ceil_div(n_rows, (int64_t)TABLE_ROW_WARPS);
+    const unsigned blocks = (unsigned)(want < 148 * 16 ? want : 148 * 16);
+    float* en = first == 0 ? energy : nullptr;
+#define HI2_TABLE_ROW(NN)                                                                                          \
+  case NN:                                                                                                         \
+    if (cudaFuncSetAttribute(table_row_kernel<NN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) \
+      return fail(HI2_ERR_LAUNCH, "quantize_rows: cannot reserve shared memory");                                  \
+    table_row_kernel<NN><<<blocks, TABLE_ROW_WARPS * 32, smem, s>>>(w, ldw, d, row_d, n_rows, k, table, first,     \
+                                                                    (int)entries, 1.0f, sse, en);                  \
+    break
+    switch (n) {
+      HI2_TABLE_ROW(1);
+      HI2_TABLE_ROW(2);
+      HI2_TABLE_ROW(3);
+      HI2_TABLE_ROW(4);
+      HI2_TABLE_ROW(5);
+      HI2_TABLE_ROW(6);
+    }
+#undef HI2_TABLE_ROW
+    rc = check_launch("quantize_rows");
+    if (rc != HI2_OK) return rc;
+    first += n;
+  }
+  return HI2_OK;
 }
 
 extern "C" int hi2_ladder_sse(const uint8_t* codes, const float* w, int64_t ldw, const float* d,

@@ -77,6 +77,36 @@ def fit(w: torch.Tensor, d: torch.Tensor, grid: tuple, refits: int, n: int, bloc
     return lo, st
 
 
+TABLE_MAX = 16  # candidates per call of the table kernels
+
+
+def error_table(w: torch.Tensor, d: torch.Tensor, candidates: list, grid: tuple, refits: int, row_group=None):
+    """``(sse [C, N], energy [N])`` of rows ``w [N, K]`` (fp32, unit column stride) at every candidate
+    ``(nbits, block)``: what :func:`fit` and :func:`quantize_rows` give one candidate at a time, with one
+    launch for all searches and one pass over the rows.  ``d`` and ``row_group`` as in :func:`fit`."""
+    dev = _lib.need_cuda(w, d)
+    rows, k = w.shape
+    if w.dtype != torch.float32 or w.stride(1) != 1:
+        raise ValueError("error_table: w must be fp32 with unit column stride")
+    if not candidates:
+        raise RuntimeError("error_table: no candidates")
+    d = d.to(dev, torch.float32).contiguous()
+    group = _row_d(d, rows, k, row_group, "error_table")
+    sse = torch.empty(len(candidates), rows, dtype=torch.float32, device=dev)
+    energy = torch.empty(rows, dtype=torch.float32, device=dev)
+    points = _lib.host_floats(grid)
+    for c0 in range(0, len(candidates), TABLE_MAX):
+        part = candidates[c0 : c0 + TABLE_MAX]
+        ladders = torch.empty(2, rows * sum(k // b for _, b in part), dtype=torch.float32, device=dev)
+        _lib.call(
+            "hi2_error_table", _lib.ptr(w), w.stride(0), _lib.ptr(d), _lib.ptr(group), points, len(grid), int(refits),
+            len(part), _lib.host_i32([nb for nb, _ in part]), _lib.host_i32([b for _, b in part]), rows, k,
+            _lib.ptr(ladders[0]), _lib.ptr(ladders[1]), _lib.ptr(sse[c0]), _lib.ptr(energy) if c0 == 0 else None,
+            _lib.stream(dev),
+        )
+    return sse, energy
+
+
 def quantize_rows(lo, step, nbits: int, block: int, k: int, w=None, d=None, *, want_params=True,
                   want_decoded=False, ldp: int | None = None, want_codes=False, want_sse=False,
                   want_energy=False, row_group=None):

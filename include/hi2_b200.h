@@ -187,6 +187,16 @@ int hi2_gemm_tf32x3(int64_t m, int64_t n, int64_t kk, const float* a_hi, const f
                     const float* bt_hi, const float* bt_lo, int64_t ldb, float* c, int64_t ldc, int accumulate,
                     int32_t* status, void* stream);
 
+/* hi2/calibrate.py:212-270, one weight's error table: the ladder search and the nearest-code error of
+ * every row at each of n_cand (at most 16) candidates (nbits, block), in one search launch and one pass
+ * over the rows.  lo and step are caller scratch of n_rows * sum(k / block) floats each; sse
+ * [n_cand, n_rows]; energy [n_rows] (sum of d w^2) or null.  Other arguments as in
+ * hi2_fit_ladder_grouped; the errors are the bits hi2_fit_ladder_grouped and
+ * hi2_quantize_rows_grouped give. */
+int hi2_error_table(const float* w, int64_t ldw, const float* d, const int32_t* row_d, const float* grid_host,
+                    int g, int refits, int n_cand, const int32_t* nbits_host, const int32_t* block_host,
+                    int64_t n_rows, int64_t k, float* lo, float* step, float* sse, float* energy, void* stream);
+
 /* hi2/hessian.py:331-338 (_finish): sse[r] = sum_j d[j] * (fp16(lo + code*step) - w[r, j])^2
  * with the decoded ladders lo/st [n_rows, ldp] of block size `block`. */
 int hi2_ladder_sse(const uint8_t* codes, const float* w, int64_t ldw, const float* d,
