@@ -285,6 +285,7 @@ __device__ __forceinline__ float dot4(float4 a, float4 b, float acc) {
 __global__ void __launch_bounds__(256, 1)
 base_kernel(const float* __restrict__ a, float* __restrict__ x, int64_t ld, int64_t off, int n, int32_t* info) {
   extern __shared__ double base_smem[];
+  chain_wait();
   float* sa = reinterpret_cast<float*>(base_smem + LEAF_DOUBLES);
   float* sx = sa + BASE * LDF;
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
@@ -407,6 +408,7 @@ base_kernel(const float* __restrict__ a, float* __restrict__ x, int64_t ld, int6
           make_float4(-acc[r][0], -acc[r][1], -acc[r][2], -acc[r][3]);
     __syncthreads();
   }
+  chain_next();
   float* dst = x + off * ld + off;
   for (int idx = tid; idx < n * (BASE / 4); idx += 256) {
     const int i = idx >> 5, j = (idx & 31) * 4;
@@ -451,6 +453,7 @@ __device__ __forceinline__ void copy16(float* dst, const float* src, int floats)
 __global__ void __launch_bounds__(256, 2)
 product_kernel(const ProductJob job0, const ProductJob job1, int64_t ld) {
   extern __shared__ __align__(16) float product_smem[];
+  chain_wait();
   const ProductJob& p = blockIdx.z ? job1 : job0;
   const int m0 = blockIdx.y * PT, n0 = blockIdx.x * PT;
   if (m0 >= p.m || n0 >= p.n) return;
@@ -531,6 +534,7 @@ product_kernel(const ProductJob job0, const ProductJob job1, int64_t ld) {
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
   __syncthreads();
+  chain_next();
   float* part = product_smem + g * P_TILE;
 #pragma unroll
   for (int i = 0; i < 4; ++i)
@@ -559,7 +563,7 @@ int launch_products(const ProductJob& j0, const ProductJob* j1, int64_t ld, cuda
   const ProductJob& other = j1 ? *j1 : j0;
   dim3 grid((unsigned)ceil_div(j0.n > other.n ? j0.n : other.n, PT), (unsigned)ceil_div(j0.m > other.m ? j0.m : other.m, PT),
             j1 ? 2 : 1);
-  product_kernel<<<grid, 256, P_SMEM, stream>>>(j0, other, ld);
+  launch_link(product_kernel, grid, 256, P_SMEM, stream, j0, other, ld);
   return check_launch("inverse_factor product");
 }
 
@@ -596,7 +600,7 @@ __global__ void merge_status_kernel(const int* status, int32_t* info) {
 int factor(const Plan& pl, int64_t off, int64_t n) {
   const int64_t ld = pl.ld;
   if (n <= BASE) {
-    base_kernel<<<1, 256, BASE_SMEM, pl.stream>>>(pl.a, pl.x, ld, off, (int)n, pl.info);
+    launch_link(base_kernel, 1, 256, BASE_SMEM, pl.stream, pl.a, pl.x, ld, off, (int)n, pl.info);
     return check_launch("inverse_factor base");
   }
   const int64_t n1 = top_half(n), n2 = n - n1;

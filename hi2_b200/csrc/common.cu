@@ -49,7 +49,8 @@ void retire_finished_graphs() {
 }
 }  // namespace
 
-ChainGraph::ChainGraph(cudaStream_t stream) : stream_(stream) {
+ChainGraph::ChainGraph(cudaStream_t stream, int64_t launches) : stream_(stream) {
+  if (launches <= CHAIN_PLAIN) return;
   cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(stream, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone) {
     (void)cudaGetLastError();

@@ -84,6 +84,9 @@ __device__ __forceinline__ void tma_store(const CUtensorMap* map, const void* sr
   asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%2, %3}], [%1];"
                ::"l"(reinterpret_cast<uint64_t>(map)), "r"(s32(src)), "r"(x), "r"(y) : "memory");
 }
+__device__ __forceinline__ void prefetch_map(const CUtensorMap* map) {
+  asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
+}
 // K-major 128-byte-swizzled operand (rows of 128 B, 8-row groups 1024 B apart)
 __device__ __forceinline__ uint64_t desc_kmajor(uint32_t saddr) {
   uint64_t d = (uint64_t)((saddr & 0x3ffffu) >> 4);
@@ -142,6 +145,7 @@ lazy_tc_kernel(const __grid_constant__ CUtensorMap map_ahi, const __grid_constan
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
+    prefetch_map(&map_ahi), prefetch_map(&map_alo), prefetch_map(&map_bhi), prefetch_map(&map_blo), prefetch_map(&map_c);
     for (int s = 0; s < LSTAGES; ++s) bar_init(&ctl->full[s], 1), bar_init(&ctl->empty[s], 1);
     for (int b = 0; b < 2; ++b) bar_init(&ctl->acc_full[b], 1), bar_init(&ctl->acc_empty[b], 4);
     ctl->abort = 0;
@@ -315,6 +319,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_ahi, const __grid_constan
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
+    prefetch_map(&map_ahi), prefetch_map(&map_alo), prefetch_map(&map_bhi), prefetch_map(&map_blo), prefetch_map(&map_c);
     for (int s = 0; s < LSTAGES; ++s) bar_init(&ctl->full[s], 1), bar_init(&ctl->empty[s], 1);
     for (int b = 0; b < 2; ++b) bar_init(&ctl->acc_full[b], 1), bar_init(&ctl->acc_empty[b], 8);
     ctl->abort = 0;
@@ -488,6 +493,7 @@ lazy_group_kernel(const __grid_constant__ CUtensorMap map_ahi, const __grid_cons
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
+    prefetch_map(&map_ahi), prefetch_map(&map_alo), prefetch_map(&map_bhi), prefetch_map(&map_blo), prefetch_map(&map_c);
     for (int s = 0; s < LSTAGES; ++s) bar_init(&ctl->full[s], 1), bar_init(&ctl->empty[s], 1);
     for (int b = 0; b < 2; ++b) bar_init(&ctl->acc_full[b], 1), bar_init(&ctl->acc_empty[b], 8);
     ctl->abort = 0;
