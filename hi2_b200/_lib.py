@@ -60,6 +60,7 @@ SIGNATURES = {
     ),
     "hi2_gptq_lazy_update_tc": (_I, [_P, _L, _L, _L, _P, _P, _P, _P]),
     "hi2_split_tf32_transposed": (_I, [_P, _P, _P, _L, _L, _P]),
+    "hi2_split_factor_transposed": (_I, [_P, _P, _P, _L, _P]),
     "hi2_split_tf32": (_I, [_P, _P, _P, _L, _P]),
     "hi2_gemm_tf32x3": (_I, [_L, _L, _L, _P, _P, _L, _P, _P, _L, _P, _L, _I, _P, _P]),
     "hi2_ladder_sse": (_I, [_P, _P, _L, _P, _P, _P, _L, _L, _L, _I, _P, _P]),

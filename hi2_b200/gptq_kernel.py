@@ -128,9 +128,20 @@ def split_tf32_transposed(x: torch.Tensor) -> torch.Tensor:
     return out
 
 
+def split_factor(u: torch.Tensor) -> torch.Tensor:
+    """:func:`split_tf32_transposed` of an upper-triangular factor ``u [K, K]`` (K a multiple of 4).  What
+    lies above the diagonal of ``u^T`` is left unwritten: the trailing updates do not read it."""
+    dev = _lib.need_cuda(u)
+    _check(u, torch.float32, "u")
+    k = u.shape[0]
+    out = torch.empty(2, k, k, dtype=torch.float32, device=dev)
+    _lib.call("hi2_split_factor_transposed", _lib.ptr(u), _lib.ptr(out[0]), _lib.ptr(out[1]), k, _lib.stream(dev))
+    return out
+
+
 def gptq_round_tc(wc, err1, codes, lo, st, row_grp, u_ptrs, blk, nmax, comp, unit_rows, unit_u_split):
     """:func:`gptq_round` with the trailing update on the tensor cores (3 x TF32, fp32-grade).
-    ``unit_u_split`` holds :func:`split_tf32_transposed` of each unit's factor.  Returns the device status
+    ``unit_u_split`` holds :func:`split_tf32_transposed` or :func:`split_factor` of each unit's factor.  Returns the device status
     word (int32 tensor): non-zero when a bounded device-side wait ran out."""
     dev = _lib.need_cuda(wc, err1, codes, lo, st, row_grp, u_ptrs, blk, nmax, comp, *unit_u_split)
     n, k = wc.shape

@@ -377,7 +377,7 @@ def _round_units(units: list[_Unit], jobs: list[GptqJob], want_comp: bool, split
         parts = []
         for u in us:
             if u.data_ptr() not in splits:
-                splits[u.data_ptr()] = (u, gptq_kernel.split_tf32_transposed(u))  # keeps u alive with its split
+                splits[u.data_ptr()] = (u, gptq_kernel.split_factor(u))  # keeps u alive with its split
             parts.append(splits[u.data_ptr()][1])
         checks.append(gptq_kernel.gptq_round_tc(wc, err1, codes, lo, st, row_grp, u_ptrs, blk, nmax, comp,
                                                 offs, parts))

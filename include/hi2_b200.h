@@ -177,6 +177,10 @@ int hi2_split_tf32(const float* x, float* hi, float* lo, int64_t n, void* stream
 int hi2_split_tf32_transposed(const float* x, float* hi, float* lo, int64_t rows, int64_t cols,
                               void* stream);
 
+/* The same for an upper-triangular factor u [k, k] (k a multiple of 4): only the parts of u^T that the
+ * trailing updates read, those on or below its diagonal, are written. */
+int hi2_split_factor_transposed(const float* u, float* hi, float* lo, int64_t k, void* stream);
+
 /* c[m, n] (ldc) = or += a . bt^T in fp32-grade arithmetic on the tensor cores: both operands as
  * their TF32 parts from hi2_split_tf32 (a [m, kk] with leading dimension lda, bt [n, kk] with ldb,
  * both K-major), three tcgen05 TF32 products per tile accumulated in windows of 64 values of k.

@@ -130,3 +130,13 @@ def test_updates_taken_together_are_the_updates_one_by_one(rows, k):
         got = run("hi2_gptq_round_tc_grouped", _lib.ptr(scratch), columns)
         for a, b in zip(got, want):
             assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("k", [4, 64, 68, 128, 1040])
+def test_split_of_the_factor_where_the_updates_read_it(k):
+    from hi2_b200.gptq_kernel import split_factor, split_tf32_transposed
+
+    u = torch.triu(torch.randn(k, k, generator=gen(k))).cuda()
+    low = torch.ones(k, k, dtype=torch.bool, device="cuda").tril()
+    for got, want in zip(split_factor(u), split_tf32_transposed(u)):
+        assert torch.equal(got[low], want[low])
