@@ -38,11 +38,12 @@ __device__ __noinline__ float2 round_careful(float col, float lo, float st, floa
 }
 
 // The same from prepared values: ladder = (lo, st, 1 / st, highest code: 0 for st == 0), diag = (U_jj,
-// 1 / U_jj).  a * (1 / st) is within 2 ulp of the quotient and rounds to the same integer unless it lies
-// within a few ulp of a half-integer; such columns, NaNs, and ladders and pivots whose reciprocal is
-// not usable (stored as NaN) take the careful path.  The integer is taken by adding and removing
-// 1.5 * 2^23, which rounds to nearest even below 2^22 and keeps anything larger beyond every ladder.
-// The error's quotient is finished with Markstein's fused correction and is the IEEE one.
+// 1 / U_jj).  a * (1 / st) is within 3 ulp of the quotient and rounds to the same integer unless it lies
+// within a few ulp of a half-integer (below 256, where every ladder ends, those are less than 1e-4);
+// such columns, NaNs, and ladders and pivots whose reciprocal is not usable (stored as NaN) take the
+// careful path.  The integer is taken by adding and removing 1.5 * 2^23, which rounds to nearest even
+// below 2^22 and keeps anything larger beyond every ladder.  The error's quotient is finished with
+// Markstein's fused correction and is the IEEE one.
 __device__ __forceinline__ void round_column(float col, float4 ladder, float2 diag, float nm, float& q_out,
                                              float& e_out) {
   const float t = (col - ladder.x) * ladder.z;
@@ -63,8 +64,8 @@ __device__ __forceinline__ void round_column(float col, float4 ladder, float2 di
 // row_window.cuh.  The prepared values of a column are its ladder and the ladder's reciprocal.
 // What bounds it: few rows, the chain (about 110 cycles a column); many rows, shared-memory reads of the
 // factor.  One lane per row with the 128 columns in its registers was bound by the chain at every size
-// and left most SMs idle at a few thousand rows; a block, lane per row -> this: 256 rows 79 -> 25 us,
-// 4096 81 -> 25, 11008 88 -> 40, 22016 107 -> 64, 32768 163 -> 89.
+// and left most SMs idle at a few thousand rows; a block, lane per row -> this: 256 rows 79 -> 23 us,
+// 4096 81 -> 23, 11008 88 -> 39, 22016 107 -> 62, 32768 163 -> 88.
 // Rows of one thread block that read different factors (a block that straddles two tensors) are
 // served one factor after the other: everybody computes, only the rows of that factor store.
 template <int R, bool WITH_COMP, bool SPLIT>
@@ -157,9 +158,10 @@ gptq_block_kernel(const float* __restrict__ wc, int64_t n_rows, int64_t k, int64
 #pragma unroll
         for (int t = 0; t < 4; ++t) {
           const float s = st_n[r][t];
-          const Recip rc = make_recip(s == 0.0f ? 1.0f : s);
-          const float pivot = diag[WIN * win + 4 * quad + t].y;
-          const float z = rc.fast && pivot == pivot ? rc.r : __int_as_float(0x7fc00000);
+          const float safe = s == 0.0f ? 1.0f : s, pivot = diag[WIN * win + 4 * quad + t].y;
+          float z;  // within an ulp of 1 / safe, which round_column's margin covers
+          asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(z) : "f"(safe));
+          if (!(fabsf(safe) > 1e-18f && fabsf(safe) < 1e18f && pivot == pivot)) z = __int_as_float(0x7fc00000);
           *reinterpret_cast<float4*>(lad + 4 * t) = make_float4(lo_n[r][t], s, z, s == 0.0f ? 0.0f : nm[r]);
         }
         *reinterpret_cast<float4*>(const_cast<float*>(swap[r]) + 4 * quad) = w[r][0];
