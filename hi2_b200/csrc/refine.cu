@@ -19,7 +19,8 @@ __global__ void __launch_bounds__(BLOCK_THREADS, (R == 1 ? 4 : 3))
 refine_block_kernel(const float* __restrict__ gb, int64_t ldg, int len, float* __restrict__ c,
                     const float* __restrict__ lo, const float* __restrict__ st,
                     const float* __restrict__ top, const float* __restrict__ hs, int64_t n_rows,
-                    int64_t k, int64_t b0, float* __restrict__ dwb, float* __restrict__ dw_lo, int64_t lddw) {
+                    int64_t k, int64_t b0, float* __restrict__ dwb, float* __restrict__ dw_lo, int64_t lddw,
+                    int32_t* __restrict__ moved_any) {
   extern __shared__ __align__(16) float refine_smem[];
   const int lane = threadIdx.x & 31, quad = lane & 3;
   const int row0 = (threadIdx.x >> 5) * 8 * R + (lane >> 2);  // this lane's rows of the block: row0 + 8 r
@@ -54,6 +55,7 @@ refine_block_kernel(const float* __restrict__ gb, int64_t ldg, int len, float* _
   };
 #pragma unroll
   for (int r = 0; r < R; ++r) fetch(r, 0);
+  bool any = false;  // a live row of this lane has moved
   asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
 
@@ -125,6 +127,7 @@ refine_block_kernel(const float* __restrict__ gb, int64_t ldg, int len, float* _
       if (!live[r]) continue;
       const int at = WIN * win + 4 * quad;
       const float4 d = *reinterpret_cast<const float4*>(swap[r] + 4 * quad);
+      any = any || d.x != 0.0f || d.y != 0.0f || d.z != 0.0f || d.w != 0.0f;
       auto moved = [](float code_j, float dw_j) { return dw_j > 0.0f ? code_j + 1.0f : (dw_j < 0.0f ? code_j - 1.0f : code_j); };
       *reinterpret_cast<float4*>(c + row[r] * k + b0 + at) =
           make_float4(moved(now_code[r].x, d.x), moved(now_code[r].y, d.y), moved(now_code[r].z, d.z), moved(now_code[r].w, d.w));
@@ -133,25 +136,55 @@ refine_block_kernel(const float* __restrict__ gb, int64_t ldg, int len, float* _
     update_behind<R, false>(w, uw, width, quad, swap, windows - 1 - win);
     __syncwarp();  // the exchange floats are overwritten next
   }
+  if (moved_any != nullptr && any) *moved_any = 1;
+}
+
+// What the sweeps start from, for one group of rows in one pass: codes as fp32, the ladder of every column
+// (decoded as hi2/format.py:45-60: lo = fp16(fma(byte, lo_scale, lo_min)), step = fp16(byte * step_scale)),
+// and the error e = fp16(lo + c step) - w, as it is or as its TF32 parts.  Bound by memory: 25 bytes
+// written and 5 read per weight; a dozen elementwise passes before, 650 -> 67 us for 4096 x 4096.
+__global__ void __launch_bounds__(256)
+refine_prepare_kernel(const float* __restrict__ w, int64_t ldw, const uint8_t* __restrict__ codes,
+                      const uint8_t* __restrict__ params, const uint16_t* __restrict__ consts, int shift, int64_t n_rows,
+                      int64_t k, float* __restrict__ c, float* __restrict__ lo_x, float* __restrict__ st_x,
+                      float* __restrict__ e, float* __restrict__ e_lo) {
+  const int64_t j = ((int64_t)blockIdx.y * 256 + threadIdx.x) * 4;
+  if (j >= k) return;
+  for (int64_t row = blockIdx.x; row < n_rows; row += gridDim.x) {
+    const float lm = __half2float(__ushort_as_half(consts[row * 3])), ls = __half2float(__ushort_as_half(consts[row * 3 + 1])),
+                ss = __half2float(__ushort_as_half(consts[row * 3 + 2]));
+    const uchar2 p = *reinterpret_cast<const uchar2*>(params + (row * (k >> shift) + (j >> shift)) * 2);
+    const float lo = round_f16(fmaf((float)p.x, ls, lm)), st = round_f16((float)p.y * ss);
+    const uchar4 q = *reinterpret_cast<const uchar4*>(codes + row * k + j);
+    const float4 v = *reinterpret_cast<const float4*>(w + row * ldw + j);
+    const float4 cf = make_float4((float)q.x, (float)q.y, (float)q.z, (float)q.w);
+    const int64_t at = row * k + j;
+    *reinterpret_cast<float4*>(c + at) = cf;
+    *reinterpret_cast<float4*>(lo_x + at) = make_float4(lo, lo, lo, lo);
+    *reinterpret_cast<float4*>(st_x + at) = make_float4(st, st, st, st);
+    store_factors(e + at, e_lo ? e_lo + at : nullptr,
+                  make_float4(round_f16(lo + cf.x * st) - v.x, round_f16(lo + cf.y * st) - v.y,
+                              round_f16(lo + cf.z * st) - v.z, round_f16(lo + cf.w * st) - v.w));
+  }
 }
 
 template <int R>
 int launch_refine_as(const float* gb, int64_t ldg, int len, float* c, const float* lo, const float* st,
                      const float* top, const float* hs, int64_t n_rows, int64_t k, int64_t b0, float* dwb,
-                     float* dw_lo, int64_t lddw, cudaStream_t stream) {
+                     float* dw_lo, int64_t lddw, int32_t* moved, cudaStream_t stream) {
   if (cudaFuncSetAttribute(refine_block_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes<R>()) !=
       cudaSuccess)
     return fail(HI2_ERR_LAUNCH, "refine_block: cannot reserve shared memory");
   refine_block_kernel<R><<<(unsigned)ceil_div(n_rows, (int64_t)rows_per_block<R>()), BLOCK_THREADS, smem_bytes<R>(), stream>>>(
-      gb, ldg, len, c, lo, st, top, hs, n_rows, k, b0, dwb, dw_lo, lddw);
+      gb, ldg, len, c, lo, st, top, hs, n_rows, k, b0, dwb, dw_lo, lddw, moved);
   return check_launch("refine_block");
 }
 int launch_refine_block(const float* gb, int64_t ldg, int len, float* c, const float* lo, const float* st,
                         const float* top, const float* hs, int64_t n_rows, int64_t k, int64_t b0, float* dwb,
-                        float* dw_lo, int64_t lddw, cudaStream_t stream) {
+                        float* dw_lo, int64_t lddw, int32_t* moved, cudaStream_t stream) {
   if (two_rows_per_lane(n_rows))
-    return launch_refine_as<2>(gb, ldg, len, c, lo, st, top, hs, n_rows, k, b0, dwb, dw_lo, lddw, stream);
-  return launch_refine_as<1>(gb, ldg, len, c, lo, st, top, hs, n_rows, k, b0, dwb, dw_lo, lddw, stream);
+    return launch_refine_as<2>(gb, ldg, len, c, lo, st, top, hs, n_rows, k, b0, dwb, dw_lo, lddw, moved, stream);
+  return launch_refine_as<1>(gb, ldg, len, c, lo, st, top, hs, n_rows, k, b0, dwb, dw_lo, lddw, moved, stream);
 }
 
 }  // namespace
@@ -169,13 +202,19 @@ extern "C" int hi2_refine_block(const float* gb, int len, float* c, const float*
   HI2_REQUIRE(aligned16(gb) && aligned16(c) && aligned16(lo) && aligned16(st) && aligned16(hs) &&
                   aligned16(dwb),
               "refine_block: buffers must be 16-byte aligned");
-  return launch_refine_block(gb, len, len, c, lo, st, top, hs, n_rows, k, b0, dwb, nullptr, len,
+  return launch_refine_block(gb, len, len, c, lo, st, top, hs, n_rows, k, b0, dwb, nullptr, len, nullptr,
                              static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int hi2_refine_block_in_place(const float* g, int len, float* c, const float* lo, const float* st,
                                          const float* top, const float* hs, int64_t n_rows, int64_t k,
                                          int64_t b0, float* dw_hi, float* dw_lo, int64_t lddw, void* stream) {
+  return hi2_refine_sweep_block(g, len, c, lo, st, top, hs, n_rows, k, b0, dw_hi, dw_lo, lddw, nullptr, stream);
+}
+
+extern "C" int hi2_refine_sweep_block(const float* g, int len, float* c, const float* lo, const float* st,
+                                      const float* top, const float* hs, int64_t n_rows, int64_t k, int64_t b0,
+                                      float* dw_hi, float* dw_lo, int64_t lddw, int32_t* moved, void* stream) {
   using namespace hi2;
   HI2_REQUIRE(k > 0 && k % 16 == 0, "refine_block_in_place: k must be a positive multiple of 16");
   HI2_REQUIRE(len > 0 && len <= LMAX && len % 16 == 0, "refine_block_in_place: block length must be 16..128");
@@ -186,6 +225,24 @@ extern "C" int hi2_refine_block_in_place(const float* g, int len, float* c, cons
   HI2_REQUIRE(aligned16(g) && aligned16(c) && aligned16(lo) && aligned16(st) && aligned16(hs) &&
                   aligned16(dw_hi) && aligned16(dw_lo),
               "refine_block_in_place: buffers must be 16-byte aligned");
-  return launch_refine_block(g + b0, k, len, c, lo, st, top, hs, n_rows, k, b0, dw_hi, dw_lo, lddw,
+  return launch_refine_block(g + b0, k, len, c, lo, st, top, hs, n_rows, k, b0, dw_hi, dw_lo, lddw, moved,
                              static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int hi2_refine_prepare(const float* w, int64_t ldw, const uint8_t* codes, const uint8_t* params,
+                                  const uint16_t* consts, int block, int64_t n_rows, int64_t k, float* c, float* lo_x,
+                                  float* st_x, float* e, float* e_lo, void* stream) {
+  using namespace hi2;
+  HI2_REQUIRE(block == 16 || block == 32 || block == 64, "refine_prepare: block must be 16, 32 or 64");
+  HI2_REQUIRE(k > 0 && k % block == 0, "refine_prepare: k must be a multiple of the block");
+  if (n_rows == 0) return HI2_OK;
+  HI2_REQUIRE(w && codes && params && consts && c && lo_x && st_x && e, "refine_prepare: null pointer");
+  HI2_REQUIRE(aligned16(w) && ldw % 4 == 0 && ldw >= k && (reinterpret_cast<uintptr_t>(codes) & 3u) == 0 &&
+                  (reinterpret_cast<uintptr_t>(params) & 1u) == 0 && aligned16(c) && aligned16(lo_x) && aligned16(st_x) &&
+                  aligned16(e) && (e_lo == nullptr || aligned16(e_lo)),
+              "refine_prepare: alignment or ldw");
+  const dim3 grid((unsigned)(n_rows < 65536 ? n_rows : 65536), (unsigned)ceil_div(k, (int64_t)1024));
+  refine_prepare_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+      w, ldw, codes, params, consts, block == 16 ? 4 : block == 32 ? 5 : 6, n_rows, k, c, lo_x, st_x, e, e_lo);
+  return check_launch("refine_prepare");
 }

@@ -34,36 +34,46 @@ def _expand(lo: torch.Tensor, step: torch.Tensor, block: int):
     return lo.repeat_interleave(block, dim=1), step.repeat_interleave(block, dim=1)
 
 
+def _use_tc(use_tc: bool, k: int) -> bool:
+    """The two products of a sweep, g = e Hs and g += dw Hs[b0:b1], run on the tensor cores as three TF32
+    products (fp32-grade; Hs is symmetric, so its rows are the K-major right operand as they lie).  Rows
+    with 256 levels and narrow inputs keep the fp32 FMA product, as in the GPTQ path."""
+    return use_tc and k >= TC_MIN_K and k % 4 == 0
+
+
 @torch.no_grad()
 def _sweeps(w, codes, lo_x, st_x, top, hs, passes: int, use_tc: bool | None, wait: bool):
-    """``(refined codes (float), status word or None)``.  With ``wait`` the host follows the device:
-    it stops after a sweep that moved no code and raises on a raised status word.  Without, nothing
-    is read back: every sweep is queued (one that moves nothing changes nothing) and the status
-    word is left to the caller, so several tensors can be refined side by side on streams."""
-    dev = _lib.need_cuda(w, codes, lo_x, st_x, top, hs)
-    if not refine_kernel.available(dev):
-        raise RuntimeError(f"refine kernel unavailable on {dev}: {refine_kernel.failure()}")
-    n_rows, k = w.shape
+    """:func:`_run` for rows given with a ladder per column."""
+    _lib.need_cuda(w, codes, lo_x, st_x, top, hs)
     c = codes.float().contiguous().clone()
     lo_x, st_x = lo_x.float().contiguous(), st_x.float().contiguous()
-    top = top.float().contiguous()
-    hs = hs.float().contiguous()
     e = ((lo_x + c * st_x).half().float() - w.float()).contiguous()
+    use_tc = _use_tc(bool((top <= 15).all()) if use_tc is None else use_tc, w.shape[1])
+    if use_tc:
+        e = refine_kernel.split_tf32(e)
+    return _run(c, lo_x, st_x, top.float().contiguous(), [e], hs.float().contiguous(), passes, use_tc, wait)
+
+
+@torch.no_grad()
+def _run(c, lo_x, st_x, top, e: list, hs, passes: int, use_tc: bool, wait: bool):
+    """``(refined codes (float), status word or None)`` from fp32 codes ``c [N, K]`` (changed in place) and
+    their errors ``e`` (one entry, taken out of the list: as TF32 parts with ``use_tc``).  With ``wait``
+    the host follows the device: it stops after a sweep that moved no code and raises on a raised
+    status word.  Without, nothing is read back: every sweep is queued (one that moves nothing changes
+    nothing) and the status word is left to the caller, so several tensors can be refined side by side
+    on streams."""
+    dev = _lib.need_cuda(c, lo_x, st_x, top, hs)
+    if not refine_kernel.available(dev):
+        raise RuntimeError(f"refine kernel unavailable on {dev}: {refine_kernel.failure()}")
+    n_rows, k = c.shape
     g = torch.empty(n_rows, k, dtype=torch.float32, device=dev)
-    # The two products of a sweep, g = e Hs and g += dw Hs[b0:b1], run on the tensor cores as three
-    # TF32 products (fp32-grade; Hs is symmetric, so its rows are the K-major right operand as they
-    # lie).  Rows with 256 levels and narrow inputs keep the fp32 FMA product, as in the GPTQ path.
-    if use_tc is None:
-        use_tc = bool((top <= 15).all())
-    use_tc = use_tc and k >= TC_MIN_K and k % 4 == 0
     status = None
     if use_tc:
         status = torch.zeros(1, dtype=torch.int32, device=dev)
         hs_split = refine_kernel.split_tf32(hs)
-        refine_kernel.gemm_tc(refine_kernel.split_tf32(e), hs_split, g, status)
+        refine_kernel.gemm_tc(e.pop(), hs_split, g, status)
     else:
-        refine_kernel.gemm(e, hs, g)
-    del e
+        refine_kernel.gemm(e.pop(), hs, g)
     # With tensor-core products the block kernel reads its slice of g in place and leaves the changes
     # as TF32 parts, and g is brought up to date lazily, as the GPTQ loop does: after a block only the
     # later blocks of its group of GROUP_BLOCKS need its moves now (a narrow product); the columns
@@ -75,16 +85,21 @@ def _sweeps(w, codes, lo_x, st_x, top, hs, passes: int, use_tc: bool | None, wai
     # a group is one block and its update one product.
     width = (GROUP_BLOCKS if n_rows * k >= GROUP_MIN_ELEMS else 1) * BLOCK_COLUMNS
     moves = torch.empty(2, n_rows, min(width, k), dtype=torch.float32, device=dev) if use_tc else None
-    for _ in range(passes):
-        start = c.clone() if wait else None
+    moved = torch.zeros(1, dtype=torch.int32, device=dev) if wait and use_tc else None
+    for sweep in range(passes):
+        last = sweep + 1 == passes  # nobody reads g behind it: only the columns still to come are updated
+        follow = wait and not last  # whether the next sweep is worth queueing
+        start = c.clone() if follow and not use_tc else None
         if not use_tc:
             for b0 in range(0, k, BLOCK_COLUMNS):
                 b1 = min(b0 + BLOCK_COLUMNS, k)
                 gb = g[:, b0:b1].contiguous()
                 dw_block = torch.empty(n_rows, b1 - b0, dtype=torch.float32, device=dev)
                 refine_kernel.refine_block(gb, c, lo_x, st_x, top, hs, b0, b1 - b0, dw_block)
-                refine_kernel.gemm(dw_block, hs[b0:b1], g, alpha=1.0, beta=1.0)
-            if wait and bool((c == start).all()):
+                first = b1 if last else 0
+                if first < k:
+                    refine_kernel.gemm(dw_block, hs[b0:b1, first:], g[:, first:], alpha=1.0, beta=1.0)
+            if follow and bool((c == start).all()):
                 break
             continue
         for g0 in range(0, k, width):
@@ -92,23 +107,27 @@ def _sweeps(w, codes, lo_x, st_x, top, hs, passes: int, use_tc: bool | None, wai
             for b0 in range(g0, g1, BLOCK_COLUMNS):
                 b1 = min(b0 + BLOCK_COLUMNS, g1)
                 dw = moves[:, :, b0 - g0 : b1 - g0]
-                refine_kernel.refine_block_in_place(g, c, lo_x, st_x, top, hs, b0, b1 - b0, dw)
+                refine_kernel.refine_block_in_place(g, c, lo_x, st_x, top, hs, b0, b1 - b0, dw, moved)
                 if b1 < g1:
                     refine_kernel.gemm_tc(dw, hs_split[:, b1:g1, b0:b1], g[:, b1:g1], status, accumulate=True)
-            if width == BLOCK_COLUMNS:  # groups of one block: the whole update in one product
-                refine_kernel.gemm_tc(moves[:, :, : g1 - g0], hs_split[:, :, g0:g1], g, status, accumulate=True)
-                continue
             group = moves[:, :, : g1 - g0]
-            if g0 > 0:
+            if width == BLOCK_COLUMNS:  # groups of one block: the whole update in one product
+                first = g1 if last else 0
+                if first < k:
+                    refine_kernel.gemm_tc(group, hs_split[:, first:, g0:g1], g[:, first:], status, accumulate=True)
+                continue
+            if g0 > 0 and not last:
                 refine_kernel.gemm_tc(group, hs_split[:, :g0, g0:g1], g[:, :g0], status, accumulate=True)
             if g1 < k:
                 refine_kernel.gemm_tc(group, hs_split[:, g1:, g0:g1], g[:, g1:], status, accumulate=True)
-            for b0 in range(g0, g1, BLOCK_COLUMNS):
+            for b0 in range(g0, g1, BLOCK_COLUMNS) if not last else ():
                 b1 = min(b0 + BLOCK_COLUMNS, g1)
                 refine_kernel.gemm_tc(moves[:, :, b0 - g0 : g1 - g0], hs_split[:, b0:b1, b0:g1], g[:, b0:b1], status,
                                       accumulate=True)
-        if wait and bool((c == start).all()):
-            break
+        if follow:
+            if not int(moved.item()):
+                break
+            moved.zero_()
     if wait and use_tc and int(status.item()):
         raise RuntimeError("refine: a bounded device-side wait ran out in a tensor-core product")
     return c, status
@@ -141,15 +160,37 @@ def refine_groups(groups, hs: torch.Tensor, passes: int, wait: bool = True):
     candidates, and of different tensors that read the same input, share the column loop); returns
     the refined codes per group.  ``wait=False`` reads nothing back and returns ``(codes per group,
     status word or None)``: the caller checks the word once it has queued everything."""
-    parts = []
-    for w, enc, nbits, block in groups:
-        lo, step = _decoded(enc)
-        lo_x, st_x = _expand(lo, step, block)
-        top = torch.full((w.shape[0],), float(2**nbits - 1), device=w.device)
-        parts.append((w.float(), enc.codes.float(), lo_x, st_x, top))
-    cat = [torch.cat([p[i] for p in parts]) for i in range(5)]
-    out, status = _sweeps(*cat, hs, passes, max(g[2] for g in groups) <= 4, wait)
-    sizes = [p[0].shape[0] for p in parts]
+    use_tc = max(g[2] for g in groups) <= 4
+    plain = all(enc.codes.dtype == torch.uint8 and enc.params.dtype == torch.uint8 and enc.consts.dtype == torch.float16
+                and block in (16, 32, 64) for _, enc, _, block in groups)
+    sizes = [w.shape[0] for w, *_ in groups]
+    if plain and groups[0][0].shape[1] % 16 == 0:  # encodes as this package leaves them: one pass over each group's rows
+        dev = _lib.need_cuda(*[w for w, *_ in groups], hs)
+        n, k = sum(sizes), groups[0][0].shape[1]
+        use_tc = _use_tc(use_tc, k)
+        c, lo_x, st_x = (torch.empty(n, k, dtype=torch.float32, device=dev) for _ in range(3))
+        e = torch.empty(*((2,) if use_tc else ()), n, k, dtype=torch.float32, device=dev)
+        top = torch.empty(n, dtype=torch.float32, device=dev)
+        r0 = 0
+        for (w, enc, nbits, block), rows in zip(groups, sizes):
+            at = slice(r0, r0 + rows)
+            wf = w.float()
+            if wf.stride(1) != 1 or wf.stride(0) % 4 or wf.data_ptr() % 16:
+                wf = wf.contiguous().clone()
+            refine_kernel.prepare(wf, enc.codes.contiguous(), enc.params.contiguous(), enc.consts.contiguous(), block, c[at],
+                                  lo_x[at], st_x[at], *((e[0, at], e[1, at]) if use_tc else (e[at],)))
+            top[at] = float(2**nbits - 1)
+            r0 += rows
+        out, status = _run(c, lo_x, st_x, top, [e], hs.float().contiguous(), passes, use_tc, wait)
+    else:
+        parts = []
+        for w, enc, nbits, block in groups:
+            lo, step = _decoded(enc)
+            lo_x, st_x = _expand(lo, step, block)
+            top = torch.full((w.shape[0],), float(2**nbits - 1), device=w.device)
+            parts.append((w.float(), enc.codes.float(), lo_x, st_x, top))
+        cat = [torch.cat([p[i] for p in parts]) for i in range(5)]
+        out, status = _sweeps(*cat, hs, passes, use_tc, wait)
     codes = [c.to(groups[i][1].codes.dtype) for i, c in enumerate(out.split(sizes))]
     return codes if wait else (codes, status)
 

@@ -43,11 +43,12 @@ def refine_block(gb, c, lo_x, st_x, top, hs, b0, length, dw_block) -> None:
     )
 
 
-def refine_block_in_place(g, c, lo_x, st_x, top, hs, b0, length, dw_split) -> None:
+def refine_block_in_place(g, c, lo_x, st_x, top, hs, b0, length, dw_split, moved=None) -> None:
     """:func:`refine_block` reading the block's slice of ``g [N, K]`` where it lies and writing the
     changes as TF32 parts ``dw_split [2, N, length]``, the left operand of :func:`gemm_tc`;
-    ``dw_split`` may be a column slice of a wider ``[2, N, W]`` buffer (unit column stride)."""
-    dev = _lib.need_cuda(g, c, lo_x, st_x, top, hs, dw_split)
+    ``dw_split`` may be a column slice of a wider ``[2, N, W]`` buffer (unit column stride).  ``moved``
+    (optional, a device int32) is set to 1 if a code moved."""
+    dev = _lib.need_cuda(g, c, lo_x, st_x, top, hs, dw_split, moved)
     for t, name in ((g, "g"), (c, "c"), (lo_x, "lo"), (st_x, "st"), (top, "top"), (hs, "hs")):
         if t.dtype != torch.float32 or not t.is_contiguous():
             raise ValueError(f"refine_block_in_place: {name} must be a contiguous float32 tensor")
@@ -61,9 +62,29 @@ def refine_block_in_place(g, c, lo_x, st_x, top, hs, b0, length, dw_split) -> No
     if n == 0:
         return
     _lib.call(
-        "hi2_refine_block_in_place", _lib.ptr(g), int(length), _lib.ptr(c), _lib.ptr(lo_x), _lib.ptr(st_x),
+        "hi2_refine_sweep_block", _lib.ptr(g), int(length), _lib.ptr(c), _lib.ptr(lo_x), _lib.ptr(st_x),
         _lib.ptr(top), _lib.ptr(hs), n, k, int(b0), _lib.ptr(dw_split[0]), _lib.ptr(dw_split[1]),
-        dw_split.stride(1), _lib.stream(dev),
+        dw_split.stride(1), _lib.ptr(moved), _lib.stream(dev),
+    )
+
+
+def prepare(w, codes, params, consts, block, c, lo_x, st_x, e, e_lo=None) -> None:
+    """Fill ``c``, ``lo_x``, ``st_x [N, K]`` (fp32) with the codes and the ladder of every column of rows
+    encoded at one ``block``, and ``e`` (with ``e_lo``: its TF32 parts) with the error of the decoded
+    values against ``w``.  ``codes`` and ``params`` uint8, ``consts`` fp16, as an encode leaves them."""
+    dev = _lib.need_cuda(w, codes, params, consts, c, lo_x, st_x, e, e_lo)
+    n, k = w.shape
+    for t, dt, shape, name in ((codes, torch.uint8, (n, k), "codes"), (params, torch.uint8, (n, k // block, 2), "params"),
+                               (consts, torch.float16, (n, 3), "consts"), (c, torch.float32, (n, k), "c"),
+                               (lo_x, torch.float32, (n, k), "lo_x"), (st_x, torch.float32, (n, k), "st_x"),
+                               (e, torch.float32, (n, k), "e")):
+        if t.dtype != dt or tuple(t.shape) != shape or not t.is_contiguous():
+            raise ValueError(f"prepare: {name} must be a contiguous {dt} tensor of shape {shape}")
+    if w.dtype != torch.float32 or w.stride(1) != 1:
+        raise ValueError("prepare: w must be fp32 with unit column stride")
+    _lib.call(
+        "hi2_refine_prepare", _lib.ptr(w), w.stride(0), _lib.ptr(codes), _lib.ptr(params), _lib.ptr(consts), int(block), n, k,
+        _lib.ptr(c), _lib.ptr(lo_x), _lib.ptr(st_x), _lib.ptr(e), _lib.ptr(e_lo), _lib.stream(dev),
     )
 
 

@@ -222,6 +222,18 @@ int hi2_refine_block(const float* gb, int len, float* c, const float* lo, const 
 int hi2_refine_block_in_place(const float* g, int len, float* c, const float* lo, const float* st,
                               const float* top, const float* hs, int64_t n_rows, int64_t k,
                               int64_t b0, float* dw_hi, float* dw_lo, int64_t lddw, void* stream);
+/* The same, setting *moved (device int32, or null) to 1 if any code of any row moved. */
+int hi2_refine_sweep_block(const float* g, int len, float* c, const float* lo, const float* st, const float* top,
+                           const float* hs, int64_t n_rows, int64_t k, int64_t b0, float* dw_hi, float* dw_lo,
+                           int64_t lddw, int32_t* moved, void* stream);
+/* What a sweep starts from (hi2/refine.py:44-60), for rows rounded at one block size: fp32 codes c, the
+ * decoded ladder of every column lo_x, st_x, and e = fp16(lo + c * step) - w, as it is (e_lo null) or as
+ * its TF32 parts.  w fp32 [n_rows, k] (ldw); codes u8 [n_rows, k], params u8 [n_rows, k / block, 2],
+ * consts fp16 [n_rows, 3] of an encode; the outputs fp32 [n_rows, k]. */
+int hi2_refine_prepare(const float* w, int64_t ldw, const uint8_t* codes, const uint8_t* params,
+                       const uint16_t* consts, int block, int64_t n_rows, int64_t k, float* c, float* lo_x,
+                       float* st_x, float* e, float* e_lo, void* stream);
+
 
 /* ---- dense helpers of the path -------------------------------------------------------------
  * C = alpha * op(A) op(B) + beta * C in fp32 (fused multiply-add accumulation, fp32 operands):

@@ -68,3 +68,42 @@ def test_rows_per_lane_do_not_change_anything(rows):
         refine_kernel.refine_block(g_all[at].contiguous(), part, lo[at].contiguous(), st[at].contiguous(), top[at].contiguous(), hs,
                                    0, 128, dwp)
         assert torch.equal(whole[at], part) and torch.equal(dw[at], dwp)
+
+
+@pytest.mark.parametrize("rows,k", [(1, 64), (3, 192), (70, 1088), (33, 4160)])
+@pytest.mark.parametrize("nbits,block", [(2, 16), (4, 64), (8, 32)])
+def test_prepare_is_the_elementwise_form(rows, k, nbits, block):
+    from hi2_b200 import refine_kernel
+    from hi2_b200.encode import encode_rows
+    from hi2_b200.refine import _decoded, _expand
+
+    w = torch.randn(rows, k, generator=gen(rows + k)).cuda()
+    w[::2, : k // 2] = 0
+    enc = encode_rows(w, torch.ones(k, device="cuda"), nbits, block, "fast")
+    lo_x, st_x = _expand(*_decoded(enc), block)
+    e = (lo_x + enc.codes.float() * st_x).half().float() - w
+    c, lo, st, got, low = (torch.empty(rows, k, device="cuda") for _ in range(5))
+    refine_kernel.prepare(w, enc.codes, enc.params, enc.consts, block, c, lo, st, got)
+    assert torch.equal(c, enc.codes.float()) and torch.equal(lo, lo_x) and torch.equal(st, st_x) and torch.equal(got, e)
+    refine_kernel.prepare(w, enc.codes, enc.params, enc.consts, block, c, lo, st, got, low)
+    assert torch.equal(torch.stack([got, low]), refine_kernel.split_tf32(e.contiguous()))
+
+
+@pytest.mark.parametrize("k", [192, 640])  # FMA and tensor-core products
+def test_sweeps_one_by_one_are_the_sweeps_together(k):
+    """The last sweep updates only what it still reads: the codes of two sweeps are those of one and one."""
+    from hi2_b200.encode import Encoded, encode_rows
+    from hi2_b200.refine import refine_groups
+
+    x = torch.randn(2 * k, k, generator=gen(k))
+    hs = (x.T @ x / x.shape[0]).cuda()
+    w = torch.randn(90, k, generator=gen(k + 1)).cuda()
+    enc = encode_rows(w, hs.diagonal().contiguous(), 4, 32, "fast")
+    for wait in (True, False):
+        two = refine_groups([(w, enc, 4, 32)], hs, 2, wait)
+        many = refine_groups([(w, enc, 4, 32)], hs, 40, wait)
+        two, many = (two[0], many[0]) if wait else (two[0][0], many[0][0])
+        assert int((two != enc.codes).sum()) > 0
+        done = Encoded(many, enc.params, enc.consts, enc.sse)
+        again = refine_groups([(w, done, 4, 32)], hs, 1)[0]  # after many sweeps nothing moves any more
+        assert (again != many).float().mean() < 1e-3
