@@ -7,12 +7,18 @@
 // move adds dw = 0, which leaves g as it is.  2 dw and (dw dw) H_jj of both moves do not depend on g and
 // are prepared a window ahead, so the chain of a column is two products, two sums and two comparisons.
 // Measured per block of 4096 x 128, us: a warp per row with a shuffle per column 47, this 19.
+#include "gemm.cuh"
 #include "row_window.cuh"
 
 namespace hi2 {
+// lazy_tc.cu; flag 32: the product is added to c
+int launch_gemm_tc2(int64_t m, int64_t n, int64_t kk, const float* a_hi, const float* a_lo, int64_t lda,
+                    const float* b_hi, const float* b_lo, int64_t ldb, float* c, int64_t ldc, int flags,
+                    int* status, cudaStream_t stream);
 namespace {
 
 using namespace row_window;
+constexpr int GT_ADD = 32;
 
 template <int R>
 __global__ void __launch_bounds__(BLOCK_THREADS, (R == 1 ? 4 : 3))
@@ -245,4 +251,68 @@ extern "C" int hi2_refine_prepare(const float* w, int64_t ldw, const uint8_t* co
   refine_prepare_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
       w, ldw, codes, params, consts, block == 16 ? 4 : block == 32 ? 5 : 6, n_rows, k, c, lo_x, st_x, e, e_lo);
   return check_launch("refine_prepare");
+}
+
+extern "C" int hi2_refine_sweep(float* g, float* c, const float* lo, const float* st, const float* top, const float* hs,
+                                const float* hs_split, float* moves, int64_t n_rows, int64_t k, int64_t width, int last,
+                                int32_t* moved, int32_t* status, void* stream) {
+  using namespace hi2;
+  HI2_REQUIRE(k > 0 && k % 16 == 0, "refine_sweep: k must be a positive multiple of 16");
+  HI2_REQUIRE(width >= LMAX && width % LMAX == 0, "refine_sweep: width must be a multiple of 128");
+  if (n_rows == 0) return HI2_OK;
+  HI2_REQUIRE(g && c && lo && st && top && hs && moves && (hs_split == nullptr || status), "refine_sweep: null pointer");
+  HI2_REQUIRE(aligned16(g) && aligned16(c) && aligned16(lo) && aligned16(st) && aligned16(hs) && aligned16(moves) &&
+                  (hs_split == nullptr || aligned16(hs_split)),
+              "refine_sweep: buffers must be 16-byte aligned");
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  ChainGraph chain(s, 2 * ceil_div(k, (int64_t)LMAX));
+  auto enqueue = [&]() -> int {
+    int rc;
+    if (hs_split == nullptr) {  // fp32 FMA products, block by block
+      for (int64_t b0 = 0; b0 < k; b0 += LMAX) {
+        const int64_t b1 = b0 + LMAX < k ? b0 + LMAX : k, first = last ? b1 : 0;
+        const int len = (int)(b1 - b0);
+        rc = launch_refine_block(g + b0, k, len, c, lo, st, top, hs, n_rows, k, b0, moves, nullptr, len, moved, s);
+        if (rc != HI2_OK) return rc;
+        if (first >= k) continue;
+        GemmArgs<float, float, float> p;
+        p.m = n_rows, p.n = k - first, p.kk = len, p.alpha = 1.0f, p.beta = 1.0f;
+        p.a = moves, p.lda = len, p.b = hs + b0 * k + first, p.ldb = k, p.c = g + first, p.ldc = k, p.flags = 0;
+        rc = launch_gemm_async<float, 8, 8, 16>(false, false, p, s, "refine_sweep");
+        if (rc != HI2_OK) return rc;
+      }
+      return HI2_OK;
+    }
+    // Tensor-core products.  After a block the rest of its group needs its moves now; the columns outside
+    // the group take the whole group's in one product; the group's own columns at or before each block
+    // are needed by the next sweep only.  hs is symmetric: its rows are the K-major right operand.
+    const int64_t ldm = width < k ? width : k;
+    float *hi = moves, *lo_part = moves + n_rows * ldm;
+    int* word = reinterpret_cast<int*>(status);
+    auto product = [&](int64_t b0, int64_t b1, int64_t g0, int64_t c0, int64_t c1) -> int {  // g[:, c0:c1] += moves of [b0, b1)
+      if (c0 >= c1) return HI2_OK;
+      return launch_gemm_tc2(n_rows, c1 - c0, b1 - b0, hi + (b0 - g0), lo_part + (b0 - g0), ldm, hs_split + c0 * k + b0,
+                             hs_split + k * k + c0 * k + b0, k, g + c0, k, GT_ADD, word, s);
+    };
+    for (int64_t g0 = 0; g0 < k; g0 += width) {
+      const int64_t g1 = g0 + width < k ? g0 + width : k;
+      for (int64_t b0 = g0; b0 < g1; b0 += LMAX) {
+        const int64_t b1 = b0 + LMAX < g1 ? b0 + LMAX : g1;
+        rc = launch_refine_block(g + b0, k, (int)(b1 - b0), c, lo, st, top, hs, n_rows, k, b0, hi + (b0 - g0),
+                                 lo_part + (b0 - g0), ldm, moved, s);
+        if (rc != HI2_OK) return rc;
+        if ((rc = product(b0, b1, g0, b1, g1)) != HI2_OK) return rc;
+      }
+      if (width == LMAX) {  // groups of one block: the whole update in one product
+        if ((rc = product(g0, g1, g0, last ? g1 : 0, k)) != HI2_OK) return rc;
+        continue;
+      }
+      if (!last && (rc = product(g0, g1, g0, 0, g0)) != HI2_OK) return rc;
+      if ((rc = product(g0, g1, g0, g1, k)) != HI2_OK) return rc;
+      for (int64_t b0 = g0; b0 < g1 && !last; b0 += LMAX)
+        if ((rc = product(b0, g1, g0, b0, b0 + LMAX < g1 ? b0 + LMAX : g1)) != HI2_OK) return rc;
+    }
+    return HI2_OK;
+  };
+  return chain.finish(enqueue(), "refine_sweep");
 }

@@ -67,7 +67,7 @@ def _run(c, lo_x, st_x, top, e: list, hs, passes: int, use_tc: bool, wait: bool)
         raise RuntimeError(f"refine kernel unavailable on {dev}: {refine_kernel.failure()}")
     n_rows, k = c.shape
     g = torch.empty(n_rows, k, dtype=torch.float32, device=dev)
-    status = None
+    status = hs_split = None
     if use_tc:
         status = torch.zeros(1, dtype=torch.int32, device=dev)
         hs_split = refine_kernel.split_tf32(hs)
@@ -84,47 +84,12 @@ def _run(c, lo_x, st_x, top, e: list, hs, passes: int, use_tc: bool, wait: bool)
     # every step a latency chain, where more launches cost more than the better products gain: then
     # a group is one block and its update one product.
     width = (GROUP_BLOCKS if n_rows * k >= GROUP_MIN_ELEMS else 1) * BLOCK_COLUMNS
-    moves = torch.empty(2, n_rows, min(width, k), dtype=torch.float32, device=dev) if use_tc else None
-    moved = torch.zeros(1, dtype=torch.int32, device=dev) if wait and use_tc else None
+    moves = torch.empty(*((2, n_rows, min(width, k)) if use_tc else (n_rows, BLOCK_COLUMNS)), dtype=torch.float32, device=dev)
+    moved = torch.zeros(1, dtype=torch.int32, device=dev) if wait else None
     for sweep in range(passes):
-        last = sweep + 1 == passes  # nobody reads g behind it: only the columns still to come are updated
-        follow = wait and not last  # whether the next sweep is worth queueing
-        start = c.clone() if follow and not use_tc else None
-        if not use_tc:
-            for b0 in range(0, k, BLOCK_COLUMNS):
-                b1 = min(b0 + BLOCK_COLUMNS, k)
-                gb = g[:, b0:b1].contiguous()
-                dw_block = torch.empty(n_rows, b1 - b0, dtype=torch.float32, device=dev)
-                refine_kernel.refine_block(gb, c, lo_x, st_x, top, hs, b0, b1 - b0, dw_block)
-                first = b1 if last else 0
-                if first < k:
-                    refine_kernel.gemm(dw_block, hs[b0:b1, first:], g[:, first:], alpha=1.0, beta=1.0)
-            if follow and bool((c == start).all()):
-                break
-            continue
-        for g0 in range(0, k, width):
-            g1 = min(g0 + width, k)
-            for b0 in range(g0, g1, BLOCK_COLUMNS):
-                b1 = min(b0 + BLOCK_COLUMNS, g1)
-                dw = moves[:, :, b0 - g0 : b1 - g0]
-                refine_kernel.refine_block_in_place(g, c, lo_x, st_x, top, hs, b0, b1 - b0, dw, moved)
-                if b1 < g1:
-                    refine_kernel.gemm_tc(dw, hs_split[:, b1:g1, b0:b1], g[:, b1:g1], status, accumulate=True)
-            group = moves[:, :, : g1 - g0]
-            if width == BLOCK_COLUMNS:  # groups of one block: the whole update in one product
-                first = g1 if last else 0
-                if first < k:
-                    refine_kernel.gemm_tc(group, hs_split[:, first:, g0:g1], g[:, first:], status, accumulate=True)
-                continue
-            if g0 > 0 and not last:
-                refine_kernel.gemm_tc(group, hs_split[:, :g0, g0:g1], g[:, :g0], status, accumulate=True)
-            if g1 < k:
-                refine_kernel.gemm_tc(group, hs_split[:, g1:, g0:g1], g[:, g1:], status, accumulate=True)
-            for b0 in range(g0, g1, BLOCK_COLUMNS) if not last else ():
-                b1 = min(b0 + BLOCK_COLUMNS, g1)
-                refine_kernel.gemm_tc(moves[:, :, b0 - g0 : g1 - g0], hs_split[:, b0:b1, b0:g1], g[:, b0:b1], status,
-                                      accumulate=True)
-        if follow:
+        last = sweep + 1 == passes  # nobody reads g behind it
+        refine_kernel.sweep(g, c, lo_x, st_x, top, hs, hs_split, moves, width, last, moved, status)
+        if wait and not last:  # whether the next sweep is worth queueing
             if not int(moved.item()):
                 break
             moved.zero_()

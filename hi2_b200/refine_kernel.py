@@ -68,6 +68,25 @@ def refine_block_in_place(g, c, lo_x, st_x, top, hs, b0, length, dw_split, moved
     )
 
 
+def sweep(g, c, lo_x, st_x, top, hs, hs_split, moves, width: int, last: bool, moved, status) -> None:
+    """One whole sweep over the columns in one call: block kernels and the products that keep ``g [N, K]``
+    up to date.  ``hs_split [2, K, K]`` (TF32 parts) selects the tensor-core products, ``None`` the fp32
+    ones; ``moves`` is scratch (``[2, N, min(width, K)]``, or ``[N, 128]``).  ``last``: ``g`` is not needed behind the
+    sweep.  ``moved`` and ``status``: device int32 words, or None."""
+    dev = _lib.need_cuda(g, c, lo_x, st_x, top, hs, hs_split, moves, moved, status)
+    n, k = c.shape
+    for t, shape, name in ((g, (n, k), "g"), (c, (n, k), "c"), (lo_x, (n, k), "lo_x"), (st_x, (n, k), "st_x"), (top, (n,), "top"),
+                           (hs, (k, k), "hs"), (hs_split, (2, k, k), "hs_split"), (moves, None, "moves")):
+        if t is not None and (t.dtype != torch.float32 or not t.is_contiguous() or (shape is not None and tuple(t.shape) != shape)):
+            raise ValueError(f"sweep: {name} must be a contiguous float32 tensor of shape {shape}")
+    if moves.numel() < (2 * n * min(width, k) if hs_split is not None else n * min(BLOCK_COLUMNS, k)):
+        raise ValueError("sweep: moves is too small")
+    _lib.call(
+        "hi2_refine_sweep", _lib.ptr(g), _lib.ptr(c), _lib.ptr(lo_x), _lib.ptr(st_x), _lib.ptr(top), _lib.ptr(hs), _lib.ptr(hs_split),
+        _lib.ptr(moves), n, k, int(width), 1 if last else 0, _lib.ptr(moved), _lib.ptr(status), _lib.stream(dev),
+    )
+
+
 def prepare(w, codes, params, consts, block, c, lo_x, st_x, e, e_lo=None) -> None:
     """Fill ``c``, ``lo_x``, ``st_x [N, K]`` (fp32) with the codes and the ladder of every column of rows
     encoded at one ``block``, and ``e`` (with ``e_lo``: its TF32 parts) with the error of the decoded

@@ -226,6 +226,15 @@ int hi2_refine_block_in_place(const float* g, int len, float* c, const float* lo
 int hi2_refine_sweep_block(const float* g, int len, float* c, const float* lo, const float* st, const float* top,
                            const float* hs, int64_t n_rows, int64_t k, int64_t b0, float* dw_hi, float* dw_lo,
                            int64_t lddw, int32_t* moved, void* stream);
+/* One whole sweep (hi2/refine.py:60-106): every block of 128 columns decided and g [n_rows, k] brought up
+ * to date.  hs_split [2, k, k], the TF32 parts of hs, selects the tensor-core products (null: fp32 FMA);
+ * moves is scratch, [2, n_rows, min(width, k)] with hs_split, else [n_rows, 128].  width (a multiple of
+ * 128): columns whose moves reach the columns outside them in one product.  last: g is not needed behind
+ * this sweep, and only the columns still to come are updated.  *moved (or null) is set to 1 if a code
+ * moved; *status (with hs_split) is raised by a bounded wait that ran out. */
+int hi2_refine_sweep(float* g, float* c, const float* lo, const float* st, const float* top, const float* hs,
+                     const float* hs_split, float* moves, int64_t n_rows, int64_t k, int64_t width, int last,
+                     int32_t* moved, int32_t* status, void* stream);
 /* What a sweep starts from (hi2/refine.py:44-60), for rows rounded at one block size: fp32 codes c, the
  * decoded ladder of every column lo_x, st_x, and e = fp16(lo + c * step) - w, as it is (e_lo null) or as
  * its TF32 parts.  w fp32 [n_rows, k] (ldw); codes u8 [n_rows, k], params u8 [n_rows, k / block, 2],
