@@ -53,6 +53,9 @@ SIGNATURES = {
         _I,
         [_P, _L, _L, _P, _P, _P, _P, _P, _L, _P, _P, _P, _P, _P, _I, _P, _P, _P, _P],
     ),
+    "hi2_rotate_groups_host_flags": (_I, [_P, _I, _P, _I, _P, _P, _L, _L, _P]),
+    "hi2_transform_sigma_host_flags": (_I, [_P, C.c_float, _P, _P, _L, _P, _P, _P]),
+    "hi2_column_weights": (_I, [_P, C.c_double, _P, _P, _L, _P, _P]),
     "hi2_error_table": (_I, [_P, _L, _P, _P, _P, _I, _I, _I, _P, _P, _L, _L, _P, _P, _P, _P, _P]),
     "hi2_gptq_round_tc_grouped": (
         _I,
@@ -224,3 +227,14 @@ def host_i64(values):
 
 def host_i32(values):
     return (C.c_int32 * len(values))(*[int(v) for v in values])
+
+
+HOST_FLAG_GROUPS = 8192  # groups whose flags fit a kernel's arguments
+
+
+def host_flags(flags: torch.Tensor) -> torch.Tensor | None:
+    """``flags`` as contiguous uint8 in host memory, ready to travel as kernel arguments; None when they
+    live on the device, are too many, or are of a type whose values would not survive."""
+    if flags.is_cuda or flags.numel() > HOST_FLAG_GROUPS or flags.dtype not in (torch.uint8, torch.bool):
+        return None
+    return flags.contiguous().view(torch.uint8)

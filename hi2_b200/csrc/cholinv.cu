@@ -597,6 +597,13 @@ __global__ void merge_status_kernel(const int* status, int32_t* info) {
   if (*status != 0) *info = -1;
 }
 
+// Launches of F on n rows, for the chain's choice between a graph and plain launches.
+int64_t chain_length(int64_t n) {
+  if (n <= BASE) return 1;
+  const int64_t n1 = top_half(n), n2 = n - n1;
+  return chain_length(n1) + chain_length(n2) + (n2 >= HI2_FACTOR_TC_MIN ? 13 : 3);
+}
+
 int factor(const Plan& pl, int64_t off, int64_t n) {
   const int64_t ld = pl.ld;
   if (n <= BASE) {
@@ -688,8 +695,7 @@ extern "C" int hi2_inverse_factor(const float* hs, const float* lam, int64_t k, 
   pl.x = pl.a + k * pl.ld;
   pl.split = split_floats(k) ? pl.x + k * pl.ld : nullptr;
   pl.k = k, pl.info = info, pl.stream = s;
-  // the whole recursion (K/64 leaves and the products between them) goes to the stream as one graph
-  ChainGraph chain(s);
+  ChainGraph chain(s, chain_length(k));  // the whole recursion
   auto enqueue = [&]() -> int {
     if (cudaMemsetAsync(pl.status, 0, 256, s) != cudaSuccess)
       return fail(HI2_ERR_LAUNCH, "inverse_factor: memset failed");

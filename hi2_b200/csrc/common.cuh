@@ -80,6 +80,31 @@ inline void launch_link(void (*kernel)(Params...), dim3 grid, dim3 block, size_t
 __device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// One flag per 16-column group: an array on the device, or bits in the kernel's own arguments for a caller
+// whose flags are on the host (they decide a few hundred bits; a copy to the device cost 25 us of host
+// time per call).
+struct GroupFlags {
+  static constexpr int64_t MAX_GROUPS = 8192;
+  const uint8_t* device;
+  uint32_t bits[MAX_GROUPS / 32];
+
+  static GroupFlags on_device(const uint8_t* flags) {
+    GroupFlags f;
+    f.device = flags;
+    return f;
+  }
+  static GroupFlags on_host(const uint8_t* flags, int64_t groups) {
+    GroupFlags f;
+    f.device = nullptr;
+    for (int64_t i = 0; i < MAX_GROUPS / 32; ++i) f.bits[i] = 0;
+    for (int64_t g = 0; g < groups; ++g) f.bits[g >> 5] |= (flags[g] != 0 ? 1u : 0u) << (g & 31);
+    return f;
+  }
+  __device__ __forceinline__ bool on(int64_t g) const {
+    return device != nullptr ? __ldg(device + g) != 0 : ((bits[g >> 5] >> (g & 31)) & 1u) != 0;
+  }
+};
+
 #define HI2_REQUIRE(cond, msg)                         \
   do {                                                 \
     if (!(cond)) return ::hi2::fail(HI2_ERR_ARG, msg); \

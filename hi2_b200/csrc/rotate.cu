@@ -99,7 +99,7 @@ __device__ __forceinline__ double fma_c(double a, double b, double c) { return f
 // Tin == Tout (C = compute type of the pair) or Tin half/bf16 with Tout float.
 template <typename Tin, typename Tout, bool kSameType>
 __global__ void __launch_bounds__(256)
-rotate_kernel(const Tin* __restrict__ x, Tout* __restrict__ y, const uint8_t* __restrict__ flags,
+rotate_kernel(const Tin* __restrict__ x, Tout* __restrict__ y, const __grid_constant__ GroupFlags flags,
               const float* __restrict__ col_scale, int64_t groups, int groups_per_row) {
   using C = typename std::conditional<kSameType, typename Quad<Tin>::C, float>::type;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -135,7 +135,7 @@ rotate_kernel(const Tin* __restrict__ x, Tout* __restrict__ y, const uint8_t* __
         }
       }
     }
-    if (__ldg(flags + g) != 0) {
+    if (flags.on(g)) {
       // All 16 outputs of the group, each the k-ascending sum.  (Measured alternatives, all slower on
       // the 11008 x 4096 bf16 -> fp32 case at 72 us: four lanes per group with shuffles 82 us; two
       // groups per trip, 96 registers, 81 us; four outputs at a time capped at 40 registers 85 us.)
@@ -157,7 +157,7 @@ rotate_kernel(const Tin* __restrict__ x, Tout* __restrict__ y, const uint8_t* __
 }
 
 template <typename Tin, typename Tout, bool kSame>
-int launch(const void* x, void* y, const uint8_t* flags, const float* scale, int64_t rows, int64_t k,
+int launch(const void* x, void* y, const GroupFlags& flags, const float* scale, int64_t rows, int64_t k,
            cudaStream_t stream) {
   const int64_t groups = rows * k / 16;
   if (groups == 0) return HI2_OK;
@@ -169,16 +169,9 @@ int launch(const void* x, void* y, const uint8_t* flags, const float* scale, int
   return check_launch("rotate_groups");
 }
 
-}  // namespace
-}  // namespace hi2
-
-extern "C" int hi2_rotate_groups(const void* x, int in_dtype, void* y, int out_dtype,
-                                 const uint8_t* flags, const float* col_scale, int64_t rows,
-                                 int64_t k, void* stream) {
-  using namespace hi2;
-  HI2_REQUIRE(rows >= 0 && k > 0 && k % 16 == 0, "rotate_groups: k must be a positive multiple of 16");
-  if (rows == 0) return HI2_OK;
-  HI2_REQUIRE(x && y && flags, "rotate_groups: null pointer");
+int rotate(const void* x, int in_dtype, void* y, int out_dtype, const GroupFlags& flags, const float* col_scale,
+           int64_t rows, int64_t k, void* stream) {
+  HI2_REQUIRE(x && y, "rotate_groups: null pointer");
   HI2_REQUIRE(aligned16(x) && aligned16(y), "rotate_groups: x and y must be 16-byte aligned");
   HI2_REQUIRE(col_scale == nullptr || aligned16(col_scale), "rotate_groups: col_scale alignment");
   HI2_REQUIRE(col_scale == nullptr || out_dtype == HI2_F32,
@@ -197,4 +190,28 @@ extern "C" int hi2_rotate_groups(const void* x, int in_dtype, void* y, int out_d
   if (in_dtype == HI2_BF16 && out_dtype == HI2_F32)
     return launch<__nv_bfloat16, float, false>(x, y, flags, col_scale, rows, k, s);
   return fail(HI2_ERR_ARG, "rotate_groups: unsupported dtype pair");
+}
+
+}  // namespace
+}  // namespace hi2
+
+extern "C" int hi2_rotate_groups(const void* x, int in_dtype, void* y, int out_dtype,
+                                 const uint8_t* flags, const float* col_scale, int64_t rows,
+                                 int64_t k, void* stream) {
+  using namespace hi2;
+  HI2_REQUIRE(rows >= 0 && k > 0 && k % 16 == 0, "rotate_groups: k must be a positive multiple of 16");
+  if (rows == 0) return HI2_OK;
+  HI2_REQUIRE(flags, "rotate_groups: null pointer");
+  return rotate(x, in_dtype, y, out_dtype, GroupFlags::on_device(flags), col_scale, rows, k, stream);
+}
+
+extern "C" int hi2_rotate_groups_host_flags(const void* x, int in_dtype, void* y, int out_dtype,
+                                            const uint8_t* flags_host, const float* col_scale, int64_t rows,
+                                            int64_t k, void* stream) {
+  using namespace hi2;
+  HI2_REQUIRE(rows >= 0 && k > 0 && k % 16 == 0, "rotate_groups: k must be a positive multiple of 16");
+  HI2_REQUIRE(k / 16 <= GroupFlags::MAX_GROUPS, "rotate_groups: too many groups for host flags");
+  if (rows == 0) return HI2_OK;
+  HI2_REQUIRE(flags_host, "rotate_groups: null pointer");
+  return rotate(x, in_dtype, y, out_dtype, GroupFlags::on_host(flags_host, k / 16), col_scale, rows, k, stream);
 }

@@ -52,7 +52,7 @@ __device__ __forceinline__ void load_tile(float4 (&quad)[4], const float* __rest
 // Tile (tr, tc) of sigma/denom (already in `quad`) scaled by inv[row]*inv[col], then M . M^T on
 // flagged groups.
 __device__ void transform_tile(float (*tile)[LD], const float4 (&quad)[4], float denom,
-                               const float* __restrict__ inv_s, const uint8_t* __restrict__ had,
+                               const float* __restrict__ inv_s, const GroupFlags& had,
                                int64_t k, int64_t tr, int64_t tc) {
   const int tid = threadIdx.x;
   const int64_t r0 = tr * TS, c0 = tc * TS;
@@ -72,7 +72,7 @@ __device__ void transform_tile(float (*tile)[LD], const float4 (&quad)[4], float
   {  // left product: thread = (column c, row group gi)
     const int c = tid & 63, gi = tid >> 6;
     const int64_t grp = (r0 >> 4) + gi;
-    if (grp * 16 < k && had[grp]) {
+    if (grp * 16 < k && had.on(grp)) {
       float v[16];
 #pragma unroll
       for (int j = 0; j < 16; ++j) v[j] = tile[gi * 16 + j][c];
@@ -85,7 +85,7 @@ __device__ void transform_tile(float (*tile)[LD], const float4 (&quad)[4], float
   {  // right product: thread = (row i, column group gj)
     const int i = tid & 63, gj = tid >> 6;
     const int64_t grp = (c0 >> 4) + gj;
-    if (grp * 16 < k && had[grp]) {
+    if (grp * 16 < k && had.on(grp)) {
       float v[16];
 #pragma unroll
       for (int q = 0; q < 16; ++q) v[q] = tile[i][gj * 16 + q];
@@ -99,7 +99,7 @@ __device__ void transform_tile(float (*tile)[LD], const float4 (&quad)[4], float
 
 __global__ void __launch_bounds__(256)
 transform_sigma_kernel(const float* __restrict__ sigma, float denom,
-                       const uint16_t* __restrict__ col_scale, const uint8_t* __restrict__ had,
+                       const uint16_t* __restrict__ col_scale, const __grid_constant__ GroupFlags had,
                        int64_t k, float* __restrict__ hs, float* __restrict__ diag) {
   const int64_t bi = blockIdx.y, bj = blockIdx.x;
   if (bi > bj) return;
@@ -229,18 +229,86 @@ extern "C" int hi2_group_moments_update(const void* x, int dtype, int64_t tokens
   return check_launch("group_moments_update");
 }
 
+namespace hi2 {
+namespace {
+int transform(const float* sigma, float denom, const uint16_t* col_scale, const GroupFlags& had, int64_t k, float* hs,
+              float* diag, void* stream) {
+  HI2_REQUIRE(sigma && hs, "transform_sigma: null pointer");
+  HI2_REQUIRE(sigma != hs, "transform_sigma: in-place operation is not supported");
+  HI2_REQUIRE(denom > 0.0f, "transform_sigma: denom must be positive");
+  const unsigned nt = (unsigned)ceil_div(k, TS);
+  transform_sigma_kernel<<<dim3(nt, nt), 256, 0, static_cast<cudaStream_t>(stream)>>>(sigma, denom, col_scale, had, k, hs,
+                                                                                      diag);
+  return check_launch("transform_sigma");
+}
+
+// The ladder weights of the columns, from the 16 x 16 group moments: the diagonal of T M T^T per flagged
+// group, of M per other group, M = S / n scaled by inv on rows and then on columns.  A thread per column,
+// sixteen groups per block staged in shared memory; fp64 as the moments are, rounded once.  (Eleven
+// elementwise and batched-product launches of a few microseconds each before.)
+__global__ void __launch_bounds__(256)
+column_weights_kernel(const double* __restrict__ s, double n, const float* __restrict__ inv,
+                      const __grid_constant__ GroupFlags flags, bool flagged, int64_t groups, float* __restrict__ out) {
+  __shared__ double m[16][257];
+  const int64_t g0 = (int64_t)blockIdx.x * 16;
+  for (int idx = threadIdx.x; idx < 16 * 256; idx += 256) {
+    const int g = idx >> 8, j = (idx >> 4) & 15, k = idx & 15;
+    if (g0 + g >= groups) continue;
+    double v = s[(g0 + g) * 256 + (idx & 255)] / n;
+    if (inv != nullptr) v = v * (double)inv[(g0 + g) * 16 + j] * (double)inv[(g0 + g) * 16 + k];
+    m[g][idx & 255] = v;
+  }
+  __syncthreads();
+  const int g = threadIdx.x >> 4, i = threadIdx.x & 15;
+  if (g0 + g >= groups) return;
+  double acc;
+  if (flagged && flags.on(g0 + g)) {
+    acc = 0.0;
+#pragma unroll 4
+    for (int j = 0; j < 16; ++j) {
+      double row = 0.0;
+#pragma unroll
+      for (int k = 0; k < 16; ++k) row += (__popc(k & i) & 1) ? -m[g][j * 16 + k] : m[g][j * 16 + k];
+      acc += (__popc(j & i) & 1) ? -row : row;
+    }
+    acc *= 0.0625;
+  } else {
+    acc = m[g][i * 17];
+  }
+  out[(g0 + g) * 16 + i] = (float)acc;
+}
+}  // namespace
+}  // namespace hi2
+
 extern "C" int hi2_transform_sigma(const float* sigma, float denom, const uint16_t* col_scale,
                                    const uint8_t* had, int64_t k, float* hs, float* diag,
                                    void* stream) {
   using namespace hi2;
   HI2_REQUIRE(k > 0 && k % 16 == 0, "transform_sigma: k must be a positive multiple of 16");
-  HI2_REQUIRE(sigma && had && hs, "transform_sigma: null pointer");
-  HI2_REQUIRE(sigma != hs, "transform_sigma: in-place operation is not supported");
-  HI2_REQUIRE(denom > 0.0f, "transform_sigma: denom must be positive");
-  const unsigned nt = (unsigned)ceil_div(k, TS);
-  transform_sigma_kernel<<<dim3(nt, nt), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      sigma, denom, col_scale, had, k, hs, diag);
-  return check_launch("transform_sigma");
+  HI2_REQUIRE(had, "transform_sigma: null pointer");
+  return transform(sigma, denom, col_scale, GroupFlags::on_device(had), k, hs, diag, stream);
+}
+
+extern "C" int hi2_transform_sigma_host_flags(const float* sigma, float denom, const uint16_t* col_scale,
+                                              const uint8_t* had_host, int64_t k, float* hs, float* diag, void* stream) {
+  using namespace hi2;
+  HI2_REQUIRE(k > 0 && k % 16 == 0, "transform_sigma: k must be a positive multiple of 16");
+  HI2_REQUIRE(k / 16 <= GroupFlags::MAX_GROUPS, "transform_sigma: too many groups for host flags");
+  HI2_REQUIRE(had_host, "transform_sigma: null pointer");
+  return transform(sigma, denom, col_scale, GroupFlags::on_host(had_host, k / 16), k, hs, diag, stream);
+}
+
+extern "C" int hi2_column_weights(const double* s, double n, const float* inv, const uint8_t* flags_host, int64_t k,
+                                  float* out, void* stream) {
+  using namespace hi2;
+  HI2_REQUIRE(k > 0 && k % 16 == 0, "column_weights: k must be a positive multiple of 16");
+  HI2_REQUIRE(k / 16 <= GroupFlags::MAX_GROUPS, "column_weights: too many groups for host flags");
+  HI2_REQUIRE(s && out && n > 0.0, "column_weights: null pointer or empty moment");
+  const int64_t groups = k / 16;
+  const GroupFlags flags = flags_host ? GroupFlags::on_host(flags_host, groups) : GroupFlags::on_device(nullptr);
+  column_weights_kernel<<<(unsigned)ceil_div(groups, (int64_t)16), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+      s, n, inv, flags, flags_host != nullptr, groups, out);
+  return check_launch("column_weights");
 }
 
 extern "C" int hi2_group_moments(const float* s, int64_t k, double* g, void* stream) {

@@ -52,13 +52,16 @@ def fwht_groups(x: torch.Tensor, flags: torch.Tensor, col_scale: torch.Tensor | 
         if out.shape != xc.shape or out.dtype != out_dtype or out.device != dev or not out.is_contiguous():
             raise ValueError("fwht_groups: out must be a contiguous tensor of the result's shape, dtype and device")
         y = out
-    fl = _lib.upload(flags, dev, torch.uint8)
+    fl = _lib.host_flags(flags)
+    name = "hi2_rotate_groups_host_flags"
+    if fl is None:
+        fl, name = _lib.upload(flags, dev, torch.uint8), "hi2_rotate_groups"
     cs = None
     if col_scale is not None:
         cs = _lib.upload(col_scale, dev, torch.float32)
     rows = xc.numel() // k
     _lib.call(
-        "hi2_rotate_groups", _lib.ptr(xc), _lib.DTYPES[x.dtype], _lib.ptr(y), _lib.DTYPES[out_dtype],
+        name, _lib.ptr(xc), _lib.DTYPES[x.dtype], _lib.ptr(y), _lib.DTYPES[out_dtype],
         _lib.ptr(fl), _lib.ptr(cs), rows, k, _lib.stream(dev),
     )
     return y

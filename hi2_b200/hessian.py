@@ -163,11 +163,13 @@ def transform_sigma(sigma: torch.Tensor, col_scale: torch.Tensor | None, had: to
     cs = None
     if col_scale is not None:
         cs = _lib.upload(col_scale, dev, torch.float16)
-    flags = _lib.upload(had, dev, torch.uint8)
-    if flags.numel() != k // GROUP:
-        raise ValueError(f"had has {flags.numel()} entries, expected {k // GROUP}")
+    if had.numel() != k // GROUP:
+        raise ValueError(f"had has {had.numel()} entries, expected {k // GROUP}")
+    flags, name = _lib.host_flags(had), "hi2_transform_sigma_host_flags"
+    if flags is None:
+        flags, name = _lib.upload(had, dev, torch.uint8), "hi2_transform_sigma"
     _lib.call(
-        "hi2_transform_sigma", _lib.ptr(s), float(denom), _lib.ptr(cs), _lib.ptr(flags), k,
+        name, _lib.ptr(s), float(denom), _lib.ptr(cs), _lib.ptr(flags), k,
         _lib.ptr(hs), _lib.ptr(diag), _lib.stream(dev),
     )
     return (hs, diag) if return_diag else hs

@@ -71,8 +71,19 @@ class ColumnStats:
         rotated: the diagonal of ``T_g M_g T_g^T`` per group, ``M_g`` the group's mean moment and
         ``T_g`` the rotation (or the identity).  fp64 throughout, returned as fp32 ``[K]``
         (hi2/stats.py:39-54)."""
+        dev = self.S.device
+        fl = None if flags is None else _lib.host_flags(flags)
+        if (self.S.is_cuda and self.S.dtype == torch.float64 and self.S.is_contiguous() and self.k // GROUP <= _lib.HOST_FLAG_GROUPS
+                and (flags is None or (fl is not None and fl.numel() == self.k // GROUP))
+                and (inv_scale is None or (inv_scale.device == dev and inv_scale.dtype == torch.float32
+                                           and inv_scale.numel() == self.k))):
+            inv = None if inv_scale is None else inv_scale.contiguous()
+            out = torch.empty(self.k, dtype=torch.float32, device=dev)
+            _lib.call("hi2_column_weights", _lib.ptr(self.S), float(max(self.n, 1)), _lib.ptr(inv), _lib.ptr(fl), self.k,
+                      _lib.ptr(out), _lib.stream(dev))
+            return out
+        # statistics of another type or on the host, flags on the device: the same in elementwise steps
         moment = self.S / max(self.n, 1)
-        dev = moment.device
         if inv_scale is not None:
             # scale first (rows, then columns), then rotate: the order the reference rounds in
             v = inv_scale.to(dev, moment.dtype).reshape(-1, GROUP)

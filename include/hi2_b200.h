@@ -54,6 +54,10 @@ long long hi2_graph_launch_count(void);
  * output summed in ascending k; half types in fp64 with one final rounding. */
 int hi2_rotate_groups(const void* x, int in_dtype, void* y, int out_dtype, const uint8_t* flags,
                       const float* col_scale, int64_t rows, int64_t k, void* stream);
+/* The same with the flags in host memory (k <= 131072): they travel as kernel arguments. */
+int hi2_rotate_groups_host_flags(const void* x, int in_dtype, void* y, int out_dtype, const uint8_t* flags_host,
+                                 const float* col_scale, int64_t rows, int64_t k, void* stream);
+
 
 /* ---- packing -------------------------------------------------------------------------------
  * hi2/format.py:73-85 pack_codes: n codes per row -> n*nbits/32 int32 words, first code in the
@@ -290,6 +294,15 @@ int hi2_group_moments_update(const void* x, int dtype, int64_t tokens, int64_t k
  * col_scale fp16 [k] or null, had u8 [k/16], diag (fp32 [k], may be null) receives diag(hs). */
 int hi2_transform_sigma(const float* sigma, float denom, const uint16_t* col_scale,
                         const uint8_t* had, int64_t k, float* hs, float* diag, void* stream);
+/* The same with the flags in host memory (k <= 131072). */
+int hi2_transform_sigma_host_flags(const float* sigma, float denom, const uint16_t* col_scale,
+                                   const uint8_t* had_host, int64_t k, float* hs, float* diag, void* stream);
+/* hi2/stats.py:39-54: out [k] = diag(T M T^T) per 16-column group, M = s / n with rows and columns scaled by
+ * inv [k] (or null), T the rotation for groups flagged in flags_host (null: none), the identity otherwise;
+ * s fp64 [k / 16, 16, 16].  k <= 131072. */
+int hi2_column_weights(const double* s, double n, const float* inv, const uint8_t* flags_host, int64_t k,
+                       float* out, void* stream);
+
 
 /* hi2/hessian.py:71-86 inverse_factor, one damping attempt: u = upper Cholesky factor of
  * (hs + *lam * I)^-1 with lam a device fp32 scalar.  *info (device int, caller zeroes it) is
