@@ -298,8 +298,8 @@ __device__ __forceinline__ void fit_tile(FitShared& shared, int64_t row_tile, in
   if (GROUPED) {
     d = d_all + (int64_t)row_d[row_c] * (nb * B) + blk * B;
   } else {
-    for (int t = lane; t < B / 4; t += 32)
-      reinterpret_cast<float4*>(shared.d[warp])[t] = __ldg(reinterpret_cast<const float4*>(d_all + blk * B) + t);
+    // one weight per lane: hi2_ladder_grid's weights may start at any float
+    for (int t = lane; t < B; t += 32) shared.d[warp][t] = __ldg(d_all + blk * B + t);
     __syncwarp();
     d = shared.d[warp];
   }
