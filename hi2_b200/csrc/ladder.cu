@@ -543,6 +543,10 @@ __device__ __forceinline__ void quantise_block(const RowConstants& c, float lo, 
 constexpr int ROW_THREADS = 256;
 constexpr int ROW_WARPS = ROW_THREADS / 32;
 constexpr int ROW_UN = 4;  // quads a lane loads before it computes
+// Shared memory a row pass may ask for.  A kernel's limit is set to this and never to what one call needs: it
+// is one setting for all threads of the process, and a thread that lowered it between another's setting and
+// launch made that launch fail.
+constexpr int ROW_SMEM_MAX = 200 * 1024;
 
 // One WARP per row: the row-wide extrema, the constants and the parameter bytes need only warp
 // shuffles, so no thread block barrier sits between the phases of a row and 64 rows are in flight
@@ -905,7 +909,7 @@ extern "C" int hi2_quantize_rows_grouped(const float* lo, const float* step, con
   HI2_REQUIRE((lo_d == nullptr && step_d == nullptr) || ldp >= k / block, "quantize_rows: ldp");
   const int64_t nb = k / block;
   const size_t smem = (size_t)ROW_WARPS * (2 * nb) * sizeof(float);
-  HI2_REQUIRE(smem <= 200 * 1024, "quantize_rows: k too large for the ladder cache");
+  HI2_REQUIRE(smem <= (size_t)ROW_SMEM_MAX, "quantize_rows: k too large for the ladder cache");
   const int64_t want = ceil_div(n_rows, (int64_t)ROW_WARPS);
   const unsigned grid = (unsigned)(want < 148 * 8 ? want : 148 * 8);
   const float nmax = (float)((1 << nbits) - 1);
@@ -914,7 +918,7 @@ extern "C" int hi2_quantize_rows_grouped(const float* lo, const float* step, con
   do {                                                                                                     \
     if (smem > 48 * 1024 &&                                                                                \
         cudaFuncSetAttribute(row_kernel<BB, CC, EE>, cudaFuncAttributeMaxDynamicSharedMemorySize,          \
-                             (int)smem) != cudaSuccess)                                                    \
+                             ROW_SMEM_MAX) != cudaSuccess)                                                 \
       return fail(HI2_ERR_LAUNCH, "quantize_rows: cannot reserve shared memory");                          \
     row_kernel<BB, CC, EE><<<grid, ROW_THREADS, smem, s>>>(lo, step, w, ldw, d, row_d, nmax, n_rows, k,      \
                                                            params, consts, lo_d, step_d, ldp, codes, sse,    \
@@ -955,7 +959,7 @@ extern "C" int hi2_error_table(const float* w, int64_t ldw, const float* d, cons
     HI2_REQUIRE(block_ok(block_host[c]), "fit_ladder: block must be 16, 32 or 64");
     HI2_REQUIRE(k > 0 && k % block_host[c] == 0, "fit_ladder: k must be a multiple of the block");
     HI2_REQUIRE(nbits_host[c] >= 1 && nbits_host[c] <= 8, "quantize_rows: nbits out of range");
-    HI2_REQUIRE(ROW_WARPS * 2 * (k / block_host[c]) * (int64_t)sizeof(float) <= 200 * 1024,
+    HI2_REQUIRE(ROW_WARPS * 2 * (k / block_host[c]) * (int64_t)sizeof(float) <= ROW_SMEM_MAX,
                 "quantize_rows: k too large for the ladder cache");  // the limit of the one-candidate pass
   }
   if (n_rows == 0) return HI2_OK;
@@ -986,7 +990,7 @@ extern "C" int hi2_error_table(const float* w, int64_t ldw, const float* d, cons
   if (rc != HI2_OK) return rc;
   // the row pass takes as many candidates at a time as their ladders fit in shared memory, six at most
   constexpr int AT_ONCE = 6;
-  constexpr int64_t ROOM = 200 * 1024 / (TABLE_ROW_WARPS * (int64_t)sizeof(TableEntry));
+  constexpr int64_t ROOM = ROW_SMEM_MAX / (TABLE_ROW_WARPS * (int64_t)sizeof(TableEntry));
   for (int first = 0; first < n_cand;) {
     int n = 0;
     int64_t entries = 0;
@@ -998,7 +1002,8 @@ extern "C" int hi2_error_table(const float* w, int64_t ldw, const float* d, cons
     float* en = first == 0 ? energy : nullptr;
 #define HI2_TABLE_ROW(NN)                                                                                          \
   case NN:                                                                                                         \
-    if (cudaFuncSetAttribute(table_row_kernel<NN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) \
+    if (cudaFuncSetAttribute(table_row_kernel<NN>, cudaFuncAttributeMaxDynamicSharedMemorySize, ROW_SMEM_MAX) !=   \
+        cudaSuccess)                                                                                               \
       return fail(HI2_ERR_LAUNCH, "quantize_rows: cannot reserve shared memory");                                  \
     table_row_kernel<NN><<<blocks, TABLE_ROW_WARPS * 32, smem, s>>>(w, ldw, d, row_d, n_rows, k, table, first,     \
                                                                     (int)entries, 1.0f, sse, en);                  \

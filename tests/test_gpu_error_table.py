@@ -54,3 +54,35 @@ def test_table_refuses_what_one_candidate_refuses():
             error_table(w, d, bad, (0.0, 0.1), 1)
     with pytest.raises(RuntimeError):
         error_table(w, d, [], (0.0, 0.1), 1)
+
+
+def test_threads_with_tables_of_different_widths():
+    """Every call needs its own amount of shared memory; what a narrow table in one thread asks for does
+    not take it from a wide one in another.  The entry point is called directly: the fewer of the
+    interpreter's steps lie between two calls, the more often they meet."""
+    import threading
+
+    from hi2_b200 import _lib
+
+    entry, failures = _lib.load().hi2_error_table, []
+    nbits, blocks = _lib.host_i32([nb for nb, _ in SIX]), _lib.host_i32([b for _, b in SIX])
+
+    def work(k):
+        stream = torch.cuda.Stream()
+        with torch.cuda.stream(stream):
+            w, d, ladders, sse = torch.randn(1, k).cuda(), torch.ones(k).cuda(), torch.empty(2, k).cuda(), torch.empty(6).cuda()
+            args = (_lib.ptr(w), k, _lib.ptr(d), None, _lib.host_floats((0.0,)), 1, 0, 6, nbits, blocks, 1, k, _lib.ptr(ladders[0]),
+                    _lib.ptr(ladders[1]), _lib.ptr(sse), None, _lib.stream(w.device))
+            for i in range(20000):
+                if entry(*args):
+                    failures.append((k, i, _lib.last_error()))
+                if i % 64 == 0:
+                    stream.synchronize()
+            stream.synchronize()
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in (11008, 64, 64, 64)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failures, failures[:3]
