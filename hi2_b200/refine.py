@@ -120,16 +120,30 @@ def _decoded(enc):
     return lo.float(), step.float()
 
 
+def _as_encoded(w, enc, block: int) -> bool:
+    """Whether ``enc`` has the types and shapes an encode of this package leaves, which
+    :func:`hi2_b200.refine_kernel.prepare` reads."""
+    n, k = w.shape
+    return (enc.codes.dtype == torch.uint8 and enc.params.dtype == torch.uint8 and enc.consts.dtype == torch.float16
+            and block in (16, 32, 64) and k % block == 0 and tuple(enc.codes.shape) == (n, k)
+            and tuple(enc.params.shape) == (n, k // block, 2) and tuple(enc.consts.shape) == (n, 3))
+
+
+def _on_grid(t: torch.Tensor, grid: int) -> torch.Tensor:
+    """``t`` contiguous at an address that is a multiple of ``grid`` bytes: itself, or a copy."""
+    t = t.contiguous()
+    return t if t.data_ptr() % grid == 0 else t.clone()
+
+
 def refine_groups(groups, hs: torch.Tensor, passes: int, wait: bool = True):
     """One sweep over the rows of every ``(w, enc, nbits, block)`` group (rows of different
     candidates, and of different tensors that read the same input, share the column loop); returns
     the refined codes per group.  ``wait=False`` reads nothing back and returns ``(codes per group,
     status word or None)``: the caller checks the word once it has queued everything."""
     use_tc = max(g[2] for g in groups) <= 4
-    plain = all(enc.codes.dtype == torch.uint8 and enc.params.dtype == torch.uint8 and enc.consts.dtype == torch.float16
-                and block in (16, 32, 64) for _, enc, _, block in groups)
+    plain = all(_as_encoded(w, enc, block) for w, enc, _, block in groups)
     sizes = [w.shape[0] for w, *_ in groups]
-    if plain and groups[0][0].shape[1] % 16 == 0:  # encodes as this package leaves them: one pass over each group's rows
+    if plain:  # one pass over each group's rows
         dev = _lib.need_cuda(*[w for w, *_ in groups], hs)
         n, k = sum(sizes), groups[0][0].shape[1]
         use_tc = _use_tc(use_tc, k)
@@ -140,9 +154,9 @@ def refine_groups(groups, hs: torch.Tensor, passes: int, wait: bool = True):
         for (w, enc, nbits, block), rows in zip(groups, sizes):
             at = slice(r0, r0 + rows)
             wf = w.float()
-            if wf.stride(1) != 1 or wf.stride(0) % 4 or wf.data_ptr() % 16:
-                wf = wf.contiguous().clone()
-            refine_kernel.prepare(wf, enc.codes.contiguous(), enc.params.contiguous(), enc.consts.contiguous(), block, c[at],
+            if wf.stride(1) != 1 or wf.stride(0) < k or wf.stride(0) % 4 or wf.data_ptr() % 16:
+                wf = wf.clone(memory_format=torch.contiguous_format)  # of one row too, whose stride may be anything
+            refine_kernel.prepare(wf, _on_grid(enc.codes, 4), _on_grid(enc.params, 2), enc.consts.contiguous(), block, c[at],
                                   lo_x[at], st_x[at], *((e[0, at], e[1, at]) if use_tc else (e[at],)))
             top[at] = float(2**nbits - 1)
             r0 += rows
