@@ -51,7 +51,7 @@ def _sweeps(w, codes, lo_x, st_x, top, hs, passes: int, use_tc: bool | None, wai
     use_tc = _use_tc(bool((top <= 15).all()) if use_tc is None else use_tc, w.shape[1])
     if use_tc:
         e = refine_kernel.split_tf32(e)
-    return _run(c, lo_x, st_x, top.float().contiguous(), [e], hs.float().contiguous(), passes, use_tc, wait)
+    return _run(c, lo_x, st_x, top.float().reshape(-1).contiguous(), [e], hs.float().contiguous(), passes, use_tc, wait)
 
 
 @torch.no_grad()

@@ -59,3 +59,14 @@ def test_layout_of_the_inputs_does_not_matter(kind, k):
     want = refine_groups([(w, enc, 4, 32)], hs, 2)[0]
     assert int((want != enc.codes).sum()) > 0
     assert torch.equal(refine_groups([(given, got_enc, 4, 32)], hs, 2)[0], want)
+
+
+@pytest.mark.parametrize("k", [192, 640])
+def test_highest_codes_as_a_column(k):
+    from hi2_b200.refine import _decoded, _expand, refine_expanded
+
+    w, enc, hs = encoded(40, k)
+    lo_x, st_x = _expand(*_decoded(enc), 32)
+    top = torch.full((40,), 15.0, device="cuda")
+    want = refine_expanded(w, enc.codes, lo_x, st_x, top, hs, 2)
+    assert torch.equal(refine_expanded(w, enc.codes, lo_x, st_x, top[:, None], hs, 2), want)
