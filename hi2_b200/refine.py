@@ -47,17 +47,18 @@ def _sweeps(w, codes, lo_x, st_x, top, hs, passes: int, use_tc: bool | None, wai
     _lib.need_cuda(w, codes, lo_x, st_x, top, hs)
     c = codes.float().contiguous().clone()
     lo_x, st_x = lo_x.float().contiguous(), st_x.float().contiguous()
-    e = ((lo_x + c * st_x).half().float() - w.float()).contiguous()
+    e = [((lo_x + c * st_x).half().float() - w.float()).contiguous()]
     use_tc = _use_tc(bool((top <= 15).all()) if use_tc is None else use_tc, w.shape[1])
     if use_tc:
-        e = refine_kernel.split_tf32(e)
-    return _run(c, lo_x, st_x, top.float().reshape(-1).contiguous(), [e], hs.float().contiguous(), passes, use_tc, wait)
+        e = [refine_kernel.split_tf32(e.pop())]
+    return _run(c, lo_x, st_x, top.float().reshape(-1).contiguous(), e, hs.float().contiguous(), passes, use_tc, wait)
 
 
 @torch.no_grad()
 def _run(c, lo_x, st_x, top, e: list, hs, passes: int, use_tc: bool, wait: bool):
     """``(refined codes (float), status word or None)`` from fp32 codes ``c [N, K]`` (changed in place) and
-    their errors ``e`` (one entry, taken out of the list: as TF32 parts with ``use_tc``).  With ``wait``
+    their errors ``e`` (as TF32 parts with ``use_tc``; a list of one entry, which the caller holds nowhere else:
+    it is taken out, and its memory is free again behind the first product).  With ``wait``
     the host follows the device: it stops after a sweep that moved no code and raises on a raised
     status word.  Without, nothing is read back: every sweep is queued (one that moves nothing changes
     nothing) and the status word is left to the caller, so several tensors can be refined side by side
@@ -148,7 +149,7 @@ def refine_groups(groups, hs: torch.Tensor, passes: int, wait: bool = True):
         n, k = sum(sizes), groups[0][0].shape[1]
         use_tc = _use_tc(use_tc, k)
         c, lo_x, st_x = (torch.empty(n, k, dtype=torch.float32, device=dev) for _ in range(3))
-        e = torch.empty(*((2,) if use_tc else ()), n, k, dtype=torch.float32, device=dev)
+        e = [torch.empty(*((2,) if use_tc else ()), n, k, dtype=torch.float32, device=dev)]
         top = torch.empty(n, dtype=torch.float32, device=dev)
         r0 = 0
         for (w, enc, nbits, block), rows in zip(groups, sizes):
@@ -157,10 +158,10 @@ def refine_groups(groups, hs: torch.Tensor, passes: int, wait: bool = True):
             if wf.stride(1) != 1 or wf.stride(0) < k or wf.stride(0) % 4 or wf.data_ptr() % 16:
                 wf = wf.clone(memory_format=torch.contiguous_format)  # of one row too, whose stride may be anything
             refine_kernel.prepare(wf, _on_grid(enc.codes, 4), _on_grid(enc.params, 2), enc.consts.contiguous(), block, c[at],
-                                  lo_x[at], st_x[at], *((e[0, at], e[1, at]) if use_tc else (e[at],)))
+                                  lo_x[at], st_x[at], *((e[0][0, at], e[0][1, at]) if use_tc else (e[0][at],)))
             top[at] = float(2**nbits - 1)
             r0 += rows
-        out, status = _run(c, lo_x, st_x, top, [e], hs.float().contiguous(), passes, use_tc, wait)
+        out, status = _run(c, lo_x, st_x, top, e, hs.float().contiguous(), passes, use_tc, wait)
     else:
         parts = []
         for w, enc, nbits, block in groups:

@@ -1,6 +1,8 @@
 """Refinement of encodes and rows whose memory layout differs from what an encode of this package leaves:
 strides, alignment and shapes of the inputs do not change the codes."""
 
+import weakref
+
 import pytest
 import torch
 
@@ -70,3 +72,32 @@ def test_highest_codes_as_a_column(k):
     top = torch.full((40,), 15.0, device="cuda")
     want = refine_expanded(w, enc.codes, lo_x, st_x, top, hs, 2)
     assert torch.equal(refine_expanded(w, enc.codes, lo_x, st_x, top[:, None], hs, 2), want)
+
+
+@pytest.mark.parametrize("k", [192, 640])
+@pytest.mark.parametrize("form", ["groups", "expanded"])
+def test_errors_are_freed_before_the_sweeps(form, k, monkeypatch):
+    """The rows' errors (8 bytes a weight as TF32 parts) are read once, by the first product."""
+    from hi2_b200 import refine, refine_kernel
+
+    w, enc, hs = encoded(40, k)
+    seen, sweeps = [], []
+    name = "gemm_tc" if k >= refine.TC_MIN_K else "gemm"
+    product, sweep = getattr(refine_kernel, name), refine_kernel.sweep
+
+    def watch(a, *args, **kw):
+        seen.append(weakref.ref(a))
+        return product(a, *args, **kw)
+
+    def check(*args):
+        sweeps.append(seen[0]() is None)
+        return sweep(*args)
+
+    monkeypatch.setattr(refine_kernel, name, watch)
+    monkeypatch.setattr(refine_kernel, "sweep", check)
+    if form == "groups":
+        refine.refine_groups([(w, enc, 4, 32)], hs, 2)
+    else:
+        lo_x, st_x = refine._expand(*refine._decoded(enc), 32)
+        refine.refine_expanded(w, enc.codes, lo_x, st_x, torch.full((40,), 15.0, device="cuda"), hs, 2)
+    assert sweeps and all(sweeps)
