@@ -412,7 +412,8 @@ fit_kernel(const float* __restrict__ w, int64_t ldw, const float* __restrict__ d
            const int32_t* __restrict__ row_d, int64_t n_rows, int64_t nb, GridSpec grid, int refits, float nmax, float* __restrict__ lo_out,
            float* __restrict__ st_out, float* __restrict__ err_out) {
   __shared__ FitShared shared;
-  fit_tile<B, GROUPED, BOUND>(shared, blockIdx.x, blockIdx.y, w, ldw, d_all, row_d, n_rows, nb, grid, refits, nmax, lo_out,
+  const int64_t blk_tile = (int64_t)blockIdx.z * gridDim.y + blockIdx.y;  // one dimension ends at 65535
+  fit_tile<B, GROUPED, BOUND>(shared, blockIdx.x, blk_tile, w, ldw, d_all, row_d, n_rows, nb, grid, refits, nmax, lo_out,
                               st_out, err_out);
 }
 
@@ -475,7 +476,8 @@ int launch_fit(const float* w, int64_t ldw, const float* d, const int32_t* row_d
                float* err, cudaStream_t stream) {
   bool clips;
   const GridSpec spec = make_grid(grid_host, g, &clips);
-  dim3 grid((unsigned)ceil_div(n_rows, block == 64 ? 16 : 32), (unsigned)ceil_div(nb, FIT_WARPS));
+  const int64_t blk_tiles = ceil_div(nb, (int64_t)FIT_WARPS), layers = ceil_div(blk_tiles, (int64_t)65535);
+  dim3 grid((unsigned)ceil_div(n_rows, block == 64 ? 16 : 32), (unsigned)ceil_div(blk_tiles, layers), (unsigned)layers);
   const float nmax = (float)(n - 1);
   // Passing over grid points that their clipped columns rule out: 11008 x 4096, normal effort, blocks of 16 /
   // 32 / 64, us: 16 levels 682 / 645 / 682 -> 483 / 502 / 590, 256 levels 770 / 739 / 780 -> 360 / 295 / 301;

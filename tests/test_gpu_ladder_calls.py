@@ -26,3 +26,15 @@ def test_weights_may_start_at_any_float(block, n, offset):
     for a, b, want in zip(got, ladder_kernel.ladder_grid(wb.cuda(), db.clone(), grid, n),
                           po.grid_search(wb, db.cpu().reshape(1, nb, block), n, grid)):
         assert torch.equal(a, b) and torch.equal(a.cpu(), want)
+
+
+@pytest.mark.parametrize("block,nb", [(16, 262145), (16, 400001), (32, 262145), (64, 262141)])
+def test_more_blocks_in_a_row_than_one_grid_dimension_holds(block, nb):
+    """Four blocks of a row go to a thread block, and a grid dimension ends at 65535."""
+    from hi2_b200.encode import fit_ladder
+
+    wb = torch.randn(1, nb, block, generator=gen(nb))
+    db = torch.rand(1, nb, block, generator=gen(block)) + 0.1
+    lo, st = fit_ladder(wb.cuda(), db.cuda(), 4, "fast")
+    want = po.search_ladder(wb, db, 4, "fast")
+    assert torch.equal(lo.cpu(), want[0]) and torch.equal(st.cpu(), want[1])
