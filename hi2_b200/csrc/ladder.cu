@@ -17,6 +17,7 @@ struct GridSpec {
   float v[8];
   int g;
   float one;  // 1.0, as a kernel argument
+  float packed_from;  // steps above it take the packed arithmetic: 0, or infinity for more levels than it holds
 };
 
 // Block sums are formed in the order of torch's CPU reduction over a contiguous inner dimension
@@ -40,7 +41,7 @@ __device__ __forceinline__ float fold_lane(const float (&v)[B / 8]) {
 // rounded reciprocal of `safe` serves the block and every quotient is finished with Markstein's
 // fused correction, which yields the correctly rounded quotient itself, so rint sees the very number
 // the division would give.  Steps outside the range the correction covers (rc.fast false: tiny, huge,
-// or a significand of all ones) and negative ones take true divisions.
+// or a significand of all ones), negative ones and ladders of more than 2^23 steps take true divisions.
 //
 // Everything else is done for two neighbouring columns per instruction (packed fp32 multiplies and
 // fused multiply-adds), since the search is bound by instruction issue: 12 instructions a pair where
@@ -81,11 +82,11 @@ struct Step {
   float2 neg_r, safe, step, off;  // -1 / step, step, step, -2^23 step
   bool fast;
 };
-__device__ __forceinline__ Step make_step(float step) {
+__device__ __forceinline__ Step make_step(float step, float packed_from) {
   Step s;
   const float safe = (step == 0.0f) ? 1.0f : step;
   const Recip rc = make_recip(safe);
-  s.fast = rc.fast && safe > 0.0f;
+  s.fast = rc.fast && safe > packed_from;
   s.neg_r = both(-rc.r), s.safe = both(safe), s.step = both(step), s.off = both(-SHIFT * step);
   return s;
 }
@@ -189,8 +190,9 @@ __device__ __forceinline__ float2 below(float2 nx, float2 lo, float2 one) { retu
 // memory.
 template <int B, bool GROUPED, bool HAVE_AN>
 __device__ __forceinline__ float block_error_exact(const Block<B>& blk, const float2* an, const float* __restrict__ x,
-                                                   const float* d, int half, float lo, float step, float nmax, float2 one) {
-  const Step s = make_step(step);
+                                                   const float* d, int half, float lo, float step, float nmax, float2 one,
+                                                   float packed_from) {
+  const Step s = make_step(step, packed_from);
   const float2 lo2 = both(lo);
   const float top = SHIFT + nmax;
   float err[1];
@@ -218,7 +220,7 @@ __device__ __forceinline__ float block_error_exact(const Block<B>& blk, const fl
 template <int B, bool GROUPED>
 __device__ __forceinline__ float block_error(const Block<B>& blk, const float2 (&an)[Block<B>::PAIRS],
                                              const float* __restrict__ x, const float* d, int half, float lo, float step,
-                                             float nmax, float2 one) {
+                                             float nmax, float2 one, float packed_from) {
   bool sure = nmax <= 15.0f && step > 1e-15f && step < 1e15f;
   if (Block<B>::SHARED) sure = __all_sync(0xffffffffu, sure);
   if (sure) {
@@ -243,7 +245,7 @@ __device__ __forceinline__ float block_error(const Block<B>& blk, const float2 (
     if (Block<B>::SHARED) sure = __all_sync(0xffffffffu, sure);
     if (sure) return err[0];
   }
-  return block_error_exact<B, GROUPED, true>(blk, an, x, d, half, lo, step, nmax, one);
+  return block_error_exact<B, GROUPED, true>(blk, an, x, d, half, lo, step, nmax, one, packed_from);
 }
 
 // Sum over the block of d * (distance beyond `edge`)^2, on the side where lo - x > 0 (LOW) or < 0: what the
@@ -360,7 +362,7 @@ __device__ __forceinline__ void fit_tile(FitShared& shared, int64_t row_tile, in
         if (SHARED) beaten = __all_sync(0xffffffffu, beaten);
         if (beaten) continue;
       }
-      const float err = block_error<B, GROUPED>(r, an, src, d, half, lo, step, nmax, one);
+      const float err = block_error<B, GROUPED>(r, an, src, d, half, lo, step, nmax, one, grid.packed_from);
       if ((gi | gj) == 0 || err < best_err) best_lo = lo, best_st = step, best_err = err;
     }
   }
@@ -369,7 +371,7 @@ __device__ __forceinline__ void fit_tile(FitShared& shared, int64_t row_tile, in
   for (int it = 0; it < refits; ++it) {
     // sums over the block of d, d c, d c^2, -d x, -d c x and -x, c the code
     float sums[6];
-    const Step s = make_step(best_st);
+    const Step s = make_step(best_st, grid.packed_from);
     const float2 lo2 = both(best_lo);
     const float top = SHIFT + nmax, safe = s.safe.x;
     block_sums<B, 6>(sums, half, one, [&](int j, int h, int p, float2 (&t)[2][6]) {
@@ -394,7 +396,7 @@ __device__ __forceinline__ void fit_tile(FitShared& shared, int64_t row_tile, in
     const bool ok = fabsf(det) > 1e-20f;
     const float step = ok ? __fdiv_rn(sd * scw - sc * sw, det) : 0.0f;
     const float lo = ok ? __fdiv_rn(sw - step * sc, fmaxf(sd, 1e-20f)) : __fdiv_rn(sum, (float)B);
-    const float err = block_error_exact<B, GROUPED, false>(r, nullptr, src, d, half, lo, step, nmax, one);
+    const float err = block_error_exact<B, GROUPED, false>(r, nullptr, src, d, half, lo, step, nmax, one, grid.packed_from);
     if (err < best_err && step > 0.0f) best_lo = lo, best_st = step, best_err = err;
   }
 
@@ -460,9 +462,10 @@ table_fit_kernel(const float* __restrict__ w, int64_t ldw, const float* __restri
 
 // The grid as the kernels take it; *clips: every point moves an end of the ladder inwards, by half the
 // range at most.
-GridSpec make_grid(const float* grid_host, int g, bool* clips) {
+GridSpec make_grid(const float* grid_host, int g, float nmax, bool* clips) {
   GridSpec spec;
   spec.g = g, spec.one = 1.0f;
+  spec.packed_from = nmax <= SHIFT ? 0.0f : INFINITY;  // 2^23 + a larger code is not a whole number
   *clips = true;
   for (int i = 0; i < 8; ++i) {
     spec.v[i] = i < g ? grid_host[i] : 0.0f;
@@ -475,10 +478,10 @@ int launch_fit(const float* w, int64_t ldw, const float* d, const int32_t* row_d
                int refits, int n, int64_t n_rows, int64_t nb, int block, float* lo, float* st,
                float* err, cudaStream_t stream) {
   bool clips;
-  const GridSpec spec = make_grid(grid_host, g, &clips);
+  const float nmax = (float)(n - 1);
+  const GridSpec spec = make_grid(grid_host, g, nmax, &clips);
   const int64_t blk_tiles = ceil_div(nb, (int64_t)FIT_WARPS), layers = ceil_div(blk_tiles, (int64_t)65535);
   dim3 grid((unsigned)ceil_div(n_rows, block == 64 ? 16 : 32), (unsigned)ceil_div(blk_tiles, layers), (unsigned)layers);
-  const float nmax = (float)(n - 1);
   // Passing over grid points that their clipped columns rule out: 11008 x 4096, normal effort, blocks of 16 /
   // 32 / 64, us: 16 levels 682 / 645 / 682 -> 483 / 502 / 590, 256 levels 770 / 739 / 780 -> 360 / 295 / 301;
   // at 4 levels next to nothing is ruled out and the bounds cost 6 %.
@@ -969,7 +972,7 @@ extern "C" int hi2_error_table(const float* w, int64_t ldw, const float* d, cons
   HI2_REQUIRE(aligned16(w) && aligned16(d) && ldw % 4 == 0 && ldw >= k, "fit_ladder: w, d alignment or ldw");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   bool clips;
-  const GridSpec spec = make_grid(grid_host, g, &clips);
+  const GridSpec spec = make_grid(grid_host, g, 255.0f, &clips);  // 8 bits at most
   TableSpec table;
   table.n = n_cand;
   int64_t tiles = 0, offset = 0;

@@ -38,3 +38,16 @@ def test_more_blocks_in_a_row_than_one_grid_dimension_holds(block, nb):
     lo, st = fit_ladder(wb.cuda(), db.cuda(), 4, "fast")
     want = po.search_ladder(wb, db, 4, "fast")
     assert torch.equal(lo.cpu(), want[0]) and torch.equal(st.cpu(), want[1])
+
+
+@pytest.mark.parametrize("block", [16, 32, 64])
+@pytest.mark.parametrize("n", [2**22, 2**23, 2**23 + 1, 2**23 + 2, 2**24])
+def test_more_levels_than_the_shifted_rounding_covers(block, n):
+    """Codes up to 2^23 stay whole numbers after 2^23 is added to them, larger ones do not."""
+    from hi2_b200.encode import fit_ladder
+
+    wb = torch.randn(33, 12, block, generator=gen(block))
+    db = torch.rand(1, 12, block, generator=gen(n % 1000)) + 0.1
+    lo, st = fit_ladder(wb.cuda(), db.cuda(), n, "normal")
+    want = po.search_ladder(wb, db, n, "normal")
+    assert torch.equal(lo.cpu(), want[0]) and torch.equal(st.cpu(), want[1])
