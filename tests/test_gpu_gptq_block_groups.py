@@ -132,6 +132,43 @@ def test_updates_taken_together_are_the_updates_one_by_one(rows, k):
             assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize("rows", [18945, 19007])
+@pytest.mark.parametrize("columns", [128, 512])
+@pytest.mark.parametrize("with_comp", [False, True])
+def test_loop_of_many_rows_is_the_loop_of_a_few(rows, columns, with_comp):
+    """Two rows per lane with the errors left as TF32 parts, in a buffer of one block's width and of a
+    group's: every row as in a launch of a few hundred rows, one per lane."""
+    from hi2_b200 import _lib
+    from hi2_b200.gptq_kernel import split_factor
+
+    k, cut = 656, 7001
+    wc, us, lo, st, _, _, _ = case(rows, k, 2, rows, (2, 4))
+    blk = (torch.arange(k) // 32).to(torch.int32).expand(2, k).contiguous().cuda()
+    grp = (torch.arange(rows) >= cut).to(torch.int32).cuda()
+    w, lo, st, nmax = wc.cuda(), lo.cuda(), st.cuda(), torch.tensor([3.0, 15.0]).cuda()
+    u = [x.cuda() * 0.5 for x in us]
+    split, ptrs = [split_factor(x) for x in u], torch.tensor([x.data_ptr() for x in u]).cuda()
+
+    def run(r0, r1):
+        n, at = r1 - r0, slice(r0, r1)
+        work, codes = w[at].clone(), torch.zeros(n, k, dtype=torch.uint8, device="cuda")
+        seen = torch.zeros(n, k, device="cuda") if with_comp else None
+        scratch, status = torch.empty(2, n, columns, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+        inner = min(max(cut - r0, 0), n)
+        lo_r, st_r, grp_r = lo[at].contiguous(), st[at].contiguous(), grp[at].contiguous()
+        _lib.call("hi2_gptq_round_tc_grouped", _lib.ptr(work), n, k, _lib.ptr(scratch), columns, _lib.ptr(codes), _lib.ptr(lo_r),
+                  _lib.ptr(st_r), k // 16, _lib.ptr(grp_r), _lib.ptr(ptrs), _lib.ptr(blk), _lib.ptr(nmax), _lib.ptr(seen), 2,
+                  _lib.host_i64([0, inner, n]), _lib.host_i64([x.data_ptr() for x in split]), _lib.ptr(status),
+                  _lib.stream(w.device))
+        assert int(status.item()) == 0
+        return [codes, work] + ([seen] if with_comp else [])
+
+    whole = run(0, rows)
+    for r0, r1 in ((0, 300), (cut - 100, cut + 150), (rows - 333, rows)):
+        for a, b in zip(whole, run(r0, r1)):
+            assert torch.equal(a[r0:r1], b)
+
+
 @pytest.mark.parametrize("k", [4, 64, 68, 128, 1040])
 def test_split_of_the_factor_where_the_updates_read_it(k):
     from hi2_b200.gptq_kernel import split_factor, split_tf32_transposed

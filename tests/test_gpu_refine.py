@@ -152,12 +152,12 @@ def test_refine_with_tensor_core_products():
 
 
 def test_block_kernel_mappings_agree():
-    """The block entry point maps a lane to a row when the rows fill the SMs (>= 148 x 64) and a warp
-    to a row below that: both must give the same codes and the same dw, bit for bit."""
+    """A lane of the block kernel serves two rows from 148 x 128 rows on and one below: both must give
+    the same codes and the same dw, bit for bit."""
     from hi2_b200 import refine_kernel
 
     g_ = torch.Generator().manual_seed(9)
-    n, k, b0, length = 148 * 64 + 37, 256, 128, 128
+    n, k, b0, length = 148 * 128 + 37, 256, 128, 128
     x = torch.randn(1024, k, generator=g_)
     hs = (x.T @ x / 1024).to(DEV).contiguous()
     c = torch.randint(0, 4, (n, k), generator=g_).float().to(DEV)
@@ -167,7 +167,7 @@ def test_block_kernel_mappings_agree():
     top = torch.full((n,), 3.0, device=DEV)
     gb = torch.randn(n, length, generator=g_).to(DEV) * 0.02
     outs = []
-    for parts in ([slice(0, n)], [slice(0, 5000), slice(5000, n)]):  # one launch with a lane per row; two with a warp per row
+    for parts in ([slice(0, n)], [slice(0, 5000), slice(5000, n)]):  # one launch with two rows per lane; two with one
         cc, dw = c.clone(), torch.zeros(n, length, device=DEV)
         for s in parts:
             cs, ds = cc[s].contiguous(), torch.empty(s.stop - s.start, length, device=DEV)
@@ -215,10 +215,13 @@ def test_refinement_of_tensors_side_by_side_equals_one_by_one():
     assert any(not torch.equal(t.codes, p.codes) for t, p in zip(together, plain))  # the sweeps did move codes
 
 
-@pytest.mark.parametrize("n", [37, 148 * 64 + 5])
-def test_block_in_place_equals_block_then_split(n):
-    """The folded entry point (slice of g read where it lies, changes written as TF32 parts) against
-    the plain one followed by the split, for both row mappings: same codes, same parts."""
+@pytest.mark.parametrize("n", [37, 148 * 64 + 5, 148 * 128 + 1, 148 * 128 + 67])
+@pytest.mark.parametrize("width", [128, 512])
+def test_block_in_place_equals_block_then_split(n, width):
+    """The folded entry point (slice of g read where it lies, changes written as TF32 parts, into a
+    buffer of their own or a column slice of a wider one) against the plain one followed by the split,
+    with one and with two rows per lane (from 148 x 128 rows on): same codes, same parts, and nothing
+    written beside them."""
     from hi2_b200 import refine_kernel
 
     g = torch.Generator().manual_seed(n)
@@ -234,9 +237,11 @@ def test_block_in_place_equals_block_then_split(n):
     dwb = torch.empty(n, length, device=DEV)
     refine_kernel.refine_block(gfull[:, b0 : b0 + length].contiguous(), c1, lo, st, top, hs, b0, length, dwb)
     want = refine_kernel.split_tf32(dwb)
-    parts = torch.full((2, n, length), 7.0, device=DEV)
+    wide = torch.full((2, n, width), 7.0, device=DEV)
+    at = width - length
+    parts = wide[:, :, at:]
     refine_kernel.refine_block_in_place(gfull, c2, lo, st, top, hs, b0, length, parts)
-    assert torch.equal(c1, c2) and torch.equal(parts, want)
+    assert torch.equal(c1, c2) and torch.equal(parts, want) and bool((wide[:, :, :at] == 7.0).all())
     assert bool((dwb != 0).any())
 
 

@@ -89,9 +89,69 @@ def test_prepare_is_the_elementwise_form(rows, k, nbits, block):
     assert torch.equal(torch.stack([got, low]), refine_kernel.split_tf32(e.contiguous()))
 
 
+@pytest.mark.parametrize("k", [192, 640, 1152])
+@pytest.mark.parametrize("width", [128, 512])
+@pytest.mark.parametrize("split", [False, True])  # FMA and tensor-core products
+def test_last_sweep_leaves_out_only_what_nobody_reads(k, width, split):
+    """A sweep that is not followed by another does not bring the columns it has passed up to date: same
+    codes, bit for bit, as a sweep that does, and the same word for whether a code moved."""
+    from hi2_b200 import refine_kernel
+
+    rows = 90
+    g_all, c, lo, st, top, hs = [t.cuda() for t in case(rows, k, k + width)]
+    parts = refine_kernel.split_tf32(hs) if split else None
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    out = []
+    for last in (False, True):
+        g, codes = g_all.clone(), c.clone()
+        moves = torch.empty(*((2, rows, min(width, k)) if split else (rows, 128)), device="cuda")
+        moved = torch.zeros(1, dtype=torch.int32, device="cuda")
+        refine_kernel.sweep(g, codes, lo, st, top, hs, parts, moves, width, False, moved, status)
+        first = codes.clone()
+        assert int(moved.item()) == 1 and bool((first != c).any())
+        moved.zero_()
+        refine_kernel.sweep(g, codes, lo, st, top, hs, parts, moves, width, last, moved, status)
+        assert int(moved.item()) == int(bool((codes != first).any())) == 1
+        out.append(codes)
+    assert torch.equal(*out) and int(status.item()) == 0
+
+
 @pytest.mark.parametrize("k", [192, 640])  # FMA and tensor-core products
-def test_sweeps_one_by_one_are_the_sweeps_together(k):
-    """The last sweep updates only what it still reads: the codes of two sweeps are those of one and one."""
+@pytest.mark.parametrize("group", [False, True])
+def test_two_sweeps_are_one_and_one(k, group, monkeypatch):
+    """Two sweeps in one call give the codes of two sweeps queued one by one from the same start."""
+    from hi2_b200 import refine, refine_kernel
+    from hi2_b200.encode import encode_rows
+    from hi2_b200.refine import refine_groups
+
+    if group:
+        monkeypatch.setattr(refine, "GROUP_MIN_ELEMS", 0)
+    rows, split = 90, k >= refine.TC_MIN_K
+    x = torch.randn(2 * k, k, generator=gen(k))
+    hs = (x.T @ x / x.shape[0]).cuda()
+    w = torch.randn(rows, k, generator=gen(k + 1)).cuda()
+    enc = encode_rows(w, hs.diagonal().contiguous(), 4, 32, "fast")
+    c, lo, st, g = (torch.empty(rows, k, device="cuda") for _ in range(4))
+    e = torch.empty(2, rows, k, device="cuda") if split else torch.empty(rows, k, device="cuda")
+    refine_kernel.prepare(w, enc.codes, enc.params, enc.consts, 32, c, lo, st, *(e if split else (e,)))
+    parts, status = refine_kernel.split_tf32(hs) if split else None, torch.zeros(1, dtype=torch.int32, device="cuda")
+    if split:
+        refine_kernel.gemm_tc(e, parts, g, status)
+    else:
+        refine_kernel.gemm(e, hs, g)
+    width = 512 if group else 128
+    moves = torch.empty(*((2, rows, min(width, k)) if split else (rows, 128)), device="cuda")
+    top = torch.full((rows,), 15.0, device="cuda")
+    for _ in range(2):
+        refine_kernel.sweep(g, c, lo, st, top, hs, parts, moves, width, False, None, status)
+    assert bool((c != enc.codes).any()) and int(status.item()) == 0
+    assert torch.equal(refine_groups([(w, enc, 4, 32)], hs, 2)[0].float(), c)
+    codes, word = refine_groups([(w, enc, 4, 32)], hs, 2, False)
+    assert torch.equal(codes[0].float(), c) and (word is None or int(word.item()) == 0)
+
+
+@pytest.mark.parametrize("k", [192, 640])
+def test_sweeps_settle(k):
     from hi2_b200.encode import Encoded, encode_rows
     from hi2_b200.refine import refine_groups
 
@@ -100,10 +160,7 @@ def test_sweeps_one_by_one_are_the_sweeps_together(k):
     w = torch.randn(90, k, generator=gen(k + 1)).cuda()
     enc = encode_rows(w, hs.diagonal().contiguous(), 4, 32, "fast")
     for wait in (True, False):
-        two = refine_groups([(w, enc, 4, 32)], hs, 2, wait)
         many = refine_groups([(w, enc, 4, 32)], hs, 40, wait)
-        two, many = (two[0], many[0]) if wait else (two[0][0], many[0][0])
-        assert int((two != enc.codes).sum()) > 0
-        done = Encoded(many, enc.params, enc.consts, enc.sse)
-        again = refine_groups([(w, done, 4, 32)], hs, 1)[0]  # after many sweeps nothing moves any more
-        assert (again != many).float().mean() < 1e-3
+        many = many[0] if wait else many[0][0]
+        again = refine_groups([(w, Encoded(many, enc.params, enc.consts, enc.sse), 4, 32)], hs, 1)[0]
+        assert (again != many).float().mean() < 1e-3  # after many sweeps nothing moves any more
