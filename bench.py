@@ -999,12 +999,9 @@ def run_reference(args, cfg):
     emit(line)
 
 
-# ncu capture of the second-moment kernel at 32768 tokens x 4096 columns
-# (profiles/hessian_tc_kernel_k4096_32k_tokens.md): DRAM reads were 2.08 x the bytes of X (L2 absorbs
-# the rest of the tile re-reads), DRAM writes the per-item output tiles.  Reads grow in proportion
-# to the tokens, the tiles do not, so a full-size launch is scaled from those two figures.
-# DRAM reads of the second-moment kernel as a multiple of the bytes of X, from ncu captures at
-# 32768 tokens: 1.05 at K = 4096 (pair kernel, X of a wave fits in L2), 6.2 at K = 11008 (one-block
+# DRAM reads of the second-moment kernel as a multiple of the bytes of X, from ncu captures at 32768 tokens
+# (profiles/hessian_pair_kernel_32k_tokens.md).  Reads grow in proportion to the tokens, the item tiles
+# that are written do not, so a full-size launch is scaled from those two: 1.05 at K = 4096 (pair kernel, X of a wave fits in L2), 6.2 at K = 11008 (one-block
 # kernel, banded tile schedule, ~13 waves of which the L2 absorbs half)
 HESSIAN_READ_FACTOR = {4096: 1.05, 11008: 6.2}
 
@@ -1384,7 +1381,7 @@ def run_kernels(args, cfg):
         hs = transform_sigma(sig, None, had)
         ms = timed(lambda: inverse_factor(hs, 0.01), reps=3, warm=1, cold=False, tag="factor")
         add(f"inverse_factor K={kk}", "fp32-grade flops", (2.0 / 3.0) * kk**3 / 1e12, "TFLOP/s", ms, fp32_peak,
-            "(2/3) K^3 against the cuBLAS fp32 peak; a chain of K/64 dependent leaves")
+            "(2/3) K^3 against the cuBLAS fp32 peak; a chain of K/128 dependent blocks")
         if kk == k:
             u_small = inverse_factor(hs, 0.01)
         del sig, hs
@@ -1407,8 +1404,8 @@ def run_kernels(args, cfg):
     add(f"row_kernel<32> INT2 {r_wide}x{k}", "hbm", (w.numel() * 5.0 + lo.numel() * 10.0) / 1e9, "GB/s", ms, pk["hbm"],
         "reads fp32 rows, writes codes, parameter bytes and sse")
     ms = timed(lambda: ladder_kernel.quantize_rows(lo, st, 2, 32, k, w, d, want_codes=False, want_sse=True), tag="row")
-    add(f"row_kernel<32> INT2 {r_wide}x{k}, table pass (no codes)", "hbm", (w.numel() * 4.0 + lo.numel() * 10.0) / 1e9,
-        "GB/s", ms, pk["hbm"], "what a table entry costs: reads fp32 rows, writes parameter bytes and sse")
+    add(f"row_kernel<32> INT2 {r_wide}x{k}, no codes", "hbm", (w.numel() * 4.0 + lo.numel() * 10.0) / 1e9,
+        "GB/s", ms, pk["hbm"], "the row pass of one candidate: reads fp32 rows, writes parameter bytes and sse")
     q = ladder_kernel.quantize_rows(lo, st, 2, 32, k, w, d, want_codes=True, want_decoded=True, ldp=k // 16)
     words = torch.empty(r_wide, k // 16, dtype=torch.int32, device=dev)
     bad = torch.zeros(1, dtype=torch.int32, device=dev)
@@ -1430,7 +1427,7 @@ def run_kernels(args, cfg):
                    cold=False, tag="gptq")
     add(f"gptq_block N={n} (128 columns)", "dependent chain", n * 128 * 140.0 / 1e12, "Tops/s", ms_blk, lane_peak,
         "140 reference operations per row and column")
-    parts = gptq_kernel.split_tf32_transposed(u_small)
+    parts = gptq_kernel.split_factor(u_small)
     ms_round = timed(lambda: gptq_kernel.gptq_round_tc(wc, err1, codes, q["lo_d"], q["step_d"], rg, up, blk, nm, None,
                                                         [0, n], [parts]), reps=3, warm=1, cold=False, tag="gptq")
     lazy_flops = float(n) * k * k * (1 - 128.0 / k)

@@ -6,7 +6,8 @@ Differences from the reference's orchestration, none of which changes a result:
 * one process drives one GPU, so there is no row sharding over an executor: the ``ex`` argument
   is accepted and ignored (matrices, not rows, are what ``hi2_b200.dist`` spreads over GPUs);
 * weights are cast, scaled and rotated in one kernel pass, straight from bf16 / fp16;
-* a table costs two launches per candidate and returns ``sse`` on the device;
+* a table costs one launch for the searches at all candidates and one pass over the rows per six of
+  them, and returns ``sse`` on the device;
 * the Hessian of a shared input is transformed and factorised once per ``sigma_id``.
 """
 
@@ -226,8 +227,8 @@ def build_tables_grouped(items: list, cfg: Config) -> list:
     """:func:`build_table` for several tensors of ONE shape that read different inputs (the experts of
     a layer): ``items`` holds ``(name, w [R, K], stats, (smoothing vector, flags), n_tokens)`` per
     tensor.  The stored rows of all of them lie one after the other in one buffer, their column
-    weights form a ``[G, K]`` matrix, and every candidate costs two launches for the whole group
-    instead of two per tensor; per row the arithmetic is that of :func:`build_table`.  Tables come
+    weights form a ``[G, K]`` matrix, and the whole group costs the launches of one table instead of
+    one table each; per row the arithmetic is that of :func:`build_table`.  Tables come
     back in the order of ``items`` (their ``sse`` are views of the group's table)."""
     if cfg.smooth_search or len(items) < 2 or any(it[3] is None for it in items):
         return [build_table(name, w, st, cfg, transform=tr, n_tokens=n) for name, w, st, tr, n in items]

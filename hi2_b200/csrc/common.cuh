@@ -41,10 +41,16 @@ inline int check_launch(const char* what) {
 // other streams meanwhile - the chains of four inputs then run one after the other instead of
 // side by side; as a graph the chain costs the host one launch and its kernels start back to back.
 // A stream that is already being captured by the caller is left alone (the launches then join the
-// caller's graph).  So is a chain of at most CHAIN_PLAIN launches: it fits the queue, and the GPU starts
-// on it while a graph would still be captured and instantiated (column loop of 4096 x 4096, 63 launches,
-// with its ladders 2.7 -> 2.4 ms; from 171 launches on the graph's shorter gaps win, 7.9 -> 7.5 ms).  Finished graphs are destroyed on later calls, once their completion event has
-// passed.
+// caller's graph), and the legacy default stream, which cannot be captured, takes every chain plain.  So
+// does any stream a chain of at most CHAIN_PLAIN launches: it fits the queue, and the GPU starts on it
+// while a graph would still be captured and instantiated.  Measured on a stream of its own, graph / plain,
+// ms: inverse factor K = 1024 (29 launches) 0.83 / 0.57, 3072 (103) 2.18 / 1.74, 4096 (155) 3.00 / 2.51;
+// column loop 1024 x 6144 (95) 1.97 / 1.76, 1024 x 8192 (127) 2.66 / 2.42, 1024 x 11008 (171) 3.66 / 3.39.
+// So a chain alone is quicker plain at every length, and the line is not where the two cross: it is a
+// tenth of the queue, which is what several streams share.  A decoder layer with its chains side by side:
+// all as graphs 54.0 ms, by the line 54.1, all plain 52.9; a layer of five experts 24.7, 21.5, 21.2 (runs
+// of one kind differ by 2 to 4 %).  Finished graphs are destroyed on later calls, once their completion
+// event has passed.
 class ChainGraph {
  public:
   static constexpr int64_t CHAIN_PLAIN = 96;

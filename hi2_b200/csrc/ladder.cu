@@ -5,9 +5,10 @@
 //              in shared memory) and the block's weights stay in registers for the whole grid search
 //              and the least-squares refits.  The work is about 350 instructions per weight (effort
 //              "normal") against 4 bytes read: bound by the fp32 pipe (70 % busy at blocks of 32).
-// row kernel   one thread block per row: row-wide extrema of (lo, step), the three fp16 row
-//              constants, the parameter bytes, the decoded fp16 ladders, and optionally the
-//              nearest codes and the weighted error of the row.  One pass over the row: HBM-bound.
+// row kernel   one warp per row: row-wide extrema of (lo, step), the three fp16 row constants, the
+//              parameter bytes, the decoded fp16 ladders, and optionally the nearest codes and the
+//              weighted error of the row, in one pass over the row.  table_row_kernel does this for all
+//              candidates of an error table at once, without codes.  Both are bound by instruction issue.
 #include "common.cuh"
 
 namespace hi2 {
@@ -556,9 +557,9 @@ constexpr int ROW_SMEM_MAX = 200 * 1024;
 // One WARP per row: the row-wide extrema, the constants and the parameter bytes need only warp
 // shuffles, so no thread block barrier sits between the phases of a row and 64 rows are in flight
 // per SM.  Dynamic shared memory: per warp the decoded lo[nb], step[nb] of its row.
-// CODES / ENERGY: whether code bytes are written and the row energy is summed.  The tables ask for
-// neither on five of their six passes, and the pass is bound by instruction issue (73 % of the
-// issue slots at a third of the copy bandwidth), so the instructions of unused outputs are compiled out.
+// CODES / ENERGY: whether code bytes are written and the row energy is summed.  The ladders of the column
+// loop ask for neither, and a pass over the weights is bound by instruction issue (73 % of the issue slots
+// at a third of the copy bandwidth), so the instructions of unused outputs are compiled out.
 template <int B, bool CODES, bool ENERGY>
 __global__ void __launch_bounds__(ROW_THREADS, 4)
 row_kernel(const float* __restrict__ lo_in, const float* __restrict__ st_in,

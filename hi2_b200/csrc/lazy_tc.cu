@@ -266,8 +266,8 @@ lazy_tc_kernel(const __grid_constant__ CUtensorMap map_ahi, const __grid_constan
 //     C[m, n] (+)= (+-) A[m, kk] . Bt[n, kk]^T
 //
 // A and Bt are given as their TF32 parts (K-major, leading dimension ldk), C is fp32 with its own
-// leading dimension.  Triangular operands are expressed as reduction ranges per tile (the same
-// flags as gemm.cuh): the skipped range holds exact zeros, so taking whole 32-wide stages of it
+// leading dimension.  Triangular operands are expressed as reduction ranges per tile (flags
+// GT_*): the skipped range holds exact zeros, so taking whole 32-wide stages of it
 // changes nothing.  The reduction of a tile is cut into windows of G_WINDOW stages (64 values of
 // k): each window is accumulated in its own TMEM buffer and added, round-to-nearest, into fp32
 // registers of the eight epilogue warps while the next window accumulates in the other buffer;
@@ -467,7 +467,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_ahi, const __grid_constan
 //     wc[:, i2:] = ((wc[:, i2:] - err_0 U_0) - err_1 U_1) - ...
 //
 // One update per block reads and writes all of wc behind the block: at 32768 x 4096 that is 1.07 GB for
-// 200 GFLOP, and memory was the bound (267 us, 375 TFLOP/s of TF32 products).  Here a tile of wc comes
+// 100 GFLOP, and memory was the bound (267 us, 375 TFLOP/s of TF32 products).  Here a tile of wc comes
 // into the registers of the eight epilogue warps once, every block's product (its own TMEM buffer, the
 // very operations of lazy_tc_kernel) is added to it round-to-nearest in the order of the blocks, and
 // the tile goes back once: the sums are the bits that one update after the other gives.  The columns

@@ -147,8 +147,9 @@ refine_block_kernel(const float* __restrict__ gb, int64_t ldg, int len, float* _
 
 // What the sweeps start from, for one group of rows in one pass: codes as fp32, the ladder of every column
 // (decoded as hi2/format.py:45-60: lo = fp16(fma(byte, lo_scale, lo_min)), step = fp16(byte * step_scale)),
-// and the error e = fp16(lo + c step) - w, as it is or as its TF32 parts.  Bound by memory: 25 bytes
-// written and 5 read per weight; a dozen elementwise passes before, 650 -> 67 us for 4096 x 4096.
+// and the error e = fp16(lo + c step) - w, as it is or as its TF32 parts.  Bound by memory: 20 bytes
+// written (16 without the low part) and 5 read per weight; a dozen elementwise passes before, 650 -> 67
+// us for 4096 x 4096.
 __global__ void __launch_bounds__(256)
 refine_prepare_kernel(const float* __restrict__ w, int64_t ldw, const uint8_t* __restrict__ codes,
                       const uint8_t* __restrict__ params, const uint16_t* __restrict__ consts, int shift, int64_t n_rows,
@@ -277,7 +278,7 @@ extern "C" int hi2_refine_sweep(float* g, float* c, const float* lo, const float
         if (first >= k) continue;
         GemmArgs<float, float, float> p;
         p.m = n_rows, p.n = k - first, p.kk = len, p.alpha = 1.0f, p.beta = 1.0f;
-        p.a = moves, p.lda = len, p.b = hs + b0 * k + first, p.ldb = k, p.c = g + first, p.ldc = k, p.flags = 0;
+        p.a = moves, p.lda = len, p.b = hs + b0 * k + first, p.ldb = k, p.c = g + first, p.ldc = k;
         rc = launch_gemm_async<float, 8, 8, 16>(false, false, p, s, "refine_sweep");
         if (rc != HI2_OK) return rc;
       }

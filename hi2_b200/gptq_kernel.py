@@ -23,8 +23,12 @@ def update_columns(rows: int, k: int) -> int:
     """Columns whose tensor-core updates reach the columns behind them in one pass over the working
     copy.  One pass per block of 128 is bound by memory once the copy no longer stays in L2 (80 MB);
     below, the products are bound by their launches and grouping only adds some.  Column loop, one by
-    one / groups of 512 / of 1024 columns, ms: 4096 x 11008 6.67 / 5.76 / 5.47, 11008 x 4096 3.02 / 2.72 /
-    2.68, 32768 x 4096 7.41 / 6.30 / 6.37, 512 x 4096 1.40 / 1.50 / 1.49."""
+    one / groups of 512 / of 1024 columns, ms, K = 4096: 4096 rows 1.38 / 1.45 / 1.38, 5120 rows (the line)
+    1.68 / 1.74 / 1.72, 6144 rows 1.82 / 1.82 / 1.76, 8192 rows 2.12 / 1.99 / 1.96, 11008 rows 2.80 / 2.48 /
+    2.44, 16384 rows 3.82 / 3.19 / 3.19.  Wider inputs: 2048 x 8192 2.73 / 2.90 / 2.85, 4096 x 8192 3.74 / 3.51
+    / 3.36, 1024 x 11008 3.39 / 3.70 / 3.66, 2048 x 11008 4.04 / 4.23 / 4.11, 4096 x 11008 6.03 / 5.33 / 5.03.
+    So the line on the size is within 4 % of the better side at every point; groups of 1024 save 0 to 4 %
+    over 512 up to K = 8192 for twice the scratch, and 6 % at K = 11008."""
     if rows * k < GROUP_MIN_ELEMS or k <= 512:
         return BLOCK_COLUMNS
     return 1024 if k > 8192 else 512
@@ -141,8 +145,9 @@ def split_factor(u: torch.Tensor) -> torch.Tensor:
 
 def gptq_round_tc(wc, err1, codes, lo, st, row_grp, u_ptrs, blk, nmax, comp, unit_rows, unit_u_split):
     """:func:`gptq_round` with the trailing update on the tensor cores (3 x TF32, fp32-grade).
-    ``unit_u_split`` holds :func:`split_tf32_transposed` or :func:`split_factor` of each unit's factor.  Returns the device status
-    word (int32 tensor): non-zero when a bounded device-side wait ran out."""
+    ``unit_u_split`` holds :func:`split_tf32_transposed` or :func:`split_factor` of each unit's factor.
+    ``err1`` is not used (the errors stay TF32 parts in scratch of this call) and may be ``None``.  Returns
+    the device status word (int32 tensor): non-zero when a bounded device-side wait ran out."""
     dev = _lib.need_cuda(wc, err1, codes, lo, st, row_grp, u_ptrs, blk, nmax, comp, *unit_u_split)
     n, k = wc.shape
     status = torch.zeros(1, dtype=torch.int32, device=dev)

@@ -371,7 +371,6 @@ def _round_units(units: list[_Unit], jobs: list[GptqJob], want_comp: bool, split
     nmax = _lib.upload(torch.tensor([2 ** jobs[x.job].nbits - 1 for x in units], dtype=torch.float32), dev)
     codes = torch.empty(total, k, dtype=torch.uint8, device=dev)
     comp = torch.empty(total, k, dtype=torch.float32, device=dev) if want_comp else None
-    err1 = torch.empty(total, BLOCK_COLUMNS, dtype=torch.float32, device=dev)
     # INT8 ladders are 64 times finer than INT2: the 3 x TF32 update (error ~1e-6 of |err||U|, ten
     # times an fp32 FMA chain) moves ~0.1 % of INT8 codes, so rows with 256 levels keep the FMA
     # product; for INT2 / INT4 the codes are the same
@@ -381,9 +380,10 @@ def _round_units(units: list[_Unit], jobs: list[GptqJob], want_comp: bool, split
             if u.data_ptr() not in splits:
                 splits[u.data_ptr()] = (u, gptq_kernel.split_factor(u))  # keeps u alive with its split
             parts.append(splits[u.data_ptr()][1])
-        checks.append(gptq_kernel.gptq_round_tc(wc, err1, codes, lo, st, row_grp, u_ptrs, blk, nmax, comp,
+        checks.append(gptq_kernel.gptq_round_tc(wc, None, codes, lo, st, row_grp, u_ptrs, blk, nmax, comp,
                                                 offs, parts))
     else:
+        err1 = torch.empty(total, BLOCK_COLUMNS, dtype=torch.float32, device=dev)
         gptq_kernel.gptq_round(wc, err1, codes, lo, st, row_grp, u_ptrs, blk, nmax, comp, offs, us)
     for x, o, n in zip(units, offs, sizes):
         x.codes = codes[o : o + n]

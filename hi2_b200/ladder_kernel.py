@@ -2,7 +2,7 @@
 
 ``ladder_grid`` is the grid part of the fit as in the reference; ``fit`` adds the least-squares
 refits and ``quantize_rows`` the row-wide parameter quantisation, decode, code assignment and
-error, so one candidate of the tables costs two launches.
+error; ``error_table`` does both for all candidates of a table together.
 """
 
 from __future__ import annotations

@@ -111,7 +111,7 @@ def start_factors(shared: dict, cfg: Config, device, only: str | None = None, in
 def tabulate(weights: dict, plan: LayerPlan, shared: dict, cfg: Config, only: str | None = None,
              into: dict | None = None, grouped: bool = False) -> dict:
     """Error tables of every weight ``{name: [R, K] tensor}`` (or of those reading input ``only``).
-    ``grouped`` tabulates the weights of one shape together, a candidate at a time for all of them
+    ``grouped`` tabulates the weights of one shape together, at all candidates in one call
     (:func:`hi2_b200.calibrate.build_tables_grouped`): what a layer of experts wants, whose hundreds
     of small tables are otherwise bound by the host's launch rate."""
     tables = into if into is not None else {}

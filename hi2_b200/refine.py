@@ -15,7 +15,11 @@ from .format import decode_params
 
 BLOCK_COLUMNS = 128
 GROUP_BLOCKS = 4  # blocks whose moves reach the far columns of g in one product
-GROUP_MIN_ELEMS = 1 << 25  # rows x columns from which grouping pays (below, a step is a latency chain)
+# Rows x columns from which grouping pays (below, a step is a latency chain).  Two sweeps at K = 4096, a block at
+# a time / groups of four, ms: 2048 rows 2.78 / 3.61, 4096 rows 3.83 / 4.44, 6144 rows 5.57 / 5.55, 8192 rows
+# (the line) 6.69 / 6.27, 11008 rows 9.02 / 8.02; 1024 x 11008 8.40 / 10.6, 4096 x 8192 11.9 / 11.6, 4096 x 11008
+# 20.5 / 18.5.  Groups of two or eight blocks are no better on either side.
+GROUP_MIN_ELEMS = 1 << 25
 TC_MIN_K = 512  # inputs at least this wide take the tensor-core products
 
 

@@ -99,7 +99,7 @@ int hi2_fit_ladder(const float* w, int64_t ldw, const float* d, const float* gri
                    float* step, void* stream);
 
 /* hi2/encode.py:95-119 quantize_params + hi2/format.py:45-60 decode_params + the code
- * assignment and error of hi2/encode.py:146-157, one row per thread block.
+ * assignment and error of hi2/encode.py:146-157, one row per warp.
  * Inputs lo/step [n_rows, k/block].  Outputs (each may be null): params u8 [n_rows, nb, 2],
  * consts fp16 [n_rows, 3], lo_d/step_d fp32 decoded ladders with leading dimension ldp,
  * codes u8 [n_rows, k], sse fp32 [n_rows], energy fp32 [n_rows] = sum d*w^2.
@@ -149,8 +149,9 @@ int hi2_gptq_round(float* wc, int64_t n_rows, int64_t k, float* err1, uint8_t* c
 /* The same column loop with the trailing update on the tensor cores: every operand split into
  * two TF32 numbers (hi + lo), three tcgen05 products with fp32 accumulation, accuracy of an fp32
  * FMA chain.  u_split_host[u] is the device address of a [2, k, k] fp32 array holding the hi and
- * lo parts of the TRANSPOSE of unit u's factor (hi2_split_tf32_transposed); err_split is caller scratch [2, n_rows, 128];
- * *status (device int32) is cleared and receives HI2_ERR_TIMEOUT if a bounded wait ran out. */
+ * lo parts of the TRANSPOSE of unit u's factor (hi2_split_tf32_transposed or
+ * hi2_split_factor_transposed); err_split is caller scratch [2, n_rows, 128]; err1 is not used and may be
+ * null; *status (device int32) is cleared and receives HI2_ERR_TIMEOUT if a bounded wait ran out. */
 int hi2_gptq_round_tc(float* wc, int64_t n_rows, int64_t k, float* err1, float* err_split,
                       uint8_t* codes, const float* lo, const float* st, int64_t ldp,
                       const int32_t* row_grp, const int64_t* u_ptrs, const int32_t* blk,
