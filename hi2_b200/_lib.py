@@ -199,6 +199,12 @@ def upload(t: torch.Tensor, dev: torch.device, dtype: torch.dtype | None = None)
     return t.to(dtype).contiguous().pin_memory().to(dev, non_blocking=True)
 
 
+def on_grid(t: torch.Tensor, grid: int) -> torch.Tensor:
+    """``t`` contiguous at an address that is a multiple of ``grid`` bytes: itself, or a copy."""
+    t = t.contiguous()
+    return t if t.data_ptr() % grid == 0 else t.clone()
+
+
 def need_cuda(*tensors: torch.Tensor) -> torch.device:
     """All tensors on one CUDA device; this package has no CPU path."""
     dev = None

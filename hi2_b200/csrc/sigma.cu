@@ -234,6 +234,7 @@ namespace {
 int transform(const float* sigma, float denom, const uint16_t* col_scale, const GroupFlags& had, int64_t k, float* hs,
               float* diag, void* stream) {
   HI2_REQUIRE(sigma && hs, "transform_sigma: null pointer");
+  HI2_REQUIRE(aligned16(sigma) && aligned16(hs), "transform_sigma: sigma and hs must be 16-byte aligned");
   HI2_REQUIRE(sigma != hs, "transform_sigma: in-place operation is not supported");
   HI2_REQUIRE(denom > 0.0f, "transform_sigma: denom must be positive");
   const unsigned nt = (unsigned)ceil_div(k, TS);

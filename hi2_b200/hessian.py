@@ -157,7 +157,7 @@ def transform_sigma(sigma: torch.Tensor, col_scale: torch.Tensor | None, had: to
     dev = _lib.need_cuda(sigma)
     k = sigma.shape[0]
     s = sigma if sigma.dtype == torch.float32 else sigma.float()
-    s = s.contiguous()
+    s = _lib.on_grid(s, 16)
     hs = torch.empty(k, k, dtype=torch.float32, device=dev)
     diag = torch.empty(k, dtype=torch.float32, device=dev) if return_diag else None
     cs = None

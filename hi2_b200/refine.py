@@ -134,12 +134,6 @@ def _as_encoded(w, enc, block: int) -> bool:
             and tuple(enc.params.shape) == (n, k // block, 2) and tuple(enc.consts.shape) == (n, 3))
 
 
-def _on_grid(t: torch.Tensor, grid: int) -> torch.Tensor:
-    """``t`` contiguous at an address that is a multiple of ``grid`` bytes: itself, or a copy."""
-    t = t.contiguous()
-    return t if t.data_ptr() % grid == 0 else t.clone()
-
-
 def refine_groups(groups, hs: torch.Tensor, passes: int, wait: bool = True):
     """One sweep over the rows of every ``(w, enc, nbits, block)`` group (rows of different
     candidates, and of different tensors that read the same input, share the column loop); returns
@@ -161,7 +155,7 @@ def refine_groups(groups, hs: torch.Tensor, passes: int, wait: bool = True):
             wf = w.float()
             if wf.stride(1) != 1 or wf.stride(0) < k or wf.stride(0) % 4 or wf.data_ptr() % 16:
                 wf = wf.clone(memory_format=torch.contiguous_format)  # of one row too, whose stride may be anything
-            refine_kernel.prepare(wf, _on_grid(enc.codes, 4), _on_grid(enc.params, 2), enc.consts.contiguous(), block, c[at],
+            refine_kernel.prepare(wf, _lib.on_grid(enc.codes, 4), _lib.on_grid(enc.params, 2), enc.consts.contiguous(), block, c[at],
                                   lo_x[at], st_x[at], *((e[0][0, at], e[0][1, at]) if use_tc else (e[0][at],)))
             top[at] = float(2**nbits - 1)
             r0 += rows
