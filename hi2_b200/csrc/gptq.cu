@@ -362,6 +362,8 @@ extern "C" int hi2_gptq_round(float* wc, int64_t n_rows, int64_t k, float* err1,
   HI2_REQUIRE(n_units >= 1 && unit_rows_host && u_host, "gptq_round: unit table missing");
   HI2_REQUIRE(unit_rows_host[0] == 0 && unit_rows_host[n_units] == n_rows,
               "gptq_round: units must cover the rows");
+  for (int un = 0; un < n_units; ++un)  // the blocks are staged with 128-bit copies
+    HI2_REQUIRE(aligned16(reinterpret_cast<const void*>(u_host[un])), "gptq_round: factors must be 16-byte aligned");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const std::vector<Span> spans = factor_spans(n_units, unit_rows_host, u_host);
   ChainGraph chain(s, ceil_div(k, LMAX) * (1 + (int64_t)spans.size()));  // the segments and their trailing updates

@@ -365,7 +365,12 @@ def _round_units(units: list[_Unit], jobs: list[GptqJob], want_comp: bool, split
     row_grp = _lib.upload(torch.repeat_interleave(
         torch.arange(len(units), dtype=torch.int32), torch.tensor(sizes)
     ), dev)
-    us = [jobs[x.job].u.to(dev, torch.float32).contiguous() for x in units]
+    factors: dict = {}  # one copy of each, where one is needed
+    for x in units:
+        u = jobs[x.job].u
+        if id(u) not in factors:
+            factors[id(u)] = _lib.on_grid(u.to(dev, torch.float32), 16)
+    us = [factors[id(jobs[x.job].u)] for x in units]
     u_ptrs = _lib.upload(torch.tensor([u.data_ptr() for u in us], dtype=torch.int64), dev)
     blk = torch.stack([x.blk_of for x in units]).contiguous()
     nmax = _lib.upload(torch.tensor([2 ** jobs[x.job].nbits - 1 for x in units], dtype=torch.float32), dev)
