@@ -28,7 +28,7 @@
 // whose own rounding dominates the difference either way.  A non-positive pivot does not trap:
 // the leaf records its index in *info, carries on with a unit pivot, and the host retries with
 // more damping.
-#include "common.cuh"
+#include "gemm.cuh"
 
 namespace hi2 {
 // lazy_tc.cu
@@ -433,20 +433,12 @@ constexpr int P_TILE = PT * P_LD;                               // floats of one
 constexpr int P_STAGE = P_GROUPS * 2 * P_TILE;                  // floats of one stage
 constexpr size_t P_SMEM = (size_t)P_STAGES * P_STAGE * sizeof(float);
 
-// Structure of a product, and the k-range an output tile then needs.
-enum : int {
-  LOWER_OUT = 1,  // output tiles strictly above the diagonal are skipped
-  KA_LE_I = 2,    // A[i, k] == 0 for k > i (A lower triangular)
-  KB_GE_J = 4,    // B[k, j] == 0 for k < j (B lower triangular)
-  KB_LE_J = 8,    // B[k, j] == 0 for k > j (Bt lower triangular)
-};
-
 struct ProductJob {
   const float* a;
   const float* b;
   float* c;
   int m, n, kk;
-  int flags;       // of the above
+  int flags;       // GEMM_* of gemm.cuh
   int trans;       // B is Bt [n, kk]
   int subtract;    // C -= instead of C =
   int negate;      // C = -(A B)
@@ -465,12 +457,12 @@ product_kernel(const ProductJob job0, const ProductJob job1, int64_t ld) {
   const ProductJob& p = blockIdx.z ? job1 : job0;
   const int m0 = blockIdx.y * PT, n0 = blockIdx.x * PT;
   if (m0 >= p.m || n0 >= p.n) return;
-  if ((p.flags & LOWER_OUT) && n0 > m0) return;
+  if ((p.flags & GEMM_LOWER_OUT) && n0 > m0) return;
   const int tid = threadIdx.x, g = tid >> 6, lt = tid & 63, tx = lt & 7, ty = lt >> 3;
   int k_lo = 0, k_hi = p.kk;
-  if (p.flags & KA_LE_I) k_hi = min(k_hi, m0 + PT);
-  if (p.flags & KB_LE_J) k_hi = min(k_hi, n0 + PT);
-  if (p.flags & KB_GE_J) k_lo = n0;  // a multiple of 32
+  if (p.flags & GEMM_KA_LE_I) k_hi = min(k_hi, m0 + PT);
+  if (p.flags & GEMM_KB_LE_J) k_hi = min(k_hi, n0 + PT);
+  if (p.flags & GEMM_KB_GE_J) k_lo = n0;  // a multiple of 32
   const int rounds = (k_hi - k_lo + P_GROUPS * P_STEP - 1) / (P_GROUPS * P_STEP);
 
   auto issue = [&](int r) {
@@ -659,16 +651,16 @@ int factor(const Plan& pl, int64_t off, int64_t n) {
   }
   const int m = (int)n2, k1 = (int)n1;
   // W (in the X21 slot) = A21 X11^T
-  const ProductJob w{a21, x11, x21, m, k1, k1, KB_LE_J, 1, 0, 0};
+  const ProductJob w{a21, x11, x21, m, k1, k1, GEMM_KB_LE_J, 1, 0, 0};
   if ((rc = launch_products(w, nullptr, ld, pl.stream)) != HI2_OK) return rc;
   // A22 -= W W^T (lower tiles), and T (in the A21 slot) = W X11, in one launch
-  const ProductJob schur{x21, x21, a22, m, m, k1, LOWER_OUT, 1, 1, 0};
-  const ProductJob t{x21, x11, a21, m, k1, k1, KB_GE_J, 0, 0, 0};
+  const ProductJob schur{x21, x21, a22, m, m, k1, GEMM_LOWER_OUT, 1, 1, 0};
+  const ProductJob t{x21, x11, a21, m, k1, k1, GEMM_KB_GE_J, 0, 0, 0};
   if ((rc = launch_products(schur, &t, ld, pl.stream)) != HI2_OK) return rc;
   rc = factor(pl, off + n1, n2);
   if (rc != HI2_OK) return rc;
   // X21 = -X22 T
-  const ProductJob last{x22, a21, x21, m, k1, m, KA_LE_I, 0, 0, 1};
+  const ProductJob last{x22, a21, x21, m, k1, m, GEMM_KA_LE_I, 0, 0, 1};
   return launch_products(last, nullptr, ld, pl.stream);
 }
 

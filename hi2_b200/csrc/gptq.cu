@@ -307,6 +307,7 @@ int launch_lazy(float* wc, int64_t n_rows, int64_t k, int64_t i1, int64_t i2, co
   p.a = err1, p.lda = i2 - i1;
   p.b = u + i1 * k + i2, p.ldb = k;
   p.c = wc + i2, p.ldc = k;
+  p.flags = 0;
   return launch_gemm_async<float, 8, 8, 16>(false, false, p, stream, "gptq_lazy_update");
 }
 
@@ -482,7 +483,7 @@ extern "C" int hi2_gemm_f32(int trans_a, int trans_b, int64_t m, int64_t n, int6
   HI2_REQUIRE(c && (kk == 0 || (a && b)), "gemm_f32: null pointer");
   GemmArgs<float, float, float> p;
   p.m = m, p.n = n, p.kk = kk, p.alpha = alpha, p.beta = beta;
-  p.a = a, p.lda = lda, p.b = b, p.ldb = ldb, p.c = c, p.ldc = ldc;
+  p.a = a, p.lda = lda, p.b = b, p.ldb = ldb, p.c = c, p.ldc = ldc, p.flags = 0;
   return launch_gemm_async<float, 8, 8, 16>(trans_a != 0, trans_b != 0, p,
                                             static_cast<cudaStream_t>(stream), "gemm_f32");
 }

@@ -463,7 +463,7 @@ int accumulate_fma(const void* x, int64_t tokens, int64_t k, float* s, cudaStrea
   GemmArgs<float, TX, TX> p;
   p.m = k, p.n = k, p.kk = tokens, p.alpha = 1.0f, p.beta = 1.0f;
   p.a = static_cast<const TX*>(x), p.lda = k, p.b = static_cast<const TX*>(x), p.ldb = k;
-  p.c = s, p.ldc = k;
+  p.c = s, p.ldc = k, p.flags = 0;
   return launch_gemm<float, TX, TX, 8, 8, 8>(true, false, p, stream, "hessian_accumulate (fma)");
 }
 

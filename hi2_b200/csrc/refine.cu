@@ -278,7 +278,7 @@ extern "C" int hi2_refine_sweep(float* g, float* c, const float* lo, const float
         if (first >= k) continue;
         GemmArgs<float, float, float> p;
         p.m = n_rows, p.n = k - first, p.kk = len, p.alpha = 1.0f, p.beta = 1.0f;
-        p.a = moves, p.lda = len, p.b = hs + b0 * k + first, p.ldb = k, p.c = g + first, p.ldc = k;
+        p.a = moves, p.lda = len, p.b = hs + b0 * k + first, p.ldb = k, p.c = g + first, p.ldc = k, p.flags = 0;
         rc = launch_gemm_async<float, 8, 8, 16>(false, false, p, s, "refine_sweep");
         if (rc != HI2_OK) return rc;
       }
